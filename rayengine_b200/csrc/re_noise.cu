@@ -10,11 +10,11 @@
 //   compute_terrain_normal                 RE/cuda-src/sdf_functions.cuh:535-546
 //
 // The permutation table travels as a 512-byte kernel parameter and is
-// expanded into shared memory by every block (one copy per lane, so
-// lattice lookups with divergent indices never conflict on a bank).  The
-// march is FP32-ALU bound; it runs as a per-lane state machine with lane
-// refills so sky rays (few steps) and grazing rays (hundreds) keep the warps
-// full.
+// expanded into shared memory by every block (the march: one copy per lane,
+// so lattice lookups with divergent indices never conflict on a bank; the
+// batch kernels: 16 copies).  The march is bound by the FP32 pipes; it runs
+// as a per-lane state machine with lane refills so sky rays (few steps) and
+// grazing rays (hundreds) keep the warps full.
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -72,12 +72,12 @@ struct SdfDev {
 // order is lane (i & 31) of 8x4 tile (i >> 5), so claims stay coherent.
 constexpr uint32_t kSdfRefill = 4;
 
-__global__ void __launch_bounds__(256) k_sdf(PermTable perm, SdfDev sp, CamDev cam, uint32_t w,
-                                             uint32_t h, float4* __restrict__ out,
-                                             uint32_t* __restrict__ cursor) {
-  extern __shared__ uint32_t perm_smem[];
-  load_perm(perm, perm_smem);
-  Perm P = perm_view(perm_smem);
+__global__ void __launch_bounds__(kRowsThreads) k_sdf(PermTable perm, SdfDev sp, CamDev cam,
+                                                      uint32_t w, uint32_t h,
+                                                      float4* __restrict__ out,
+                                                      uint32_t* __restrict__ cursor) {
+  extern __shared__ uint32_t rows_smem[];
+  const FieldRows P = load_rows(perm, rows_smem);
   uint32_t lane = threadIdx.x & 31u;
   uint32_t tiles_x = (w + 7) / 8;
   uint32_t total = tiles_x * ((h + 3) / 4) * 32u;
@@ -253,13 +253,8 @@ RE_API re_status re_sdf_trace(const re_sdf_params* p, const re_camera* cam, uint
   cudaStream_t st = (cudaStream_t)stream;
   RE_CUDA(cudaMemsetAsync(counter, 0, 4, st));
   RE_CUDA(cudaFuncSetAttribute(re::k_sdf, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)re::kPermSmemBytes));
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, re::k_sdf, 256, re::kPermSmemBytes) !=
-          cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
-  re::k_sdf<<<per_sm * re::sm_count(), 256, re::kPermSmemBytes, st>>>(
+                               (int)re::kRowsSmemBytes));
+  re::k_sdf<<<re::sm_count(), re::kRowsThreads, re::kRowsSmemBytes, st>>>(
       t, sp, cd, w, h, reinterpret_cast<float4*>(d_out), counter);
   RE_CHECK_LAUNCH("re_sdf_trace: launch");
   return RE_OK;

@@ -52,13 +52,12 @@ __device__ __forceinline__ uint32_t mix32(uint32_t a, uint32_t b, uint32_t c) {
 __device__ __forceinline__ float u01(uint32_t h) { return (float)(h >> 8) * 5.9604644775390625e-08f; }
 
 // ------------------------------------------------------ data generation
-__global__ void __launch_bounds__(256) k_nsdf_data(PermTable perm, FieldDev f, CamDev cam,
-                                                   uint32_t w, uint32_t h, float3 bmin, float3 bmax,
-                                                   uint32_t n, uint32_t seed,
-                                                   float4* __restrict__ out) {
-  extern __shared__ uint32_t perm_smem[];
-  load_perm(perm, perm_smem);
-  Perm P = perm_view(perm_smem);
+__global__ void __launch_bounds__(kRowsThreads) k_nsdf_data(PermTable perm, FieldDev f, CamDev cam,
+                                                            uint32_t w, uint32_t h, float3 bmin,
+                                                            float3 bmax, uint32_t n, uint32_t seed,
+                                                            float4* __restrict__ out) {
+  extern __shared__ uint32_t rows_smem[];
+  const FieldRows P = load_rows(perm, rows_smem);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float px = 0.f, py = 0.f, pz = 0.f;
     bool placed = false;
@@ -1319,16 +1318,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_nsdf_cone(InputMap m,
 // evaluations (normals excluded, as in the exact tracer).
 enum : uint32_t { kMarch = 0, kProbe = 1, kRoot = 2, kNormal = 3 };
 
+// the field's table, then the warps' rings (64 entries of 32 bytes each)
+constexpr uint32_t kRefineSmemBytes = kRowsSmemBytes + (kRowsThreads / 32) * 64 * 32;
+
 // NT: the normal (RefineDev::normal_taps), fixed at compile time so that
 // the analytic-gradient form (1) carries no stencil state.
 template <uint32_t NT>
-__global__ void __launch_bounds__(256) k_sdf_refine(PermTable perm, FieldDev f, RefineDev rd,
-                                                    CamDev cam, uint32_t w, uint32_t h, int direct,
-                                                    const uint4* __restrict__ queue,
-                                                    uint32_t* __restrict__ counters,
-                                                    unsigned long long* __restrict__ totals,
-                                                    float4* __restrict__ out) {
-  extern __shared__ uint32_t perm_smem[];
+__global__ void __launch_bounds__(kRowsThreads) k_sdf_refine(
+    PermTable perm, FieldDev f, RefineDev rd, CamDev cam, uint32_t w, uint32_t h, int direct,
+    const uint4* __restrict__ queue, uint32_t* __restrict__ counters,
+    unsigned long long* __restrict__ totals, float4* __restrict__ out) {
+  extern __shared__ uint32_t rows_smem[];
   // Per-warp ring of set-up rays (64 entries): the warp claims 32 work
   // indices at a time and all its lanes set those rays up together (pixel,
   // two divisions and three normalisations for the direction, the cone
@@ -1336,10 +1336,9 @@ __global__ void __launch_bounds__(256) k_sdf_refine(PermTable perm, FieldDev f, 
   // the few lanes that happen to be idle; idle lanes then take entries.
   // Entry: {d.xyz, t} and {pixel (0xFFFFFFFF: no ray), t_lo bits, base
   // steps, 0}.
-  __shared__ float4 ring_a[8][64];
-  __shared__ uint4 ring_b[8][64];
-  load_perm(perm, perm_smem);
-  Perm P = perm_view(perm_smem);
+  float4(*ring_a)[64] = reinterpret_cast<float4(*)[64]>(rows_smem + kRowsSmemBytes / 4);
+  uint4(*ring_b)[64] = reinterpret_cast<uint4(*)[64]>(ring_a + kRowsThreads / 32);
+  const FieldRows P = load_rows(perm, rows_smem);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   // direct mode claims pixels in 8x4 tiles (claim i = lane i & 31 of tile
   // i >> 5), so a warp's rays start close together
@@ -1997,8 +1996,8 @@ RE_API re_status re_nsdf_generate(re_nsdf* s, const re_sdf_params* field, const 
   bmax.y = s->map.center[1] + 1.f / s->map.inv_half[1];
   bmax.z = s->map.center[2] + 1.f / s->map.inv_half[2];
   RE_CUDA(cudaFuncSetAttribute(re::nsdf::k_nsdf_data, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)re::kPermSmemBytes));
-  re::nsdf::k_nsdf_data<<<re::sm_count() * 3, 256, re::kPermSmemBytes, cs>>>(
+                               (int)re::kRowsSmemBytes));
+  re::nsdf::k_nsdf_data<<<re::sm_count(), re::kRowsThreads, re::kRowsSmemBytes, cs>>>(
       re::perm_of(field->seed), re::field_of(*field), re::cam_dev(*cam), w, h, bmin, bmax,
       num_points, seed, s->data);
   RE_CHECK_LAUNCH("re_nsdf_generate: launch");
@@ -2324,12 +2323,7 @@ RE_API re_status re_nsdf_trace_exact(re_nsdf* s, const re_sdf_params* field,
             : tp->normal_taps == 4u ? re::nsdf::k_sdf_refine<4u>
                                     : re::nsdf::k_sdf_refine<6u>;
   RE_CUDA(cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)re::kPermSmemBytes));
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kr, 256, re::kPermSmemBytes) !=
-          cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
+                               (int)re::nsdf::kRefineSmemBytes));
   re::nsdf::RefineDev rd;
   rd.max_steps = tp->max_exact_steps ? tp->max_exact_steps : field->max_steps;
   rd.root_steps = tp->root_steps ? tp->root_steps : 4;
@@ -2344,7 +2338,7 @@ RE_API re_status re_nsdf_trace_exact(re_nsdf* s, const re_sdf_params* field,
   rd.tile_t = cone ? s->cone_t : nullptr;
   rd.cone_tile = cone ? s->cone_tile : 1u;
   rd.cone_tiles_x = cone ? s->cone_tiles_x : 0u;
-  kr<<<per_sm * re::sm_count(), 256, re::kPermSmemBytes, cs>>>(
+  kr<<<re::sm_count(), re::kRowsThreads, re::nsdf::kRefineSmemBytes, cs>>>(
       re::perm_of(field->seed), re::field_of(*field), rd, re::cam_dev(*cam), w, h,
       exact_only || cone ? 1 : 0, s->queue, s->counters, totals, reinterpret_cast<float4*>(d_out));
   RE_CHECK_LAUNCH("re_nsdf_trace_exact: refine launch");

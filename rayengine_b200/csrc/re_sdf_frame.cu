@@ -301,14 +301,12 @@ __device__ __forceinline__ uint32_t finish_pixel(const ShadeDev& S, V3 col, V3 o
 // Same operations, in the same order per pixel, as one loop per pixel.
 constexpr uint32_t kShadeRefill = 4;
 
-__global__ void __launch_bounds__(256) k_sdf_shadow(PermTable perm, ShadeDev S, uint32_t w,
-                                                    uint32_t h, const float4* __restrict__ hits,
-                                                    uint32_t* __restrict__ rgba,
-                                                    uint32_t* __restrict__ cursor,
-                                                    unsigned long long* __restrict__ evals_out) {
-  extern __shared__ uint32_t perm_smem[];
-  load_perm(perm, perm_smem);
-  Perm P = perm_view(perm_smem);
+__global__ void __launch_bounds__(kRowsThreads) k_sdf_shadow(
+    PermTable perm, ShadeDev S, uint32_t w, uint32_t h, const float4* __restrict__ hits,
+    uint32_t* __restrict__ rgba, uint32_t* __restrict__ cursor,
+    unsigned long long* __restrict__ evals_out) {
+  extern __shared__ uint32_t rows_smem[];
+  const FieldRows P = load_rows(perm, rows_smem);
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t tiles_x = (w + 7) / 8;
   const uint32_t total = tiles_x * ((h + 3) / 4) * 32u;
@@ -476,13 +474,8 @@ re_status shade(const re_sdf_params& f, const re_sdf_shade_params& s, const re_c
   if (s.flags & RE_SDF_SHADE) {
     RE_CUDA(cudaMemsetAsync(ctr, 0, 4, st));
     RE_CUDA(cudaFuncSetAttribute(k_sdf_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kPermSmemBytes));
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sdf_shadow, 256,
-                                                      kPermSmemBytes) != cudaSuccess ||
-        per_sm < 1)
-      per_sm = 1;
-    k_sdf_shadow<<<per_sm * sm_count(), 256, kPermSmemBytes, st>>>(
+                                 (int)kRowsSmemBytes));
+    k_sdf_shadow<<<sm_count(), kRowsThreads, kRowsSmemBytes, st>>>(
         perm_table(f.seed), shade_dev(f, s), w, h, reinterpret_cast<const float4*>(d_hits),
         d_rgba, ctr, reinterpret_cast<unsigned long long*>(d_evals));
     RE_CHECK_LAUNCH("re_render_sdf_frame: shadow launch");

@@ -93,11 +93,11 @@ __device__ __forceinline__ float sample(const GridDev& g, uint32_t quality, V3 p
   return result;
 }
 
-__global__ void k_bake(PermTable perm, uint32_t octaves, float scale, float amp, GridDev g,
-                       float2* __restrict__ out) {
-  extern __shared__ uint32_t perm_smem[];
-  load_perm(perm, perm_smem);
-  Perm P = perm_view(perm_smem);
+__global__ void __launch_bounds__(kRowsThreads) k_bake(PermTable perm, uint32_t octaves,
+                                                       float scale, float amp, GridDev g,
+                                                       float2* __restrict__ out) {
+  extern __shared__ uint32_t rows_smem[];
+  const FieldRows P = load_rows(perm, rows_smem);
   size_t n = (size_t)g.dim[0] * g.dim[1] * g.dim[2];
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
@@ -277,8 +277,8 @@ RE_API re_status re_voxel_bake(const re_sdf_params* field, const re_voxel_grid* 
   re::PermTable t;
   for (int i = 0; i < 512; ++i) t.p[i] = (uint8_t)full[i];
   RE_CUDA(cudaFuncSetAttribute(re::voxel::k_bake, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)re::kPermSmemBytes));
-  re::voxel::k_bake<<<2 * re::sm_count(), 256, re::kPermSmemBytes, (cudaStream_t)stream>>>(
+                               (int)re::kRowsSmemBytes));
+  re::voxel::k_bake<<<re::sm_count(), re::kRowsThreads, re::kRowsSmemBytes, (cudaStream_t)stream>>>(
       t, field->octaves, field->scale, field->amplitude, re::grid_dev(g, d_grid),
       reinterpret_cast<float2*>(d_grid));
   RE_CHECK_LAUNCH("re_voxel_bake: launch");

@@ -1,0 +1,42 @@
+"""The field evaluated two octaves at a time against the CPU oracle, bit for
+bit: octave counts around the pairs (odd ones end on half a pair), and
+coordinates below, across and beyond the range of the paired form (the
+largest |scale * p| times 2^octaves below 2^22) on both sides of zero."""
+import numpy as np
+import pytest
+
+import rayengine_b200 as rb
+from oracle import pyoracle as po
+
+pytestmark = pytest.mark.gpu
+
+DIM = (37, 6, 11)
+
+
+def _bake(octaves, scale, spacing, origin):
+    field = rb.sdf_params(octaves=octaves, scale=scale, amplitude=3.0)
+    got = rb.VoxelGrid.bake(field, DIM, spacing, origin).data.cpu().numpy()
+    want = po.voxel_bake(po.perm(2016), octaves, scale, 3.0, DIM, spacing, origin)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    assert len(np.unique(got)) > DIM[1]
+
+
+@pytest.mark.parametrize("octaves", [1, 2, 3, 7, 8, 9, 16])
+def test_octave_counts(cuda, octaves):
+    # about zero, lattice points (multiples of 4) among the samples
+    _bake(octaves, 0.25, (0.5, 1.0, 0.37), (-9.0, -3.0, -2.0))
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("sign", [-1.0, 1.0])
+@pytest.mark.parametrize("octaves", [7, 8])
+def test_across_the_paired_range(cuda, octaves, axis, sign):
+    # |scale p| crosses 2^(22 - octaves) within the grid
+    edge = 2.0 ** (22 - octaves) / 0.25
+    origin = [-9.0, -3.0, -2.0]
+    origin[axis] = sign * edge - 2.5
+    _bake(octaves, 0.25, (0.5, 1.0, 0.5), tuple(origin))
+
+
+def test_far_from_the_origin(cuda):
+    _bake(8, 1.0, (3.0, 1024.0, 513.0), (3.0e6, -3.0, -7.0e8))
