@@ -8,13 +8,13 @@
 //   data      k_nsdf_data: 50% points uniform in the view box, 50% near the
 //             surface (exact-traced camera hits + N(0, 0.02) offsets),
 //             labelled by the exact field's first-order distance d / |grad d|
-//   training  tcgen05 as well: k_tc_train_fwd (features, 4 MMA layers with
-//             FP32 bias + softplus epilogues, head, L1 loss) and
-//             k_tc_train_bwd per layer (dA_prev = dZ W and dW^T = A^T dZ, the
-//             weight gradient accumulated in tensor memory over the CTA's
-//             tiles), BF16 operands and FP32 accumulation; then k_reduce and
-//             hand-written Adam; one step is captured once in a CUDA graph
-//             and replayed
+//   training  tcgen05 as well: k_tc_train runs a tile's features, 4 MMA layers
+//             with FP32 bias + softplus epilogues, head, L1 loss and the whole
+//             backward pass (dA_prev = dZ W and dW^T = A^T dZ) without leaving
+//             the SM, pre-activations and weight gradients in tensor memory,
+//             BF16 operands and FP32 accumulation; then k_train_reduce sums
+//             the CTAs' gradients and applies hand-written Adam; one step is
+//             captured once in a CUDA graph and replayed
 //   inference tcgen05 (sm_100a): 128-point tiles, BF16 operands in shared
 //             memory (K-major canonical layout, no swizzle), FP32
 //             accumulators in tensor memory, one elected thread issues the
@@ -110,66 +110,66 @@ __global__ void __launch_bounds__(kRowsThreads) k_nsdf_data(PermTable perm, Fiel
 }
 
 // ------------------------------------------------------------- training
-// One step on a batch of B rows (a multiple of 512): k_pack_train packs the
-// BF16 weights, k_tc_train_fwd runs the four hidden layers and the head on
-// the tensor cores (128-row tiles) and stores what the backward pass needs,
-// then k_tc_train_bwd runs once per hidden layer (4 -> 1): dZ = dA softplus'(Z),
-// dA_prev = dZ W and the weight gradient dW^T = A_prev^T dZ, accumulated in
-// tensor memory over the CTA's tiles; k_reduce sums the CTAs' partial
-// gradients and k_adam updates the parameters.
+// One step on a batch of B rows (a multiple of 512): k_tc_train (below) leaves
+// one partial gradient and loss per CTA, k_train_reduce sums them and, when
+// training, applies Adam.
 constexpr int kRowsBwd = 512;   // batch granularity of the training API
-constexpr int kTrRows = 128;    // rows per tensor-core tile (one thread each)
+constexpr int kTrRows = 128;    // rows per tensor-core tile
+// one CTA's partial sums: the gradient in the parameters' order, then the loss
+constexpr uint32_t kPartStride = (uint32_t)kNumParams + 1u;
 
-struct TrainBufs {
-  __nv_bfloat16* x0;  // [B][128] BF16 features (the first layer's input)
-  float* z[4];        // [B][64] pre-activations
-  __nv_bfloat16* a[3];  // [B][64] BF16 activations of layers 1-3 (inputs of 2-4)
-  float* da;          // [B][64] gradient w.r.t. the current layer's output
-  float* da2;         // [B][64]
-  float* part;        // [grid][kNumParams] partial gradients of W1..W4, b1..b4
-  float* part_head;   // [B / 128][kHidden + 2] partial gradients of w5, b5 and the loss
-};
-
-// grad[p] = sum of the partial gradients; the loss of the step is appended
-// to loss_hist.
-__global__ void k_reduce(TrainBufs tb, uint32_t nbwd, uint32_t nfwd, float* __restrict__ grad,
-                         float* __restrict__ loss_hist, const uint32_t* __restrict__ step_ctr,
-                         uint32_t batch) {
-  uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < (uint32_t)OFF_W5) {
-    float s = 0.f;
-    for (uint32_t b = 0; b < nbwd; ++b) s += tb.part[(size_t)b * kNumParams + p];
-    grad[p] = s;
-  } else if (p < (uint32_t)kNumParams + 1) {
-    uint32_t c = p - OFF_W5;  // 0..63 w5, 64 b5, 65 loss
-    float s = 0.f;
-    for (uint32_t b = 0; b < nfwd; ++b) s += tb.part_head[(size_t)b * (kHidden + 2) + c];
-    if (p < (uint32_t)kNumParams)
-      grad[p] = s;
-    else if (loss_hist)
-      loss_hist[*step_ctr] = s / (float)batch;
+// Sum of the partial gradients, in a fixed order: 8 warps of a block each sum
+// every 8th CTA's partials of the block's 32 parameters, then one warp adds
+// the 8 sums.  adam_m null: grad gets the sums.  Otherwise the parameters
+// get one Adam step, the step's loss is appended to loss_hist, and the last
+// block to finish advances the step counter (ctr[0]; ctr[1] counts blocks).
+// A thread per parameter that walked every partial by itself took as long as
+// its chain of loads (82 blocks, 444 + 512 dependent additions); here 651
+// blocks walk at most 19.
+constexpr uint32_t kReduceWarps = 8;
+__global__ void __launch_bounds__(32 * kReduceWarps) k_train_reduce(
+    const float* __restrict__ part, uint32_t nparts, float* __restrict__ grad,
+    float* __restrict__ params, float* __restrict__ adam_m, float* __restrict__ adam_v,
+    float* __restrict__ loss_hist, uint32_t* __restrict__ ctr, float lr, uint32_t batch) {
+  __shared__ float sums[kReduceWarps][32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t p = blockIdx.x * 32u + lane;
+  float s = 0.f;
+  if (p < kPartStride) {
+#pragma unroll 4
+    for (uint32_t b = warp; b < nparts; b += kReduceWarps) s += part[(size_t)b * kPartStride + p];
   }
-}
-
-__global__ void k_adam(float* __restrict__ params, const float* __restrict__ grad,
-                       float* __restrict__ m, float* __restrict__ v, uint32_t* __restrict__ step_ctr,
-                       float lr) {
-  uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t step = *step_ctr + 1;
+  sums[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0) return;
+#pragma unroll
+  for (uint32_t k = 1; k < kReduceWarps; ++k) s += sums[k][lane];
+  if (!adam_m) {
+    if (p < (uint32_t)kNumParams) grad[p] = s;
+    return;
+  }
+  const uint32_t step = *(volatile const uint32_t*)ctr;
   if (p < (uint32_t)kNumParams) {
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    float g = grad[p];
-    float mm = b1 * m[p] + (1.f - b1) * g;
-    float vv = b2 * v[p] + (1.f - b2) * g * g;
-    m[p] = mm;
-    v[p] = vv;
-    float mh = mm / (1.f - powf(b1, (float)step));
-    float vh = vv / (1.f - powf(b2, (float)step));
+    float mm = b1 * adam_m[p] + (1.f - b1) * s;
+    float vv = b2 * adam_v[p] + (1.f - b2) * s * s;
+    adam_m[p] = mm;
+    adam_v[p] = vv;
+    float mh = mm / (1.f - powf(b1, (float)(step + 1u)));
+    float vh = vv / (1.f - powf(b2, (float)(step + 1u)));
     params[p] -= lr * mh / (sqrtf(vh) + eps);
+  } else if (p == (uint32_t)kNumParams) {
+    loss_hist[step] = s / (float)batch;
+  }
+  __syncwarp();
+  if (lane == 0) {
+    __threadfence();  // this block has read the step before it counts as done
+    if (atomicAdd(&ctr[1], 1u) == gridDim.x - 1u) {
+      ctr[1] = 0u;
+      ctr[0] = step + 1u;
+    }
   }
 }
-
-__global__ void k_step_inc(uint32_t* step_ctr) { *step_ctr += 1; }
 
 // ------------------------------------------------ tensor-core inference
 // Canonical K-major BF16 layout without swizzle: 8 rows x 8 k-elements
@@ -224,8 +224,11 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t sbo_bytes) {
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128u >> 4) << 16) |
+// Operand descriptor.  sbo: stride between groups of 8 along M or N; lbo:
+// between groups of 8 along K (128 bytes when K is the contiguous dimension).
+__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t sbo_bytes,
+                                              uint32_t lbo_bytes = 128u) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16) |
          ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
@@ -233,11 +236,12 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t sbo_bytes
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) |
                             ((128u >> 4) << 24);
 
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t acc) {
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t acc,
+                                         uint32_t idesc = kIdesc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(kIdesc), "r"(acc));
+      "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -584,372 +588,388 @@ __global__ void __launch_bounds__(128) k_ref_eval(InputMap m, const float* __res
 }
 
 // ------------------------------------------------ tensor-core training
-// Training weight pack: the forward's W1..W4 as in the inference pack but
-// without the first-layer bias columns (the training adds b1 in FP32), then
-// W2^T..W4^T (canonical rows = layer inputs), the B operands of dA_prev = dZ W.
-constexpr uint32_t kTrPackBytes = kPackWBytes + 3 * kPackWh;  // 65536
+// k_tc_train: one CTA takes 128-row tiles of the batch and carries each
+// through the forward pass, the loss and the backward pass.
+//
+// Four threads share a row (warp w: rows 32 (w & 3) .. + 31, the lanes of
+// tensor memory it may read; columns 16 (w >> 2) .. + 15 of a layer), so an
+// epilogue holds 16 values a thread and 16 warps are there to hide the
+// latency of the chain MMA -> load -> softplus -> store -> MMA, 8 links a
+// tile.
+//
+// Nothing of a tile goes to memory.  The pre-activations Z1..Z4 stay in
+// tensor memory as FP32 accumulators (columns 0..255) until the backward
+// pass has read them; dA of the layer below then takes the same columns.
+// The weight gradients dW1^T..dW4^T stay in columns 256..511 over all of the
+// CTA's tiles.  Activations (BF16, the MMA operands) stay in shared memory.
+//
+// Every operand is stored once: a core matrix of 8 rows x 16 bytes reads as
+// K-major when the contiguous 8 elements run along K, and as MN-major when
+// they run along M or N, with the two strides exchanged.  So A_prev (rows x
+// inputs) is the A operand of the layer (K = inputs) and, transposed by the
+// descriptor, of dW^T = A_prev^T dZ (M = inputs, K = rows); dZ is the A
+// operand of dA = dZ W and the B operand of dW^T; W (outputs x inputs) is
+// the B operand of the layer and of dA.
+//
+// The bias gradient rides in dW^T: an input column of ones (99 of the
+// features, whose weights are packed as zero, and 64 of the activations)
+// makes that accumulator row sum_b dZ.  With 64 inputs, M = 128 reads past
+// the ones column into the next row group; those accumulator rows are never
+// read.
+//
+// Measured on B200, 65,536 rows: one forward launch that stored 257 MB of
+// activations and four backward launches that read them back and transposed
+// the operands with 2-byte stores, the reduction and the copies took 308 us
+// a re_nsdf_loss_grad call; this kernel 59 us, the reduction 6 us, the call
+// 92 us.  What is left is the chain of links (issue slots 48 % busy, 4 rounds
+// of tiles at 15 us).
+constexpr int kTrainThreads = 512;
+constexpr uint32_t kActCols = 72;       // 64 activations, the ones column, 7 zeros
+constexpr uint32_t kOnesX = 99;         // column of ones in the features
+constexpr uint32_t kFeatK = 112;        // features in use (99) and the ones, in steps of 16
+constexpr uint32_t kTrainCols = 512;    // tensor-memory columns
+constexpr uint32_t kIdescTransA = 1u << 15, kIdescTransB = 1u << 16;  // MN-major A, B
 
-__global__ void k_pack_train(const float* __restrict__ params, unsigned char* __restrict__ pack) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < (uint32_t)(kHidden * kIn)) {
-    uint32_t n = i / kIn, k = i % kIn;
-    *reinterpret_cast<__nv_bfloat16*>(pack + canon_off(n, k, kIn)) =
-        __float2bfloat16_rn(params[OFF_W1 + i]);
-  }
-  if (i < (uint32_t)(3 * kHidden * kHidden)) {
-    uint32_t l = i / (kHidden * kHidden), e = i % (kHidden * kHidden);
-    uint32_t n = e / kHidden, k = e % kHidden;
-    __nv_bfloat16 w = __float2bfloat16_rn(params[w_off(1 + l) + e]);
-    *reinterpret_cast<__nv_bfloat16*>(pack + kPackW1 + l * kPackWh + canon_off(n, k, kHidden)) = w;
-    *reinterpret_cast<__nv_bfloat16*>(pack + kPackWBytes + l * kPackWh +
-                                      canon_off(k, n, kHidden)) = w;
-  }
-}
-
-// Issues `steps` MMAs of K = 16 (M 128, N 64): D (+)= A B^T, A and B K-major
-// canonical with rows of `ka` / `kb` elements.
-__device__ __forceinline__ void mma_chain(uint32_t d_tmem, uint32_t a, uint32_t ka, uint32_t b,
-                                          uint32_t kb, uint32_t steps, bool accumulate) {
-#pragma unroll 1
-  for (uint32_t kk = 0; kk < steps; ++kk)
-    mma_bf16(d_tmem, umma_desc(a + kk * 256u, ka * 16u), umma_desc(b + kk * 256u, kb * 16u),
-             (accumulate || kk > 0) ? 1u : 0u);
-}
-
-struct __align__(1024) TrFwdSmem {
-  unsigned char w[kPackWBytes];          // W1..W4, canonical
-  unsigned char x[kTrRows * kIn * 2];    // layer input (K 128 or 64); FP32 scratch for the head
+struct __align__(1024) TrainSmem {
+  unsigned char w[kPackWBytes];                   // W1..W4, canonical
+  unsigned char x[kTrRows * kIn * 2];             // features
+  unsigned char a[3][kTrRows * kActCols * 2];     // activations of layers 1..3
+  unsigned char dz[2][kTrRows * kHidden * 2];     // dZ, two layers in turn
   float bias[4][kHidden];
   float w5[kHidden];
-  float gs[kTrRows], ls[kTrRows];
+  float head[4][kTrRows];                         // the row's output by column quarter
+  float red[4][kHidden + 2];                      // w5, b5 and loss sums by row quarter
   float b5;
   uint64_t bar;
   uint32_t tmem;
 };
-constexpr size_t kTrFwdSmemBytes = sizeof(TrFwdSmem) + 1024;
+constexpr size_t kTrainSmemBytes = sizeof(TrainSmem) + 1024;
 
-// Forward of one training step: features, four hidden layers (MMA + FP32
-// bias + softplus, Z kept in FP32 and the activations in BF16 for the
-// backward pass), head, L1 loss and its gradient dA4 = sign(out - label) / B
-// * w5; partial gradients of w5, b5 and the loss per tile.
-__global__ void __launch_bounds__(kTrRows) k_tc_train_fwd(InputMap m,
-                                                          const float4* __restrict__ data,
-                                                          uint32_t npts,
-                                                          const uint32_t* __restrict__ step_ctr,
-                                                          uint32_t seed, int direct,
-                                                          const unsigned char* __restrict__ pack,
-                                                          const float* __restrict__ params,
-                                                          TrainBufs tb, uint32_t batch,
-                                                          float* __restrict__ pred_out,
-                                                          int* __restrict__ err) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+        "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Octaves 4 half .. 4 half + 3 of a chain's features (chain_features, 24 of
+// its 48 values), the doublings below them carried through.
+__device__ __forceinline__ void half_chain(const InputMap& m, const float q[3], int chain,
+                                           int half, float out[24]) {
+  float f = chain ? m.f0 * 1.41421356f : m.f0;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    float arg = f * q[j];
+    float r = arg - rintf(arg);
+    float s, c;
+    __sincosf(6.28318531f * r, &s, &c);
+    for (int o = 0; o < 4 * half; ++o) {
+      float s2 = 2.0f * s * c;
+      c = __fmaf_rn(-2.0f * s, s, 1.0f);
+      s = s2;
+    }
+#pragma unroll
+    for (int o = 0; o < kOctaves / 2; ++o) {
+      out[o * 6 + 2 * j] = s;
+      out[o * 6 + 2 * j + 1] = c;
+      float s2 = 2.0f * s * c;
+      c = __fmaf_rn(-2.0f * s, s, 1.0f);
+      s = s2;
+    }
+  }
+}
+
+// softplus_approx of two values, rounded to BF16, and its derivative (u times
+// the derivative of the polynomial; one minus that for x > 0), the
+// polynomials in packed FP32 (each half rounded as the scalar form rounds).
+__device__ __forceinline__ f32x2 splat2(float c) { return pack2(c, c); }
+__device__ __forceinline__ f32x2 exp_neg_abs2(float x0, float x1) {
+  return pack2(__expf(-fabsf(x0)), __expf(-fabsf(x1)));
+}
+__device__ __forceinline__ uint32_t softplus_pair(float x0, float x1) {
+  const f32x2 u = exp_neg_abs2(x0, x1);
+  f32x2 p = fma2(u, splat2(-0.017806457f), splat2(0.083866805f));
+  p = fma2(u, p, splat2(-0.19167475f));
+  p = fma2(u, p, splat2(0.31643057f));
+  p = fma2(u, p, splat2(-0.49753284f));
+  p = fma2(u, p, splat2(0.9998613f));
+  float a, b;
+  unpack2(mul2(u, p), a, b);
+  return pack_bf16x2(__fadd_rn(fmaxf(x0, 0.0f), a), __fadd_rn(fmaxf(x1, 0.0f), b));
+}
+__device__ __forceinline__ f32x2 softplus_deriv2(float x0, float x1) {
+  const f32x2 u = exp_neg_abs2(x0, x1);
+  f32x2 p = fma2(u, splat2(6.0f * -0.017806457f), splat2(5.0f * 0.083866805f));
+  p = fma2(u, p, splat2(4.0f * -0.19167475f));
+  p = fma2(u, p, splat2(3.0f * 0.31643057f));
+  p = fma2(u, p, splat2(2.0f * -0.49753284f));
+  p = fma2(u, p, splat2(0.9998613f));
+  float g0, g1;
+  unpack2(mul2(u, p), g0, g1);
+  return pack2(x0 > 0.0f ? __fsub_rn(1.0f, g0) : g0, x1 > 0.0f ? __fsub_rn(1.0f, g1) : g1);
+}
+
+// z += this thread's 16 biases.
+__device__ __forceinline__ void add_bias16(float (&z)[16], const float* bias) {
+  const float4* b4 = reinterpret_cast<const float4*>(bias);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float4 b = b4[j];
+    unpack2(add2(pack2(z[4 * j], z[4 * j + 1]), pack2(b.x, b.y)), z[4 * j], z[4 * j + 1]);
+    unpack2(add2(pack2(z[4 * j + 2], z[4 * j + 3]), pack2(b.z, b.w)), z[4 * j + 2], z[4 * j + 3]);
+  }
+}
+
+// Stores are visible to the MMAs and every thread's tensor-memory reads are
+// done before the next ones are issued.
+__device__ __forceinline__ void train_sync() {
+  fence_async_smem();
+  fence_before();
+  __syncthreads();
+  fence_after();
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1) k_tc_train(
+    InputMap m, const float4* __restrict__ data, uint32_t npts,
+    const uint32_t* __restrict__ step_ctr, uint32_t seed, int direct,
+    const float* __restrict__ params, float* __restrict__ part, uint32_t batch,
+    float* __restrict__ pred_out, int* __restrict__ err) {
   extern __shared__ unsigned char smem_raw[];
-  TrFwdSmem& s = *reinterpret_cast<TrFwdSmem*>(
+  TrainSmem& s = *reinterpret_cast<TrainSmem*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int row = threadIdx.x;
-  for (uint32_t i = row; i < kPackWBytes / 16; i += kTrRows)
-    reinterpret_cast<uint4*>(s.w)[i] = __ldg(reinterpret_cast<const uint4*>(pack) + i);
-  for (uint32_t i = row; i < 4 * kHidden; i += kTrRows)
-    s.bias[i / kHidden][i % kHidden] = params[b_off(i / kHidden) + i % kHidden];
-  if (row < kHidden) s.w5[row] = bf16_round(params[OFF_W5 + row]);
-  if (row == 0) {
+  const int tid = threadIdx.x;
+  const int row = tid & 127, quarter = tid >> 7;  // quarter: columns 16 quarter .. + 15
+  const int col = 16 * quarter;
+  // BF16 weights, 8 inputs of an output at a time
+  for (int i = tid; i < kHidden * (kIn + 3 * kHidden) / 8; i += kTrainThreads) {
+    const bool first = i < kHidden * kIn / 8;
+    const int l = first ? 0 : 1 + (i - kHidden * kIn / 8) / (kHidden * kHidden / 8);
+    const int e = first ? i : (i - kHidden * kIn / 8) % (kHidden * kHidden / 8);
+    const uint32_t K = first ? kIn : kHidden;
+    const uint32_t n = (uint32_t)e / (K / 8), k = ((uint32_t)e % (K / 8)) * 8u;
+    const float4* src = reinterpret_cast<const float4*>(params + w_off(l) + n * K + k);
+    float4 u = src[0], v = src[1];
+    if (first && k >= 96u) {  // the features end at column 98
+      if (k > 96u) u = make_float4(0.f, 0.f, 0.f, 0.f);
+      u.w = 0.f;
+      v = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    store_chunk(s.w + (first ? 0u : kPackW1 + (uint32_t)(l - 1) * kPackWh), (int)n, (int)k, K,
+                pack_bf16x2(u.x, u.y), pack_bf16x2(u.z, u.w), pack_bf16x2(v.x, v.y),
+                pack_bf16x2(v.z, v.w));
+  }
+  if (tid < 4 * kHidden)
+    s.bias[tid / kHidden][tid % kHidden] = params[b_off(tid / kHidden) + tid % kHidden];
+  else if (tid < 5 * kHidden)
+    s.w5[tid - 4 * kHidden] = bf16_round(params[OFF_W5 + tid - 4 * kHidden]);
+  // the constant columns: zeros past the features, the activations' ones
+  if (quarter == 0) {
+#pragma unroll
+    for (int c = 13; c < 16; ++c) store_chunk(s.x, row, 8 * c, kIn, 0u, 0u, 0u, 0u);
+  } else {
+    store_chunk(s.a[quarter - 1], row, kHidden, kActCols, 0x3F80u, 0u, 0u, 0u);
+  }
+  if (tid == 0) {
     s.b5 = params[OFF_B5];
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s.bar)));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if ((row >> 5) == 0) {
+  // every column of the SM: shared memory admits no second CTA of this
+  // kernel, and the inference kernels' CTAs give theirs back when they end
+  if (tid < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_addr(&s.tmem)),
-                 "r"(64));
+                 "r"(kTrainCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  fence_before();
-  __syncthreads();
-  fence_after();
-  const uint32_t tcol = s.tmem + ((32u * (uint32_t)(row >> 5)) << 16);
+  train_sync();
+  // this thread's lanes and columns of a 64-column accumulator
+  const uint32_t tme = s.tmem + ((32u * (uint32_t)(row >> 5)) << 16) + (uint32_t)col;
+  const uint32_t xa = smem_addr(s.x), aa = smem_addr(s.a), da = smem_addr(s.dz),
+                 wa = smem_addr(s.w);
+  constexpr uint32_t kActBytes = kTrRows * kActCols * 2, kDzBytes = kTrRows * kHidden * 2;
   const uint32_t step = *step_ctr;
   uint32_t phase = 0;
-  bool ok = true;
+  bool ok = true, started = false;
+  float gw5[16], gb5 = 0.f, loss = 0.f;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) gw5[j] = 0.f;
   const uint32_t tiles = batch / kTrRows;
-  for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-    uint32_t b = tile * kTrRows + row;
-    uint32_t idx = direct ? b : mix32(seed, step, b) % npts;
-    float4 pt = __ldg(&data[idx]);
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const uint32_t b = tile * kTrRows + (uint32_t)row;
+    const uint32_t idx = direct ? b : mix32(seed, step, b) % npts;
+    const float4 pt = __ldg(&data[idx]);
     float q[3];
     normalise(m, pt.x, pt.y, pt.z, q);
     {
-      uint4* xg = reinterpret_cast<uint4*>(tb.x0 + (size_t)b * kIn);
-      float v[48];
+      float v[24];
+      const int chain = quarter >> 1, half = quarter & 1;
+      half_chain(m, q, chain, half, v);
+      // the previous tile's last MMAs read the features
+      if (started && ok) ok = mbar_wait(&s.bar, phase);
+      if (started) phase ^= 1u;
 #pragma unroll
-      for (int chain = 0; chain < 2; ++chain) {
-        chain_features(m, q, chain, v);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-          uint4 u = make_uint4(pack_bf16x2(v[c * 8 + 0], v[c * 8 + 1]),
-                               pack_bf16x2(v[c * 8 + 2], v[c * 8 + 3]),
-                               pack_bf16x2(v[c * 8 + 4], v[c * 8 + 5]),
-                               pack_bf16x2(v[c * 8 + 6], v[c * 8 + 7]));
-          store_chunk(s.x, row, (chain * 6 + c) * 8, kIn, u.x, u.y, u.z, u.w);
-          xg[chain * 6 + c] = u;
-        }
-      }
-      uint4 u = make_uint4(pack_bf16x2(q[0], q[1]), pack_bf16x2(q[2], 0.f), 0u, 0u);
-      store_chunk(s.x, row, 96, kIn, u.x, u.y, u.z, u.w);
-      xg[12] = u;
-#pragma unroll
-      for (int c = 13; c < 16; ++c) {
-        store_chunk(s.x, row, c * 8, kIn, 0u, 0u, 0u, 0u);
-        xg[c] = make_uint4(0u, 0u, 0u, 0u);
-      }
+      for (int c = 0; c < 3; ++c)
+        store_chunk(s.x, row, (chain * 6 + half * 3 + c) * 8, kIn,
+                    pack_bf16x2(v[c * 8 + 0], v[c * 8 + 1]), pack_bf16x2(v[c * 8 + 2], v[c * 8 + 3]),
+                    pack_bf16x2(v[c * 8 + 4], v[c * 8 + 5]), pack_bf16x2(v[c * 8 + 6], v[c * 8 + 7]));
+      if (quarter == 0)
+        store_chunk(s.x, row, 96, kIn, pack_bf16x2(q[0], q[1]), pack_bf16x2(q[2], 1.0f), 0u, 0u);
     }
-    float d = 0.f;
-    uint32_t a4[32];
+    float z[16], d = 0.f;
+    uint32_t a4[8];
 #pragma unroll 1
-    for (int layer = 0; layer < 4; ++layer) {
-      const uint32_t K = layer == 0 ? kIn : kHidden;
-      fence_async_smem();
-      fence_before();
-      __syncthreads();
-      fence_after();
-      if (row == 0) {
-        mma_chain(s.tmem, smem_addr(s.x), K,
-                  smem_addr(s.w + (layer == 0 ? 0u : kPackW1 + (layer - 1) * kPackWh)), K, K / 16,
-                  false);
+    for (int l = 0; l < 4; ++l) {
+      train_sync();
+      if (tid == 0) {
+        const uint32_t A = l == 0 ? xa : aa + (uint32_t)(l - 1) * kActBytes;
+        const uint32_t B = l == 0 ? wa : wa + kPackW1 + (uint32_t)(l - 1) * kPackWh;
+        const uint32_t sa = (l == 0 ? kIn : kActCols) * 16u, sb = (l == 0 ? kIn : kHidden) * 16u;
+        const uint32_t steps = (l == 0 ? kFeatK : (uint32_t)kHidden) / 16u;
+        for (uint32_t k = 0; k < steps; ++k)
+          mma_bf16(s.tmem + 64u * (uint32_t)l, umma_desc(A + k * 256u, sa),
+                   umma_desc(B + k * 256u, sb), k > 0u ? 1u : 0u);
         mma_commit(&s.bar);
       }
-      ok = __syncthreads_and(mbar_wait(&s.bar, phase) && ok);  // CTA-uniform
+      if (ok) ok = mbar_wait(&s.bar, phase);
       phase ^= 1u;
+      __syncwarp();
       fence_after();
+      tmem_ld16(tme + 64u * (uint32_t)l, z);
+      add_bias16(z, &s.bias[l][col]);
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        float acc[32];
-        tmem_ld32(tcol + 32u * (uint32_t)half, acc);
-        float4* zg = reinterpret_cast<float4*>(tb.z[layer] + (size_t)b * kHidden + 32 * half);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) acc[j] += s.bias[layer][32 * half + j];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          zg[j] = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
-        uint32_t a[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          a[j] = pack_bf16x2(softplus_approx(acc[2 * j]), softplus_approx(acc[2 * j + 1]));
-        if (layer < 3) {
-          uint4* ag = reinterpret_cast<uint4*>(tb.a[layer] + (size_t)b * kHidden + 32 * half);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            store_chunk(s.x, row, 32 * half + 8 * c, kHidden, a[4 * c], a[4 * c + 1],
-                        a[4 * c + 2], a[4 * c + 3]);
-            ag[c] = make_uint4(a[4 * c], a[4 * c + 1], a[4 * c + 2], a[4 * c + 3]);
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            a4[16 * half + j] = a[j];
-            int c = 32 * half + 2 * j;
-            d = __fmaf_rn(__uint_as_float(a[j] << 16), s.w5[c], d);
-            d = __fmaf_rn(__uint_as_float(a[j] & 0xFFFF0000u), s.w5[c + 1], d);
-          }
-        }
+      for (int j = 0; j < 8; ++j) a4[j] = softplus_pair(z[2 * j], z[2 * j + 1]);
+      if (l < 3) {
+        store_chunk(s.a[l], row, col, kActCols, a4[0], a4[1], a4[2], a4[3]);
+        store_chunk(s.a[l], row, col + 8, kActCols, a4[4], a4[5], a4[6], a4[7]);
       }
-      fence_before();
     }
     // head and L1 loss
-    float pred = d + s.b5;
-    float diff = pred - pt.w;
-    float g = (diff > 0.f ? 1.f : (diff < 0.f ? -1.f : 0.f)) / (float)batch;
-    if (pred_out) pred_out[b] = pred;
-    float4* dag = reinterpret_cast<float4*>(tb.da + (size_t)b * kHidden);
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
-      dag[j] = make_float4(g * s.w5[4 * j], g * s.w5[4 * j + 1], g * s.w5[4 * j + 2],
-                           g * s.w5[4 * j + 3]);
-    // every MMA of the tile has completed: the input buffer is free for the
-    // head's reduction (row-major FP32 [128][64])
+    for (int j = 0; j < 8; ++j) {
+      d = __fmaf_rn(__uint_as_float(a4[j] << 16), s.w5[col + 2 * j], d);
+      d = __fmaf_rn(__uint_as_float(a4[j] & 0xFFFF0000u), s.w5[col + 2 * j + 1], d);
+    }
+    s.head[quarter][row] = d;
     __syncthreads();
-    float* red = reinterpret_cast<float*>(s.x);
+    const float pred =
+        ((s.head[0][row] + s.head[1][row]) + (s.head[2][row] + s.head[3][row])) + s.b5;
+    const float diff = pred - pt.w;
+    const float g = (diff > 0.f ? 1.f : (diff < 0.f ? -1.f : 0.f)) / (float)batch;
+    if (quarter == 0) {
+      if (pred_out) pred_out[b] = pred;
+      gb5 += g;
+      loss += fabsf(diff);
+    }
+    float dv[16];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      red[row * kHidden + 2 * j] = g * __uint_as_float(a4[j] << 16);
-      red[row * kHidden + 2 * j + 1] = g * __uint_as_float(a4[j] & 0xFFFF0000u);
+    for (int j = 0; j < 8; ++j) {
+      gw5[2 * j] = __fmaf_rn(g, __uint_as_float(a4[j] << 16), gw5[2 * j]);
+      gw5[2 * j + 1] = __fmaf_rn(g, __uint_as_float(a4[j] & 0xFFFF0000u), gw5[2 * j + 1]);
+      dv[2 * j] = g * s.w5[col + 2 * j];
+      dv[2 * j + 1] = g * s.w5[col + 2 * j + 1];
     }
-    s.gs[row] = g;
-    s.ls[row] = fabsf(diff);
-    __syncthreads();
-    float* ph = tb.part_head + (size_t)tile * (kHidden + 2);
-    if (row < kHidden) {
-      float acc = 0.f;
-      for (int r = 0; r < kTrRows; ++r) acc += red[r * kHidden + row];
-      ph[row] = acc;
-    } else if (row == kHidden) {
-      float acc = 0.f;
-      for (int r = 0; r < kTrRows; ++r) acc += s.gs[r];
-      ph[kHidden] = acc;
-    } else if (row == kHidden + 1) {
-      float acc = 0.f;
-      for (int r = 0; r < kTrRows; ++r) acc += s.ls[r];
-      ph[kHidden + 1] = acc;
+    // backward: dv = dA and z = Z of layer l
+#pragma unroll 1
+    for (int l = 3; l >= 0; --l) {
+      const uint32_t buf = (uint32_t)(3 - l) & 1u;
+      uint32_t pk[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float d0, d1;
+        unpack2(mul2(pack2(dv[2 * j], dv[2 * j + 1]), softplus_deriv2(z[2 * j], z[2 * j + 1])), d0,
+                d1);
+        pk[j] = pack_bf16x2(d0, d1);
+      }
+      store_chunk(s.dz[buf], row, col, kHidden, pk[0], pk[1], pk[2], pk[3]);
+      store_chunk(s.dz[buf], row, col + 8, kHidden, pk[4], pk[5], pk[6], pk[7]);
+      train_sync();
+      if (tid == 0) {
+        const uint32_t D = da + buf * kDzBytes;
+        if (l > 0) {
+          // dA of the layer below, in Z_l's columns (every thread has read them)
+          const uint32_t W = wa + kPackW1 + (uint32_t)(l - 1) * kPackWh;
+#pragma unroll 1
+          for (uint32_t k = 0; k < kHidden / 16u; ++k)
+            mma_bf16(s.tmem + 64u * (uint32_t)l, umma_desc(D + k * 256u, kHidden * 16u),
+                     umma_desc(W + k * 2u * kHidden * 16u, 128u, kHidden * 16u), k > 0u ? 1u : 0u,
+                     kIdesc | kIdescTransB);
+          mma_commit(&s.bar);
+        }
+        // dW^T over the tile's rows; it runs while the next layer's dZ is
+        // made, and the next commit covers it, so this dZ buffer is free
+        // again two layers on
+        const uint32_t A = l == 0 ? xa : aa + (uint32_t)(l - 1) * kActBytes;
+        const uint32_t ga = (l == 0 ? kIn : kActCols) * 16u;
+#pragma unroll 1
+        for (uint32_t k = 0; k < kTrRows / 16u; ++k)
+          mma_bf16(s.tmem + 256u + 64u * (uint32_t)l, umma_desc(A + k * 2u * ga, 128u, ga),
+                   umma_desc(D + k * 2u * kHidden * 16u, 128u, kHidden * 16u),
+                   started || k > 0u ? 1u : 0u, kIdesc | kIdescTransA | kIdescTransB);
+        if (l == 0) mma_commit(&s.bar);
+      }
+      if (l > 0) {
+        if (ok) ok = mbar_wait(&s.bar, phase);
+        phase ^= 1u;
+        __syncwarp();
+        fence_after();
+        tmem_ld16(tme + 64u * (uint32_t)l, dv);
+        tmem_ld16(tme + 64u * (uint32_t)(l - 1), z);
+        add_bias16(z, &s.bias[l - 1][col]);
+      }
     }
-    __syncthreads();  // the reduction has read the scratch before the next tile's features
+    started = true;
   }
-  if (!ok && row == 0) atomicExch(err, 1);
+  // the grid has no CTA without a tile, so `started` holds here
+  if (ok) ok = mbar_wait(&s.bar, phase);
+  __syncwarp();
+  fence_after();
+  // this CTA's sums; tensor-memory lane = input k, column = output n
+  float* pp = part + (size_t)blockIdx.x * kPartStride;
+#pragma unroll 1
+  for (int l = 0; l < 4; ++l) {
+    const int Kin = l == 0 ? kIn : kHidden, ones = l == 0 ? (int)kOnesX : kHidden;
+    float acc[16];
+    tmem_ld16(tme + 256u + 64u * (uint32_t)l, acc);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      if (row < Kin) pp[w_off(l) + (col + j) * Kin + row] = row == ones ? 0.f : acc[j];
+      if (row == ones) pp[b_off(l) + col + j] = acc[j];
+    }
+  }
+  // w5, b5 and the loss over the CTA's rows
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) gw5[j] += __shfl_xor_sync(0xFFFFFFFFu, gw5[j], off);
+    gb5 += __shfl_xor_sync(0xFFFFFFFFu, gb5, off);
+    loss += __shfl_xor_sync(0xFFFFFFFFu, loss, off);
+  }
+  if ((tid & 31) == 0) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) s.red[row >> 5][col + j] = gw5[j];
+    if (quarter == 0) {
+      s.red[row >> 5][kHidden] = gb5;
+      s.red[row >> 5][kHidden + 1] = loss;
+    }
+  }
+  ok = __syncthreads_and(ok);
+  if (tid < kHidden + 2)
+    pp[OFF_W5 + tid] = (s.red[0][tid] + s.red[1][tid]) + (s.red[2][tid] + s.red[3][tid]);
+  if (!ok && tid == 0) atomicExch(err, 1);
   fence_before();
   __syncthreads();
   fence_after();
-  if ((row >> 5) == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem), "r"(64));
-}
-
-struct __align__(1024) TrBwdSmem {
-  unsigned char wt[kPackWh];                // W^T of this layer (rows = inputs), canonical
-  unsigned char dz[kTrRows * kHidden * 2];  // dZ, rows = batch rows, K = 64
-  unsigned char dzt[kHidden * kTrRows * 2]; // dZ^T, rows = outputs, K = 128 batch rows
-  unsigned char at[kIn * kTrRows * 2];      // A_prev^T, rows = inputs (128), K = 128 batch rows
-  uint64_t bar;
-  uint32_t tmem;
-};
-constexpr size_t kTrBwdSmemBytes = sizeof(TrBwdSmem) + 1024;
-
-__device__ __forceinline__ void st_bf16(unsigned char* base, uint32_t off, uint32_t bits16) {
-  *reinterpret_cast<uint16_t*>(base + off) = (uint16_t)bits16;
-}
-
-// Backward through hidden layer `layer` (0-based) over 128-row tiles:
-//   dZ      = dA * softplus'(Z)                      (FP32, then BF16)
-//   dA_prev = dZ W          (layers > 0)            TMEM columns [0, 64)
-//   dW^T   += A_prev^T dZ   over the CTA's tiles     TMEM columns [64, 128)
-// The bias gradient rides in dW^T: the A_prev^T row just past the inputs
-// (row 64; row 99, an always-zero feature, for the first layer) is all ones,
-// so that accumulator row is sum_b dZ.  The CTA's dW, db go to its slot of
-// the partial-gradient buffer.
-__global__ void __launch_bounds__(kTrRows) k_tc_train_bwd(int layer,
-                                                          const unsigned char* __restrict__ pack,
-                                                          TrainBufs tb,
-                                                          const float* __restrict__ da_in,
-                                                          float* __restrict__ da_out,
-                                                          uint32_t batch, int* __restrict__ err) {
-  extern __shared__ unsigned char smem_raw[];
-  TrBwdSmem& s = *reinterpret_cast<TrBwdSmem*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int row = threadIdx.x;
-  const uint32_t Kin = layer == 0 ? kIn : kHidden;
-  const uint32_t ones_row = layer == 0 ? 99u : (uint32_t)kHidden;
-  const uint32_t one = 0x3F80u;  // BF16 1.0
-  if (layer > 0)
-    for (uint32_t i = row; i < kPackWh / 16; i += kTrRows)
-      reinterpret_cast<uint4*>(s.wt)[i] = __ldg(
-          reinterpret_cast<const uint4*>(pack + kPackWBytes + (layer - 1) * kPackWh) + i);
-  // rows of A_prev^T past the inputs: the ones row, then zeros (hidden layers)
-  if (layer > 0)
-    for (uint32_t k = kHidden; k < (uint32_t)kIn; ++k)
-      st_bf16(s.at, canon_off(k, row, kTrRows), k == ones_row ? one : 0u);
-  if (row == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s.bar)));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if ((row >> 5) == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_addr(&s.tmem)),
-                 "r"(128));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
-  fence_before();
-  __syncthreads();
-  fence_after();
-  const uint32_t lane_off = (32u * (uint32_t)(row >> 5)) << 16;
-  uint32_t phase = 0;
-  bool ok = true, first = true;
-  const uint32_t tiles = batch / kTrRows;
-  for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-    size_t b = (size_t)tile * kTrRows + row;
-    const float4* dg = reinterpret_cast<const float4*>(da_in + b * kHidden);
-    const float4* zg = reinterpret_cast<const float4*>(tb.z[layer] + b * kHidden);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {  // 8 dZ values per 16-byte chunk
-      float dz[8];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float4 dd = dg[2 * c + h], zz = zg[2 * c + h];
-        dz[4 * h] = dd.x * softplus_approx_deriv(zz.x);
-        dz[4 * h + 1] = dd.y * softplus_approx_deriv(zz.y);
-        dz[4 * h + 2] = dd.z * softplus_approx_deriv(zz.z);
-        dz[4 * h + 3] = dd.w * softplus_approx_deriv(zz.w);
-      }
-      uint32_t p0 = pack_bf16x2(dz[0], dz[1]), p1 = pack_bf16x2(dz[2], dz[3]);
-      uint32_t p2 = pack_bf16x2(dz[4], dz[5]), p3 = pack_bf16x2(dz[6], dz[7]);
-      store_chunk(s.dz, row, 8 * c, kHidden, p0, p1, p2, p3);
-      uint32_t pk[4] = {p0, p1, p2, p3};
-#pragma unroll
-      for (int e = 0; e < 8; ++e)
-        st_bf16(s.dzt, canon_off(8 * c + e, row, kTrRows), (pk[e >> 1] >> (16 * (e & 1))) & 0xFFFFu);
-    }
-    const uint4* ag = layer == 0 ? reinterpret_cast<const uint4*>(tb.x0 + b * kIn)
-                                 : reinterpret_cast<const uint4*>(tb.a[layer - 1] + b * kHidden);
-    for (uint32_t c = 0; c < Kin / 8; ++c) {
-      uint4 u = ag[c];
-      uint32_t w4[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        uint32_t k = 8 * c + e;
-        uint32_t v = (w4[e >> 1] >> (16 * (e & 1))) & 0xFFFFu;
-        st_bf16(s.at, canon_off(k, row, kTrRows), k == ones_row ? one : v);
-      }
-    }
-    fence_async_smem();
-    fence_before();
-    __syncthreads();
-    fence_after();
-    if (row == 0) {
-      if (layer > 0)
-        mma_chain(s.tmem, smem_addr(s.dz), kHidden, smem_addr(s.wt), kHidden, kHidden / 16, false);
-      mma_chain(s.tmem + 64u, smem_addr(s.at), kTrRows, smem_addr(s.dzt), kTrRows, kTrRows / 16,
-                !first);
-      mma_commit(&s.bar);
-    }
-    ok = __syncthreads_and(mbar_wait(&s.bar, phase) && ok);  // CTA-uniform
-    phase ^= 1u;
-    fence_after();
-    if (layer > 0) {
-      float4* og = reinterpret_cast<float4*>(da_out + b * kHidden);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        float acc[32];
-        tmem_ld32(s.tmem + lane_off + 32u * (uint32_t)half, acc);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          og[8 * half + j] = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
-      }
-    }
-    fence_before();
-    __syncthreads();  // the next tile overwrites the operands and dA_prev
-    fence_after();
-    first = false;
-  }
-  // this CTA's weight and bias gradients: TMEM lane = input index k', column = output n
-  float* pp = tb.part + (size_t)blockIdx.x * kNumParams;
-  const uint32_t k = (uint32_t)row;
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    float acc[32];
-    if (!first) {
-      tmem_ld32(s.tmem + lane_off + 64u + 32u * (uint32_t)half, acc);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) acc[j] = 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      uint32_t n = 32u * (uint32_t)half + (uint32_t)j;
-      if (k == ones_row)
-        pp[b_off(layer) + n] = acc[j];
-      if (k < Kin) pp[w_off(layer) + n * Kin + k] = k == ones_row ? 0.f : acc[j];
-    }
-  }
-  if (!ok && row == 0) atomicExch(err, 1);
-  fence_before();
-  __syncthreads();
-  fence_after();
-  if ((row >> 5) == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem), "r"(128));
+  if (tid < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem),
+                 "r"(kTrainCols));
 }
 
 // ------------------------------------------------------------- tracing
@@ -1622,21 +1642,19 @@ struct re_nsdf {
   re::nsdf::InputMap map;
   uint32_t seed = 1;
   float* params = nullptr;  // [kNumParams]
-  float* grad = nullptr;
   float* adam_m = nullptr;
   float* adam_v = nullptr;
   unsigned char* pack = nullptr;
   bool pack_valid = false;
-  uint32_t* step_ctr = nullptr;
+  uint32_t* step_ctr = nullptr;  // [0] steps done [1] reduction blocks done
   float4* data = nullptr;
   uint32_t npts = 0;
-  // training buffers for `batch` rows
+  // partial gradients of the training CTAs, for `batch` rows
   uint32_t batch = 0;
-  re::nsdf::TrainBufs tb{};
+  float* part = nullptr;
+  int train_grid = 0;
   float* loss_hist = nullptr;
   uint32_t loss_cap = 0;
-  unsigned char* train_pack = nullptr;  // BF16 weights of the training kernels
-  int fwd_grid = 0, bwd_grid = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   float graph_lr = -1.f;
@@ -1667,67 +1685,22 @@ void free_train(re_nsdf* s) {
   if (s->graph) cudaGraphDestroy(s->graph);
   s->graph_exec = nullptr;
   s->graph = nullptr;
-  cudaFree(s->tb.x0);
-  for (int l = 0; l < 4; ++l) cudaFree(s->tb.z[l]);
-  for (int l = 0; l < 3; ++l) cudaFree(s->tb.a[l]);
-  cudaFree(s->tb.da);
-  cudaFree(s->tb.da2);
-  cudaFree(s->tb.part);
-  cudaFree(s->tb.part_head);
-  cudaFree(s->train_pack);
-  s->train_pack = nullptr;
-  s->tb = TrainBufs{};
+  cudaFree(s->part);
+  s->part = nullptr;
   s->batch = 0;
 }
 
-// Persistent grids of the training kernels: as many CTAs per SM as shared
-// memory holds (the occupancy API answers 1 for these tensor-memory kernels,
-// measured, where the SM fits 2 forward or 3 backward CTAs), and never more
-// than tensor memory holds (512 columns: 64 per forward CTA, 128 per
-// backward CTA), so that no tcgen05.alloc has to wait.
-template <typename K>
-int train_grid(K kernel, size_t smem, int tmem_cols, uint32_t tiles) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTrRows, smem) !=
-          cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
-  int dev = 0, smem_sm = 0, reserved = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess &&
-      cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) ==
-          cudaSuccess &&
-      cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) ==
-          cudaSuccess)
-    per_sm = std::max(per_sm, smem_sm / (int)(smem + (size_t)reserved));
-  per_sm = std::min(per_sm, 512 / tmem_cols);
-  return (int)std::min<uint32_t>(tiles, (uint32_t)(per_sm * sm_count()));
-}
-
+// One CTA per SM (512 tensor-memory columns), every CTA with the same number
+// of tiles as far as they go round.
 re_status alloc_train(re_nsdf* s, uint32_t batch) {
   if (s->batch == batch) return RE_OK;
   free_train(s);
-  // the whole shared-memory carveout, so that 2-3 of these 75 KB CTAs fit on
-  // an SM (measured: the default carveout held one, 4 warps per SM)
-  RE_CUDA(cudaFuncSetAttribute(k_tc_train_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kTrFwdSmemBytes));
-  RE_CUDA(cudaFuncSetAttribute(k_tc_train_fwd, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               100));
-  RE_CUDA(cudaFuncSetAttribute(k_tc_train_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kTrBwdSmemBytes));
-  RE_CUDA(cudaFuncSetAttribute(k_tc_train_bwd, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               100));
-  size_t B = batch;
-  uint32_t tiles = batch / kTrRows;
-  s->fwd_grid = train_grid(k_tc_train_fwd, kTrFwdSmemBytes, 64, tiles);
-  s->bwd_grid = train_grid(k_tc_train_bwd, kTrBwdSmemBytes, 128, tiles);
-  RE_CUDA(cudaMalloc(&s->tb.x0, B * kIn * 2));
-  for (int l = 0; l < 4; ++l) RE_CUDA(cudaMalloc(&s->tb.z[l], B * kHidden * 4));
-  for (int l = 0; l < 3; ++l) RE_CUDA(cudaMalloc(&s->tb.a[l], B * kHidden * 2));
-  RE_CUDA(cudaMalloc(&s->tb.da, B * kHidden * 4));
-  RE_CUDA(cudaMalloc(&s->tb.da2, B * kHidden * 4));
-  RE_CUDA(cudaMalloc(&s->tb.part, (size_t)s->bwd_grid * kNumParams * 4));
-  RE_CUDA(cudaMalloc(&s->tb.part_head, (size_t)tiles * (kHidden + 2) * 4));
-  RE_CUDA(cudaMalloc(&s->train_pack, kTrPackBytes));
+  RE_CUDA(cudaFuncSetAttribute(k_tc_train, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kTrainSmemBytes));
+  const uint32_t tiles = batch / kTrRows;
+  const uint32_t rounds = (tiles + (uint32_t)sm_count() - 1u) / (uint32_t)sm_count();
+  s->train_grid = (int)((tiles + rounds - 1u) / rounds);
+  RE_CUDA(cudaMalloc(&s->part, (size_t)s->train_grid * kPartStride * 4));
   s->batch = batch;
   return RE_OK;
 }
@@ -1742,33 +1715,17 @@ re_status check(const re_nsdf* s, const char* fn) {
   return RE_OK;
 }
 
-// One optimisation step on a batch (sampled from s->data, or given points
-// when direct): pack, forward + L1 loss, backward, reduction, optional Adam.
+// One pass over a batch (sampled from s->data, or given points when direct):
+// forward, L1 loss, backward and the reduction, whose sums go to `grad`, or
+// into an Adam step when grad is null.
 re_status enqueue_step(re_nsdf* s, const float4* data, uint32_t npts, int direct, float lr,
-                       bool adam, float* pred, cudaStream_t st) {
-  uint32_t B = s->batch;
-  uint32_t nfwd = B / kTrRows, nbwd = (uint32_t)s->bwd_grid;
-  k_pack_train<<<(3 * kHidden * kHidden + 255) / 256, 256, 0, st>>>(s->params, s->train_pack);
-  k_tc_train_fwd<<<s->fwd_grid, kTrRows, kTrFwdSmemBytes, st>>>(
-      s->map, data, npts, s->step_ctr, s->seed, direct, s->train_pack, s->params, s->tb, B, pred,
-      s->err);
-  // backward: da holds dA4; alternate da / da2
-  float* din = s->tb.da;
-  float* dout = s->tb.da2;
-  for (int l = 3; l >= 0; --l) {
-    k_tc_train_bwd<<<s->bwd_grid, kTrRows, kTrBwdSmemBytes, st>>>(l, s->train_pack, s->tb, din,
-                                                                  l > 0 ? dout : nullptr, B,
-                                                                  s->err);
-    std::swap(din, dout);
-  }
-  k_reduce<<<(kNumParams + 2 + 255) / 256, 256, 0, st>>>(s->tb, nbwd, nfwd, s->grad,
-                                                         adam ? s->loss_hist : nullptr,
-                                                         s->step_ctr, B);
-  if (adam) {
-    k_adam<<<(kNumParams + 255) / 256, 256, 0, st>>>(s->params, s->grad, s->adam_m, s->adam_v,
-                                                     s->step_ctr, lr);
-    k_step_inc<<<1, 1, 0, st>>>(s->step_ctr);
-  }
+                       float* grad, float* pred, cudaStream_t st) {
+  const uint32_t B = s->batch;
+  k_tc_train<<<s->train_grid, kTrainThreads, kTrainSmemBytes, st>>>(
+      s->map, data, npts, s->step_ctr, s->seed, direct, s->params, s->part, B, pred, s->err);
+  k_train_reduce<<<(kPartStride + 31) / 32, 32 * kReduceWarps, 0, st>>>(
+      s->part, (uint32_t)s->train_grid, grad, s->params, grad ? nullptr : s->adam_m, s->adam_v,
+      s->loss_hist, s->step_ctr, lr, B);
   RE_CHECK_LAUNCH("nsdf training step launch");
   return RE_OK;
 }
@@ -1896,7 +1853,6 @@ RE_API re_status re_nsdf_create(const re_nsdf_config* cfg, re_nsdf** out) {
   s->map.f0 = cfg->f0;
   s->seed = cfg->seed;
   if (e == cudaSuccess) e = cudaMalloc(&s->params, kNumParams * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&s->grad, kNumParams * 4);
   if (e == cudaSuccess) e = cudaMalloc(&s->adam_m, kNumParams * 4);
   if (e == cudaSuccess) e = cudaMalloc(&s->adam_v, kNumParams * 4);
   if (e == cudaSuccess) e = cudaMalloc(&s->pack, re::nsdf::kPackBytes);
@@ -1936,7 +1892,6 @@ RE_API re_status re_nsdf_destroy(re_nsdf* s) {
   if (!s) return RE_OK;
   re::free_train(s);
   cudaFree(s->params);
-  cudaFree(s->grad);
   cudaFree(s->adam_m);
   cudaFree(s->adam_v);
   cudaFree(s->pack);
@@ -2051,7 +2006,7 @@ RE_API re_status re_nsdf_train(re_nsdf* s, uint32_t steps, uint32_t batch, float
     RE_CUDA(cudaStreamCreateWithFlags(&cap_stream, cudaStreamNonBlocking));
     cudaError_t e = cudaStreamBeginCapture(cap_stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      st = re::enqueue_step(s, s->data, s->npts, 0, lr, true, nullptr, cap_stream);
+      st = re::enqueue_step(s, s->data, s->npts, 0, lr, nullptr, nullptr, cap_stream);
       e = cudaStreamEndCapture(cap_stream, &s->graph);
     }
     if (e == cudaSuccess && st == RE_OK) e = cudaGraphInstantiate(&s->graph_exec, s->graph, 0);
@@ -2087,9 +2042,8 @@ RE_API re_status re_nsdf_loss_grad(re_nsdf* s, const float* d_xyzl, uint32_t n, 
   st = re::alloc_train(s, n);
   if (st != RE_OK) return st;
   RE_CUDA(cudaMemsetAsync(s->err, 0, 4, cs));
-  st = re::enqueue_step(s, reinterpret_cast<const float4*>(d_xyzl), n, 1, 0.f, false, d_pred, cs);
+  st = re::enqueue_step(s, reinterpret_cast<const float4*>(d_xyzl), n, 1, 0.f, d_grad, d_pred, cs);
   if (st != RE_OK) return st;
-  RE_CUDA(cudaMemcpyAsync(d_grad, s->grad, re::nsdf::kNumParams * 4, cudaMemcpyDeviceToDevice, cs));
   int herr = 0;
   RE_CUDA(cudaMemcpyAsync(&herr, s->err, 4, cudaMemcpyDeviceToHost, cs));
   RE_CUDA(cudaStreamSynchronize(cs));

@@ -1,7 +1,7 @@
 // Neural SDF surrogate of the volumetric terrain: shared definitions of the
-// network used by the training kernels (SIMT FP32 with BF16-rounded weights
-// and activations) and the tensor-core inference kernels (BF16 operands in
-// shared memory, FP32 accumulators in tensor memory).
+// network used by the training and inference kernels (both on the tensor
+// cores: BF16 operands in shared memory, FP32 accumulators in tensor memory)
+// and the FP32 reference evaluation.
 //
 // Network: 3 -> 128 Fourier features -> 64 -> 64 -> 64 -> 64 -> 1, softplus
 // after each hidden layer.  The reference has no learned component; this is
@@ -95,23 +95,9 @@ __device__ __forceinline__ float lp_poly(float u) {
   p = __fmaf_rn(u, p, 0.9998613f);
   return u * p;
 }
-__device__ __forceinline__ float lp_poly_deriv(float u) {
-  float p = __fmaf_rn(u, 6.0f * -0.017806457f, 5.0f * 0.083866805f);
-  p = __fmaf_rn(u, p, 4.0f * -0.19167475f);
-  p = __fmaf_rn(u, p, 3.0f * 0.31643057f);
-  p = __fmaf_rn(u, p, 2.0f * -0.49753284f);
-  p = __fmaf_rn(u, p, 0.9998613f);
-  return p;
-}
 __device__ __forceinline__ float softplus_approx(float x) {
   float u = __expf(-fabsf(x));
   return fmaxf(x, 0.0f) + lp_poly(u);
 }
-__device__ __forceinline__ float softplus_approx_deriv(float x) {
-  float u = __expf(-fabsf(x));
-  float g = u * lp_poly_deriv(u);
-  return x > 0.0f ? 1.0f - g : g;
-}
-
 }  // namespace nsdf
 }  // namespace re

@@ -245,3 +245,38 @@ def test_trace_parameter_checks(cuda):
                     phase="exact")
         with pytest.raises(rb.RayEngineError):
             m.trace(field, tp, cam, tc.width + 8, tc.height, phase="exact")
+
+
+@pytest.mark.parametrize("n", [1024, 37888, 38912, 131072])
+def test_gradient_is_the_mean_over_the_halves(cuda, n):
+    """Tiles split over the CTAs: a few, one each on 148 SMs (18,944 rows),
+    two each, several.  Halving the batch doubles every dZ exactly, so the
+    whole batch's gradient differs from the mean of its halves' only in the
+    order of FP32 sums: at most n additions of relative error 2^-24, in
+    practice their square root."""
+    with _model() as m:
+        pts = _pts(n, 4)
+        labels = np.random.default_rng(5).normal(0, 1, n).astype(np.float32)
+        xyzl = torch.from_numpy(np.concatenate([pts, labels[:, None]], 1)).cuda()
+        g, pred = m.loss_grad(xyzl)
+        h = n // 2
+        g0, p0 = m.loss_grad(xyzl[:h].contiguous())
+        g1, p1 = m.loss_grad(xyzl[h:].contiguous())
+        assert torch.equal(pred, torch.cat([p0, p1]))
+        mean = 0.5 * (g0.double() + g1.double())
+        err = (g.double() - mean).norm() / mean.norm()
+        assert err < n ** 0.5 * 2.0 ** -24, err
+
+
+def test_training_steps_follow_one_another(cuda):
+    """Two calls of one step and one call of two leave the same parameters
+    and losses: the reduction's last block advances the step count."""
+    tc = rb.configs.TerrainConfig(width=192, height=108)
+    out = []
+    for calls in ((2, 1), (1, 2)):
+        with _model() as m:
+            m.generate(tc.params(), tc.camera(), tc.width, tc.height, 1 << 14, seed=9)
+            losses = np.concatenate([m.train(calls[1], batch=512) for _ in range(calls[0])])
+            out.append((losses, m.get_params()))
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
