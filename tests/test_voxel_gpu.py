@@ -73,3 +73,45 @@ def test_brush_edits_match_oracle(cuda):
     # the edits changed the field
     assert not np.array_equal(grid, po.voxel_bake(po.perm(tc.seed), tc.octaves, tc.scale,
                                                   tc.amplitude, DIM, SP, ORG))
+
+
+@pytest.mark.parametrize("quality", [rb.VOXEL_LOW, rb.VOXEL_MEDIUM, rb.VOXEL_HIGH])
+@pytest.mark.parametrize("dim", [(2, 2, 2), (3, 5, 4), (4, 4, 4), (5, 4, 7), (33, 17, 9)])
+def test_small_grids_and_ragged_frames(cuda, dim, quality):
+    """Grids with no cell, one cell and a few whose neighbours all lie inside;
+    points on voxels, across every face and far outside; frames from 2x2 to
+    several ragged tiles.  Bit for bit against the oracle."""
+    rng = np.random.default_rng(dim[0])
+    sp, org = (0.5, 0.75, 0.4), (-1.0, 0.5, 2.0)
+    nx, ny, nz = dim
+    y = np.arange(ny, dtype=np.float32)[None, :, None] - 0.45 * ny
+    data = np.zeros((nz, ny, nx, 2), np.float32)
+    data[..., 0] = 0.5 * y + rng.normal(0, 0.1, (nz, ny, nx)).astype(np.float32)
+    g = rb.VoxelGrid(dim, sp, org, data)
+    grid = g.data.cpu().numpy()
+    ext = np.array(dim, np.float64) * sp
+    pts = rng.uniform(np.array(org) - 2.5, np.array(org) + ext + 2.5, (4000, 3))
+    on = np.stack([rng.integers(-3, d + 3, 500) * np.float32(s) + np.float32(o)
+                   for d, s, o in zip(dim, sp, org)], 1)
+    pts = np.concatenate([pts, on, [[1e9, -1e9, 1e30]]]).astype(np.float32)
+    got = g.sample(torch.from_numpy(pts).cuda(), quality).cpu().numpy()
+    want = po.voxel_sample(grid, dim, sp, org, quality, pts)
+    # the C oracle's conversion to int is defined below 2^31 only: the point
+    # at z = 1e30 is looked up (a voxel of the grid) but has no oracle value
+    fits = np.abs((pts.astype(np.float64) - org) / sp).max(1) < 2.0 ** 31 - 4.0
+    assert np.array_equal(fits, np.arange(len(pts)) < len(pts) - 1)
+    assert np.array_equal(got.view(np.uint32)[fits], want.view(np.uint32)[fits])
+    assert np.isfinite(got).all()
+    march = rb.sdf_params(step_factor=0.6, eps=1e-3, tmax=100.0, max_steps=64)
+    mid = np.array(org) + 0.5 * ext
+    for w, h in ((2, 2), (9, 5), (70, 43)):
+        cam = rb.build_camera(tuple(mid + (0.3, 4.0, -5.0)), tuple(mid), (60.0, 45.0))
+        u = g.trace(quality, march, cam, w, h).cpu().numpy().view(np.uint32).reshape(-1, 8)
+        ref = po.voxel_trace(grid, dim, sp, org, quality, 0.6, 1e-3, 100.0, 64, cam, w, h)
+        assert np.array_equal(u[:, 7], ref["status"])
+        assert np.array_equal(u[:, 6], ref["steps"])
+        hit = ref["status"] == 1
+        assert np.array_equal(u[hit, 0:3], ref["pos"][hit].view(np.uint32))
+        # a flat neighbourhood (nearest voxel) has no normal: NaN on both sides
+        assert np.array_equal(u[hit, 3:6].view(np.float32), ref["normal"][hit], equal_nan=True)
+        assert not u[~hit, 0:6].any()
