@@ -107,9 +107,10 @@ typedef struct re_tuning {
   uint32_t refill_min;       /* idle lanes before a warp claims new secondary rays, 1..32 */
   uint32_t ray_refill_min;   /* the same for primary and caller rays (re_trace_primary,
                                 re_count_primary, re_trace_rays), 1..32; 32 (default):
-                                each lane runs its ray to the end, no refill */
+                                chosen by the number of rays */
   uint32_t ray_lanes;        /* lanes per primary ray in re_trace_primary: 1 (default; 0
-                                reads as 1), 2, 4 or 8.  Above 1 the lanes of a ray split
+                                reads as 1; with ray_refill_min 32: chosen by the number of
+                                rays and the tree's leaves), 2, 4 or 8.  Above 1 the lanes of a ray split
                                 each leaf's triangle tests (same hits); it shortens the
                                 longest walks of frames too small to fill the GPU.  32:
                                 one ray per lane, and the warp tests the triangles of all

@@ -192,12 +192,14 @@ __device__ __forceinline__ void trav_init(Trav& s, const KdDev& kd, V3 o, V3 d, 
 // of its lanes' bests.  The sequential acceptance rule (smaller t, or equal
 // t and smaller id, with id -1 for "no hit yet") is that same lexicographic
 // minimum, and a leaf holds each triangle once, so the merged best, its
-// slot and its leaf equal the one-lane walk's.  Closest hit only.
+// slot and its leaf equal the one-lane walk's.  Any hit: the one-lane walk
+// stops at the leaf's first accepted slot, so each lane stops at its own and
+// the group keeps the smallest.
 template <int MODE, bool ANYHIT, bool COUNT, uint32_t G = 1>
 __device__ __forceinline__ void trav_step(Trav& s, const KdDev& kd, const uint2* snodes,
                                           Counters& c) {
-  static_assert(G == 1 || G == 2 || G == 4 || G == 8, "lanes per ray: 1, 2, 4 or 8");
-  static_assert(G == 1 || (!ANYHIT && !COUNT), "shared rays: closest hit, no counters");
+  static_assert(G >= 1 && G <= 32 && (G & (G - 1u)) == 0u, "lanes per ray: a power of two");
+  static_assert(G == 1 || !COUNT, "shared rays: no counters");
   const uint32_t sub = G > 1 ? (threadIdx.x & (G - 1u)) : 0u;
   const V3 o = s.o, d = s.d, inv = s.inv;
   const float t_entry = s.t_entry;
@@ -219,7 +221,7 @@ __device__ __forceinline__ void trav_step(Trav& s, const KdDev& kd, const uint2*
   // closest-hit walks fetch that triangle together with the leaf record
   // (measured: any-hit walks, which often stop at the first hit of a leaf,
   // run faster without the extra live registers)
-  constexpr bool kEarlyFirst = !ANYHIT;
+  constexpr bool kEarlyFirst = !ANYHIT || G > 1;
   uint32_t first = nd.x & 0x7FFFFFFFu;
   // this lane's first slot; with G > 1 it may lie past the leaf (fetched
   // only inside the triangle array, and used only if the leaf reaches it)
@@ -273,13 +275,14 @@ __device__ __forceinline__ void trav_step(Trav& s, const KdDev& kd, const uint2*
         s.best_leaf = node;
         if (ANYHIT) {
           s.live = false;
-          return;
+          if (G == 1) return;
+          break;
         }
       }
     }
   }
   if (G > 1) {
-    const uint32_t gmask = ((1u << G) - 1u) << ((threadIdx.x & 31u) & ~(G - 1u));
+    const uint32_t gmask = (0xFFFFFFFFu >> (32u - G)) << ((threadIdx.x & 31u) & ~(G - 1u));
 #pragma unroll
     for (uint32_t off = 1; off < G; off <<= 1) {
       float ot = __shfl_xor_sync(gmask, s.best_t, off);
@@ -288,7 +291,8 @@ __device__ __forceinline__ void trav_step(Trav& s, const KdDev& kd, const uint2*
       float ov = __shfl_xor_sync(gmask, s.best_v, off);
       uint32_t oref = __shfl_xor_sync(gmask, s.best_ref, off);
       // the other lane differs only if it accepted a triangle of this leaf
-      if (ot < s.best_t || (ot == s.best_t && oid < s.best_id)) {
+      // (any hit: an empty best has the largest slot)
+      if (ANYHIT ? oref < s.best_ref : ot < s.best_t || (ot == s.best_t && oid < s.best_id)) {
         s.best_t = ot;
         s.best_id = oid;
         s.best_u = ou;
@@ -296,6 +300,10 @@ __device__ __forceinline__ void trav_step(Trav& s, const KdDev& kd, const uint2*
         s.best_ref = oref;
         s.best_leaf = node;
       }
+    }
+    if (ANYHIT && s.best_id >= 0) {
+      s.live = false;
+      return;
     }
   }
   if (face < 0) {
@@ -334,7 +342,15 @@ __device__ __forceinline__ void trav_step(Trav& s, const KdDev& kd, const uint2*
 // smaller t, or equal t and smaller id once a hit exists; a leaf holds each
 // triangle once).  The tester whose key is the minimum writes u, v and the
 // triangle slot for its owner.  key and rec: this warp's 32 slots.
-template <int MODE>
+//
+// ANYHIT: the one-lane walk stops at the first slot of the leaf it accepts,
+// so the key is the slot (its minimum over the accepting testers), and the
+// tester that holds it writes the hit.
+//
+// INCOHERENT: the walk refills its lanes from rays in no order, where sharing
+// a leaf's tests pays a little sooner (measured on B200, 300,007 random rays
+// in the 4096-triangle soup 257 -> 235 us; 2048x2048 frames 1.5 % slower).
+template <int MODE, bool ANYHIT = false, bool INCOHERENT = false>
 __device__ __forceinline__ void trav_step_warp(Trav& s, const KdDev& kd, const uint2* snodes,
                                                unsigned long long* key, float4* rec) {
   const uint32_t lane = threadIdx.x & 31u;
@@ -369,18 +385,49 @@ __device__ __forceinline__ void trav_step_warp(Trav& s, const KdDev& kd, const u
     if (tz < texit) { texit = tz; face = d.z > 0.0f ? 5 : 4; }
     rope = face >= 0 ? __ldg(reinterpret_cast<const int32_t*>(L + 2) + face) : -1;
   }
-  uint32_t incl = count;
-#pragma unroll
-  for (uint32_t off = 1; off < 32; off <<= 1) {
-    uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, off);
-    if (lane >= off) incl += y;
+  // Lanes that share leaves (coherent rays) leave nothing to share out: their
+  // longest list, one test after another, is then the shorter way.
+  const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, count);
+  const uint32_t longest = __reduce_max_sync(0xFFFFFFFFu, count);
+  const uint32_t rounds = (total + 31u) / 32u;
+  const bool together =
+      INCOHERENT ? 5u * rounds < 4u * longest : 3u * rounds + 1u < 2u * longest;
+  if (!together) {
+    for (uint32_t i = first, end = first + count; i < end; ++i) {
+      const float4* T = kd.tris + 3 * (size_t)i;
+      const float4 T0 = __ldg(T), T1 = __ldg(T + 1), T2 = __ldg(T + 2);
+      const int32_t id = __float_as_int(T0.w);
+      float t, u, v;
+      if (ray_tri<MODE>(o, d, T0, T1, T2, t, u, v) &&
+          (t < s.best_t || (t == s.best_t && id < s.best_id && s.best_id >= 0))) {
+        s.best_t = t;
+        s.best_id = id;
+        s.best_u = u;
+        s.best_v = v;
+        s.best_ref = i;
+        s.best_leaf = node;
+        if (ANYHIT) {
+          s.live = false;
+          break;
+        }
+      }
+    }
   }
-  const uint32_t excl = incl - count, total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-  if (total > 0u) {
+  uint32_t incl = count;
+  if (together) {
+#pragma unroll
+    for (uint32_t off = 1; off < 32; off <<= 1) {
+      uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+      if (lane >= off) incl += y;
+    }
+  }
+  const uint32_t excl = incl - count;
+  if (together) {
     unsigned long long seed = 0ull;
     if (live) {
-      seed = ((unsigned long long)__float_as_uint(s.best_t) << 32) |
-             (uint32_t)(s.best_id >= 0 ? s.best_id : 0);
+      seed = ANYHIT ? ~0ull
+                    : ((unsigned long long)__float_as_uint(s.best_t) << 32) |
+                          (uint32_t)(s.best_id >= 0 ? s.best_id : 0);
       key[lane] = seed;
     }
     __syncwarp();
@@ -398,40 +445,51 @@ __device__ __forceinline__ void trav_step_warp(Trav& s, const KdDev& kd, const u
                      __shfl_sync(0xFFFFFFFFu, o.z, own)};
       const V3 rd = {__shfl_sync(0xFFFFFFFFu, d.x, own), __shfl_sync(0xFFFFFFFFu, d.y, own),
                      __shfl_sync(0xFFFFFFFFu, d.z, own)};
+      const float rt = ANYHIT ? __shfl_sync(0xFFFFFFFFu, s.best_t, own) : 0.f;
       bool hit = false;
       unsigned long long k = 0ull;
-      float u = 0.f, v = 0.f;
-      uint32_t ref = 0;
+      float t = 0.f, u = 0.f, v = 0.f;
+      uint32_t ref = 0, id = 0;
       if (p < total) {
         ref = ofirst + (p - oex);
         const float4* T = kd.tris + 3 * (size_t)ref;
         float4 T0 = __ldg(T), T1 = __ldg(T + 1), T2 = __ldg(T + 2);
-        float t;
-        if (ray_tri<MODE>(ro, rd, T0, T1, T2, t, u, v)) {
-          k = ((unsigned long long)__float_as_uint(t) << 32) | (uint32_t)__float_as_int(T0.w);
+        if (ray_tri<MODE>(ro, rd, T0, T1, T2, t, u, v) && (!ANYHIT || t < rt)) {
+          id = __float_as_uint(T0.w);
+          k = ANYHIT ? (unsigned long long)ref
+                     : ((unsigned long long)__float_as_uint(t) << 32) | id;
           hit = true;
           atomicMin(&key[own], k);
         }
       }
       __syncwarp();
-      if (hit && key[own] == k) rec[own] = make_float4(u, v, __uint_as_float(ref), 0.f);
+      if (hit && key[own] == k)
+        rec[own] = ANYHIT ? make_float4(u, v, t, __uint_as_float(id))
+                          : make_float4(u, v, __uint_as_float(ref), 0.f);
       __syncwarp();
     }
     if (live) {
       const unsigned long long k = key[lane];
       if (k != seed) {
         const float4 r = rec[lane];
-        s.best_t = __uint_as_float((uint32_t)(k >> 32));
-        s.best_id = (int32_t)(uint32_t)k;
         s.best_u = r.x;
         s.best_v = r.y;
-        s.best_ref = __float_as_uint(r.z);
         s.best_leaf = node;
+        if (ANYHIT) {
+          s.best_t = r.z;
+          s.best_id = __float_as_int(r.w);
+          s.best_ref = (uint32_t)k;
+          s.live = false;
+        } else {
+          s.best_t = __uint_as_float((uint32_t)(k >> 32));
+          s.best_id = (int32_t)(uint32_t)k;
+          s.best_ref = __float_as_uint(r.z);
+        }
       }
     }
     __syncwarp();
   }
-  if (!live) return;
+  if (ANYHIT ? !s.live : !live) return;
   if (face < 0) {
     s.live = false;
     return;

@@ -124,28 +124,27 @@ __global__ void __launch_bounds__(256, 6) k_primary_tiles(KdDev kd, CamDev cam, 
   }
 }
 
-// Primary rays with G lanes per ray (ray_lanes 2, 4 or 8): persistent warps
-// over tiles of 32 / G pixels, 4 wide; the lanes of a ray split each leaf's
-// triangle tests (trav_step with G).  For frames whose pass time is set by
-// the longest walks rather than by throughput (a 512x512 frame of a 2^20-
-// triangle soup takes as long as a 64x64 one), the G-fold shorter test
-// chain per leaf shortens the critical path.
+// Primary rays with G lanes per ray: persistent warps over tiles of 32 / G
+// pixels, up to 4 wide; the lanes of a ray split each leaf's triangle tests
+// (trav_step with G).  For frames whose pass time is set by the longest walks
+// rather than by throughput: the test chain of a leaf is G times shorter, and
+// a walk waits for G times fewer others in its warp (ray_form has the sizes).
 template <int MODE, uint32_t G>
 __global__ void __launch_bounds__(256, 6) k_primary_lanes(KdDev kd, CamDev cam, uint32_t w,
                                                        uint32_t h, re_hit* __restrict__ out,
                                                        uint4* __restrict__,
                                                        uint32_t* __restrict__ tile_counter,
                                                        uint32_t) {
-  constexpr uint32_t kRows = 32u / G / 4u;  // tile height; 4 pixels wide
+  constexpr uint32_t kWide = G <= 8u ? 4u : 32u / G, kRows = 32u / G / kWide;  // the warp's tile
   extern __shared__ uint2 snodes[];
   stage_nodes(kd, snodes);
   const uint32_t lane = threadIdx.x & 31u, r = lane / G;
-  const uint32_t tiles_x = (w + 3) / 4, tiles = tiles_x * ((h + kRows - 1) / kRows);
+  const uint32_t tiles_x = (w + kWide - 1) / kWide, tiles = tiles_x * ((h + kRows - 1) / kRows);
   for (;;) {
     uint32_t tile = warp_fetch(tile_counter);
     if (tile >= tiles) break;
-    uint32_t x = (tile % tiles_x) * 4 + (r & 3u);
-    uint32_t y = (tile / tiles_x) * kRows + (r >> 2);
+    uint32_t x = (tile % tiles_x) * kWide + (r % kWide);
+    uint32_t y = (tile / tiles_x) * kRows + (r / kWide);
     if (x >= w || y >= h) continue;  // the whole group skips
     V3 o, d;
     generate_ray(cam, w, h, x, y, o, d);
@@ -279,6 +278,85 @@ __global__ void __launch_bounds__(256, 6) k_rays(KdDev kd, const float4* __restr
     store_hit(out, i, hs);
   };
   refill_walk<MODE, ANYHIT, false>(kd, snodes, n, refill_min, counter, gen, done);
+}
+
+// Caller rays with G lanes per ray, 32 / G rays to a warp (as
+// k_primary_lanes): for calls of few rays.
+template <int MODE, bool ANYHIT, uint32_t G>
+__global__ void __launch_bounds__(256, 6) k_rays_lanes(KdDev kd, const float4* __restrict__ rays,
+                                                    uint32_t n, re_hit* __restrict__ out,
+                                                    uint32_t* __restrict__ counter, uint32_t) {
+  extern __shared__ uint2 snodes[];
+  stage_nodes(kd, snodes);
+  const uint32_t lane = threadIdx.x & 31u;
+  for (;;) {
+    const uint32_t first = warp_fetch(counter) * (32u / G);
+    if (first >= n) break;
+    const uint32_t i = first + lane / G;
+    if (i >= n) continue;  // the whole group skips
+    const float4 R0 = __ldg(&rays[2 * (size_t)i]), R1 = __ldg(&rays[2 * (size_t)i + 1]);
+    Trav s;
+    Counters c = {0, 0, 0, 0};
+    trav_init(s, kd, v3(R0.x, R0.y, R0.z), v3(R1.x, R1.y, R1.z), R0.w, 0u);
+    while (s.live) trav_step<MODE, ANYHIT, false, G>(s, kd, snodes, c);
+    HitState hs;
+    trav_result(s, hs);
+    if ((lane & (G - 1u)) == 0u) store_hit(out, i, hs);
+  }
+}
+
+// Caller rays, lane refill, the warp testing the triangles of all its lanes'
+// leaves together (trav_step_warp): incoherent rays end at very different
+// leaves, and here a lane whose ray has ended takes a new one while the
+// tests of the others' leaves still use every lane.
+template <int MODE, bool ANYHIT>
+__global__ void __launch_bounds__(256, 4) k_rays_warp(KdDev kd, const float4* __restrict__ rays,
+                                                   uint32_t n, re_hit* __restrict__ out,
+                                                   uint32_t* __restrict__ counter,
+                                                   uint32_t refill_min) {
+  extern __shared__ uint2 snodes[];
+  __shared__ unsigned long long wkey[8][32];
+  __shared__ float4 wrec[8][32];
+  stage_nodes(kd, snodes);
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  Trav s;
+  s.live = false;
+  uint32_t cur = 0;
+  bool exhausted = false;
+  for (;;) {
+    const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !s.live);
+    const uint32_t nidle = __popc(idle);
+    if (!exhausted && nidle >= refill_min) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(counter, nidle);
+      base = __shfl_sync(0xFFFFFFFFu, base, 0);
+      if (base + nidle >= n) exhausted = true;
+      if (!s.live) {
+        const uint32_t i = base + __popc(idle & ((1u << lane) - 1u));
+        if (i < n) {
+          const float4 R0 = __ldg(&rays[2 * (size_t)i]), R1 = __ldg(&rays[2 * (size_t)i + 1]);
+          cur = i;
+          trav_init(s, kd, v3(R0.x, R0.y, R0.z), v3(R1.x, R1.y, R1.z), R0.w, 0u);
+          if (!s.live) {
+            HitState hs;
+            trav_result(s, hs);
+            store_hit(out, cur, hs);
+          }
+        }
+      }
+    }
+    const bool live = s.live;
+    if (__ballot_sync(0xFFFFFFFFu, live) == 0u) {
+      if (exhausted) break;
+      continue;
+    }
+    trav_step_warp<MODE, ANYHIT, true>(s, kd, snodes, wkey[warp], wrec[warp]);
+    if (live && !s.live) {
+      HitState hs;
+      trav_result(s, hs);
+      store_hit(out, cur, hs);
+    }
+  }
 }
 
 // Pixel mask bit of the AO frame: one of the pixel's rays (primary, shadow
@@ -651,9 +729,43 @@ re_status create_from_packed(const float* tris, uint32_t n, const re_kd_params* 
 namespace re {
 namespace {
 
-// One primary pass: G lanes per ray when ray_lanes > 1 (hits only), else
-// whole-warp tiles when ray_refill_min is 32, else lane refill.  All
-// kernels take the same arguments.
+// The form of a ray pass: lanes per ray (1, 2, 4, 8 or kWholeWarp), or 32
+// for one ray per lane with the warp's tests together.  A tuning other than
+// the default says which (caller rays: ray_refill_min only).  By default it
+// follows the number of rays and the tree; every form finds the same hits.
+//   Few rays leave the GPU idle and their time is that of the longest walk,
+// which the other rays of its warp stretch (their descents and tests take
+// turns): give each more lanes.  Measured on B200, one lane per ray against
+// 32, 8 and 4 lanes, us per call: 64x48 frames of soups of 4096, 65,536 and
+// 262,144 triangles and of a 131,072-triangle heightfield 72, 167, 123, 108
+// -> 32, 72, 48, 60 (32 lanes); 192x192 70, 160, 120, 106 -> 45, 91, 74, 87
+// (8 lanes); 256x256 69, 172, 140, 118 -> 50, 109, 93, 97 (4 lanes).  Random
+// rays: 1000 121, 180, 141, 110 -> 38, 65, 56, 57 (32 lanes), 20,000 150,
+// 266, 190, 145 -> 71, 125, 92, 105 (8 lanes); at 60,000 four lanes are level
+// with the shared tests.
+//   More rays in a tree of long leaves share their tests (the soups hold 5.3
+// to 5.6 references per leaf; 2048x2048 481, 882, 673 -> 450, 750, 635 us,
+// 300,007 random rays 349, 509, 319 -> 235, 299, 204); where leaves are short
+// (the heightfield: 1.36, tuned to at most 2) there is little to share and
+// the plain walk stays (2048x2048 489 us against 544).
+constexpr uint32_t kWholeWarp = 64;
+uint32_t ray_form(const re_scene* s, uint32_t n, bool frame) {
+  const bool by_size = s->tune.ray_refill_min >= 32u && (!frame || s->tune.ray_lanes <= 1u);
+  if (!by_size) return frame ? s->tune.ray_lanes : 1u;
+  if (n <= 4096u) return kWholeWarp;
+  if (n <= 40960u) return 8u;
+  if (frame && n <= 81920u) return 4u;
+  return s->host.num_refs >= 3ull * s->host.num_leaves ? 32u : 1u;
+}
+
+int blocks_for(int grid, uint32_t rays, uint32_t rays_per_warp) {
+  const uint32_t warps = (rays + rays_per_warp - 1u) / rays_per_warp;
+  return (int)std::min<uint32_t>((uint32_t)grid, warps);
+}
+
+// One primary pass: G lanes per ray or the warp's tests together (ray_form;
+// hits only), else whole-warp tiles when ray_refill_min is 32, else lane
+// refill.  All kernels take the same arguments.
 template <int MODE, bool COUNT>
 re_status launch_primary(re_scene* s, const re_camera& cam, uint32_t w, uint32_t h, re_hit* out,
                          uint4* counts, cudaStream_t st) {
@@ -662,16 +774,20 @@ re_status launch_primary(re_scene* s, const re_camera& cam, uint32_t w, uint32_t
   if (COUNT) kd.entry = nullptr;
   CamDev cd = cam_view(cam);
   size_t smem = kd.stage * sizeof(uint2);
-  uint32_t refill = s->tune.ray_refill_min, lanes = COUNT ? 1u : s->tune.ray_lanes;
+  uint32_t refill = s->tune.ray_refill_min, lanes = COUNT ? 1u : ray_form(s, w * h, true);
   auto k = lanes == 2u    ? k_primary_lanes<MODE, 2>
            : lanes == 4u  ? k_primary_lanes<MODE, 4>
            : lanes == 8u  ? k_primary_lanes<MODE, 8>
+           : lanes == kWholeWarp ? k_primary_lanes<MODE, 32>
            : lanes == 32u ? k_primary_warp<MODE>
            : refill >= 32u ? k_primary_tiles<MODE, COUNT>
                            : k_primary<MODE, COUNT>;
   RE_CUDA(cudaMemsetAsync(s->d_counters, 0, RE_SCENE_RESET_BYTES, st));
   RE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k<<<grid_for(k, smem), 256, smem, st>>>(kd, cd, w, h, out, counts, s->d_counters, refill);
+  // no more blocks than warps with work: few tiles spread over the SMs
+  const uint32_t per_warp = lanes == kWholeWarp ? 1u : 32u / (lanes < 32u ? lanes : 1u);
+  k<<<blocks_for(grid_for(k, smem), w * h, per_warp), 256, smem, st>>>(kd, cd, w, h, out, counts,
+                                                                       s->d_counters, refill);
   RE_CHECK_LAUNCH(COUNT ? "re_count_primary: launch" : "re_trace_primary: launch");
   return RE_OK;
 }
@@ -681,10 +797,19 @@ re_status launch_rays(re_scene* s, const float4* rays, uint32_t n, re_hit* out, 
   KdDev kd = kd_view(s);
   size_t smem = kd.stage * sizeof(uint2);
   uint32_t refill = s->tune.ray_refill_min;
-  auto k = refill >= 32u ? k_rays_chunks<MODE, ANYHIT> : k_rays<MODE, ANYHIT>;
+  // refill thresholds of 4 to 16 idle lanes measured within 2 %; 8
+  const uint32_t lanes = ray_form(s, n, false);
+  if (lanes == 32u) refill = std::min(refill, 8u);
+  auto k = lanes == kWholeWarp ? k_rays_lanes<MODE, ANYHIT, 32>
+           : lanes == 8u       ? k_rays_lanes<MODE, ANYHIT, 8>
+           : lanes == 32u      ? k_rays_warp<MODE, ANYHIT>
+           : refill >= 32u     ? k_rays_chunks<MODE, ANYHIT>
+                               : k_rays<MODE, ANYHIT>;
   RE_CUDA(cudaMemsetAsync(s->d_counters, 0, RE_SCENE_RESET_BYTES, st));
   RE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k<<<grid_for(k, smem), 256, smem, st>>>(kd, rays, n, out, s->d_counters, refill);
+  const uint32_t per_warp = lanes == kWholeWarp ? 1u : 32u / (lanes < 32u ? lanes : 1u);
+  k<<<blocks_for(grid_for(k, smem), n, per_warp), 256, smem, st>>>(kd, rays, n, out,
+                                                                   s->d_counters, refill);
   RE_CHECK_LAUNCH("re_trace_rays: launch");
   return RE_OK;
 }

@@ -1,0 +1,94 @@
+"""The forms a ray pass takes by its number of rays and its tree (lanes per
+ray, shared tests, one lane per ray), at the sizes where they change, bit for
+bit: frames and closest-hit rays against the oracle, any-hit rays against the
+lane-refill walk (the oracle's any-hit triangle may differ)."""
+import numpy as np
+import pytest
+import torch
+
+import rayengine_b200 as rb
+from oracle import pyoracle as po
+
+pytestmark = pytest.mark.gpu
+
+
+def _kd(sc):
+    st = sc.stats()
+    nodes, leaves, tris = sc.export()
+    return st, po.KdTree(nodes, leaves, tris, st["bmin"], st["bmax"])
+
+
+def _scene(long_leaves, **kw):
+    cfg = rb.configs.SoupConfig(num_tris=6000)
+    params = rb.kd_params(max_depth=24, leaf_size=8, **kw) if long_leaves else rb.kd_params(**kw)
+    sc = rb.KDScene.from_packed(cfg.packed(), params)
+    st = sc.stats()
+    assert (st["num_refs"] >= 3 * st["num_leaves"]) == long_leaves
+    return sc
+
+
+def _rays(n):
+    rng = np.random.default_rng(6)
+    o = rng.uniform(-1.6, 1.6, (n, 3))
+    d = rng.normal(size=(n, 3))
+    d[: n // 10, 1:] = 0.0
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    tmax = rng.choice([np.inf, 0.5, 1e20], n)
+    return np.concatenate([o, tmax[:, None], d, np.zeros((n, 1))], 1).astype(np.float32)
+
+
+# widths x heights at and just past 4096, 40,960 and 81,920 pixels, and the
+# smallest frame
+SIZES = [(2, 2), (64, 64), (241, 17), (256, 160), (283, 145), (320, 256), (331, 248)]
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("long_leaves", [False, True])
+def test_frames(cuda, long_leaves, mode):
+    with _scene(long_leaves) as sc:
+        st, kd = _kd(sc)
+        for w, h in SIZES:
+            cam = rb.build_camera((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), (60.0, 50.0))
+            ref = po.primary_kd(kd, cam, w, h, mode=mode).view(np.int32).reshape(-1, 4)
+            got = sc.trace_primary(cam, w, h, mode).cpu().numpy()
+            assert np.array_equal(got, ref), (w, h)
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("long_leaves", [False, True])
+def test_caller_rays(cuda, long_leaves, mode):
+    rays = _rays(50001)
+    with _scene(long_leaves) as sc:
+        st, kd = _kd(sc)
+        ref = po.rays_kd(kd, rays, mode=mode).view(np.int32).reshape(-1, 4)
+        dr = torch.from_numpy(rays).cuda()
+        t = sc.tuning()
+        any_hit = mode | rb.TRACE_ANY_HIT
+        sc.set_tuning(t["stage_nodes"], t["queue_kind_major"], t["refill_min"], 8)
+        first = sc.trace_rays(dr, any_hit)
+        assert np.array_equal(first[:, 0].cpu().numpy() >= 0, ref[:, 0] >= 0)
+        sc.set_tuning(t["stage_nodes"], t["queue_kind_major"], t["refill_min"], 32)
+        for n in (1, 3, 33, 4096, 4097, 40960, 40961, 50001):
+            part = dr[:n].contiguous()
+            assert np.array_equal(sc.trace_rays(part, mode).cpu().numpy(), ref[:n]), n
+            assert torch.equal(sc.trace_rays(part, any_hit), first[:n]), n
+
+
+@pytest.mark.parametrize("n", [1000, 20000, 45000])
+def test_visit_cap(cuda, n):
+    """A walk stopped at the leaf-visit cap is counted once in every form."""
+    rays = _rays(n)
+    with _scene(True, max_leaf_visits=2) as sc:
+        st, kd = _kd(sc)
+        ref = po.rays_kd(kd, rays, max_visits=2).view(np.int32).reshape(-1, 4)
+        dr = torch.from_numpy(rays).cuda()
+        t = sc.tuning()
+        got, cut = sc.trace_rays(dr).cpu().numpy(), sc.truncated()
+        assert np.array_equal(got, ref)
+        hit = sc.trace_rays(dr, rb.TRACE_ANY_HIT)
+        any_cut = sc.truncated()
+        sc.set_tuning(t["stage_nodes"], t["queue_kind_major"], t["refill_min"], 8)
+        assert np.array_equal(sc.trace_rays(dr).cpu().numpy(), ref)
+        assert sc.truncated() == cut > n // 20
+        assert torch.equal(sc.trace_rays(dr, rb.TRACE_ANY_HIT), hit)
+        assert sc.truncated() == any_cut > 0
