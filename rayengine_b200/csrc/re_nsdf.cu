@@ -524,36 +524,6 @@ __device__ __forceinline__ TcSmem& tc_smem(unsigned char* raw) {
   return *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
 }
 
-// Batch evaluation: out[i] = network(pts[i]).  Group tiles are claimed
-// round-robin: tile = (block * kGroups + g) + k * (grid * kGroups).
-__global__ void __launch_bounds__(kTcThreads, 1) k_tc_eval(InputMap m,
-                                                           const unsigned char* __restrict__ pack,
-                                                           const float* __restrict__ pts, uint32_t n,
-                                                           float* __restrict__ out,
-                                                           int* __restrict__ err) {
-  extern __shared__ unsigned char smem_raw[];
-  TcSmem& s = tc_smem(smem_raw);
-  tc_setup(s, pack);
-  const int tid = threadIdx.x, g = tid >> 7, row = tid & 127;
-  uint32_t phase = 0;
-  const uint32_t tiles = (n + kGroupRows - 1) / kGroupRows;
-  const uint32_t stride = gridDim.x * kGroups;
-  bool ok = true;
-  for (uint32_t tile = blockIdx.x * kGroups + g; tile < tiles; tile += stride) {
-    uint32_t i = tile * kGroupRows + row;
-    bool live = i < n;
-    float p0 = live ? pts[3 * (size_t)i] : 0.f, p1 = live ? pts[3 * (size_t)i + 1] : 0.f,
-          p2 = live ? pts[3 * (size_t)i + 2] : 0.f;
-    float q[3];
-    normalise(m, p0, p1, p2, q);
-    float dv = mlp_row(s, m, g, row, q, phase, ok);
-    if (live) out[i] = dv;
-    if (!group_and(g, ok)) break;
-  }
-  if (!ok && row == 0) report(err);
-  tc_teardown(s);
-}
-
 // Reference evaluation with the training arithmetic (SIMT FP32, BF16-rounded
 // weights and activations), one thread per point.
 __global__ void __launch_bounds__(128) k_ref_eval(InputMap m, const float* __restrict__ params,
@@ -976,6 +946,172 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_tc_train(
   if (tid < 32)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem),
                  "r"(kTrainCols));
+}
+
+// Batch evaluation: out[i] = network(pts[i]), with mlp_row's arithmetic.
+//
+// What bounds it is the chain of a group's links (store, barrier, MMA, wait,
+// load, softplus): 4 groups of 128 rows left the issue slots half idle.
+// Here 8 groups share the SM, as many as tensor memory holds, one thread a
+// row.  Their operand buffers fit because a row keeps 64 columns: the first
+// layer runs as two MMAs over the features of one chain each (48 columns,
+// then 48 with the position and bias inputs), which add in the order of one.
+//
+// Measured on B200, 1,000,003 points: kernel 154 -> 127 us, call 155 -> 128
+// (issue slots 53 -> 65 % busy; 4 groups with two threads a row: 139 us).
+constexpr int kEvalGroups = 8;
+constexpr int kEvalThreads = kEvalGroups * kGroupRows;  // 1024
+constexpr uint32_t kEvalCols = 64 * kEvalGroups;        // tensor-memory columns
+
+struct __align__(1024) EvalSmem {
+  unsigned char w[kPackWBytes];                             // W1..W4, canonical
+  unsigned char x[kEvalGroups][kGroupRows * kHidden * 2];   // per-group MMA operand
+  float bias[3][kHidden];                                   // b2..b4 (b1 rides in W1)
+  float w5[kHidden];
+  float b5;
+  uint64_t bar[kEvalGroups];
+  uint32_t tmem;
+};
+constexpr size_t kEvalSmemBytes = sizeof(EvalSmem) + 1024;
+
+// One chain's 48 features (chain_features, packed as they are made).
+__device__ __forceinline__ void eval_chain(unsigned char* x, const InputMap& m, int row,
+                                           const float q[3], int chain) {
+  const float f = chain ? m.f0 * 1.41421356f : m.f0;
+  float s[3], c[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const float arg = f * q[j];
+    const float r = arg - rintf(arg);
+    __sincosf(6.28318531f * r, &s[j], &c[j]);
+  }
+  uint32_t w[4];
+#pragma unroll
+  for (int o = 0; o < kOctaves; ++o) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int k = 3 * o + j;
+      w[k & 3] = pack_bf16x2(s[j], c[j]);
+      if ((k & 3) == 3) store_chunk(x, row, 2 * (k - 3), kHidden, w[0], w[1], w[2], w[3]);
+      const float s2 = 2.0f * s[j] * c[j];
+      c[j] = __fmaf_rn(-2.0f * s[j], s[j], 1.0f);
+      s[j] = s2;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kEvalThreads, 1) k_tc_eval(InputMap m,
+                                                             const unsigned char* __restrict__ pack,
+                                                             const float* __restrict__ pts,
+                                                             uint32_t n, float* __restrict__ out,
+                                                             int* __restrict__ err) {
+  extern __shared__ unsigned char smem_raw[];
+  EvalSmem& s = *reinterpret_cast<EvalSmem*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int tid = threadIdx.x, g = tid >> 7, row = tid & 127;
+  for (uint32_t i = tid; i < kPackWBytes / 16; i += kEvalThreads)
+    reinterpret_cast<uint4*>(s.w)[i] = __ldg(reinterpret_cast<const uint4*>(pack) + i);
+  const float* f = reinterpret_cast<const float*>(pack + kPackWBytes);
+  if (tid < 3 * kHidden) s.bias[tid / kHidden][tid % kHidden] = f[kHidden + tid];
+  else if (tid < 4 * kHidden) s.w5[tid - 3 * kHidden] = f[4 * kHidden + tid - 3 * kHidden];
+  if (tid == 0) {
+    s.b5 = f[5 * kHidden];
+    for (int k = 0; k < kEvalGroups; ++k)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s.bar[k])));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // every column: shared memory admits no second CTA of the kernels that use
+  // tensor memory
+  if (tid < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_addr(&s.tmem)),
+                 "r"(kEvalCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  unsigned char* x = s.x[g];
+  const uint32_t dcol = s.tmem + 64u * (uint32_t)g;  // the group's accumulator
+  const uint32_t tme = dcol + ((32u * (uint32_t)(row >> 5)) << 16);
+  const uint32_t tiles = (n + kGroupRows - 1) / kGroupRows;
+  uint32_t phase = 0;
+  bool ok = true;
+  // group 0 of every CTA first, so that a small call spreads over the SMs
+  for (uint32_t tile = g * gridDim.x + blockIdx.x; tile < tiles;
+       tile += gridDim.x * kEvalGroups) {
+    const uint32_t i = tile * kGroupRows + row;
+    const bool live = i < n;
+    float q[3];
+    normalise(m, live ? __ldg(&pts[3 * (size_t)i]) : 0.f,
+              live ? __ldg(&pts[3 * (size_t)i + 1]) : 0.f,
+              live ? __ldg(&pts[3 * (size_t)i + 2]) : 0.f, q);
+    eval_chain(x, m, row, q, 0);
+    float d = 0.f;
+    // stage 0, 1: the first layer's two halves; 2, 3, 4: the hidden layers
+#pragma unroll 1
+    for (int stage = 0; stage < 5; ++stage) {
+      fence_async_smem();
+      fence_before();
+      group_sync(g);
+      fence_after();
+      if (row == 0) {
+        const uint32_t xa = smem_addr(x);
+        const uint32_t wa =
+            smem_addr(s.w) + (stage < 2 ? 768u * (uint32_t)stage  // inputs from column 48
+                                        : kPackW1 + (uint32_t)(stage - 2) * kPackWh);
+        const uint32_t sw = (stage < 2 ? (uint32_t)kIn : (uint32_t)kHidden) * 16u;
+        const uint32_t steps = stage == 0 ? 3u : 4u;
+#pragma unroll 1
+        for (uint32_t k = 0; k < steps; ++k)
+          mma_bf16(dcol, umma_desc(xa + k * 256u, kHidden * 16u), umma_desc(wa + k * 256u, sw),
+                   stage == 1 || k > 0 ? 1u : 0u);
+        mma_commit(&s.bar[g]);
+      }
+      if (ok) ok = mbar_wait(&s.bar[g], phase);
+      phase ^= 1u;
+      __syncwarp();
+      fence_after();
+      if (stage == 0) {
+        eval_chain(x, m, row, q, 1);
+        store_chunk(x, row, 48, kHidden, pack_bf16x2(q[0], q[1]), pack_bf16x2(q[2], 1.0f),
+                    pack_bf16x2(1.0f, 0.f), 0u);
+        store_chunk(x, row, 56, kHidden, 0u, 0u, 0u, 0u);
+        continue;
+      }
+#pragma unroll
+      for (int part = 0; part < 4; ++part) {
+        float acc[16];
+        uint32_t a[8];
+        tmem_ld16(tme + 16u * (uint32_t)part, acc);
+        if (stage > 1) add_bias16(acc, &s.bias[stage - 2][16 * part]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] = softplus_bf16x2(pack_bf16x2(acc[2 * j], acc[2 * j + 1]));
+        if (stage < 4) {
+          store_chunk(x, row, 16 * part, kHidden, a[0], a[1], a[2], a[3]);
+          store_chunk(x, row, 16 * part + 8, kHidden, a[4], a[5], a[6], a[7]);
+        } else {
+          const float4* w4 = reinterpret_cast<const float4*>(s.w5) + 4 * part;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float4 ww = w4[j];
+            d = __fmaf_rn(__uint_as_float(a[2 * j] << 16), ww.x, d);
+            d = __fmaf_rn(__uint_as_float(a[2 * j] & 0xFFFF0000u), ww.y, d);
+            d = __fmaf_rn(__uint_as_float(a[2 * j + 1] << 16), ww.z, d);
+            d = __fmaf_rn(__uint_as_float(a[2 * j + 1] & 0xFFFF0000u), ww.w, d);
+          }
+        }
+      }
+    }
+    if (live) out[i] = d + s.b5;
+  }
+  if (!ok && row == 0) report(err);
+  fence_before();
+  __syncthreads();
+  fence_after();
+  if (tid < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem),
+                 "r"(kEvalCols));
 }
 
 // ------------------------------------------------------------- tracing
@@ -2076,11 +2212,15 @@ RE_API re_status re_nsdf_eval(re_nsdf* s, const float* d_pts, uint32_t n, float*
   st = re::ensure_pack(s, cs);
   if (st != RE_OK) return st;
   auto k = re::nsdf::k_tc_eval;
-  RE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)re::kTcSmemBytes));
-  int grid = std::min<int>(re::tc_grid(k), (int)((n + 511) / 512));
+  RE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)re::nsdf::kEvalSmemBytes));
+  // one CTA per SM; no more CTAs than 128-row tiles, so that a small call's
+  // tiles spread over the SMs
+  const uint32_t tiles = (n + re::nsdf::kGroupRows - 1) / re::nsdf::kGroupRows;
+  const int grid = (int)std::min<uint32_t>((uint32_t)re::sm_count(), tiles);
   *s->sync_err = 0;
-  k<<<grid, re::nsdf::kTcThreads, re::kTcSmemBytes, cs>>>(s->map, s->pack, d_pts, n, d_out,
-                                                          s->sync_err_dev);
+  k<<<grid, re::nsdf::kEvalThreads, re::nsdf::kEvalSmemBytes, cs>>>(s->map, s->pack, d_pts, n,
+                                                                    d_out, s->sync_err_dev);
   RE_CHECK_LAUNCH("re_nsdf_eval: launch");
   RE_CUDA(cudaStreamSynchronize(cs));
   if (*s->sync_err) return re::fail(RE_ERR_INTERNAL, "re_nsdf_eval: tensor-core wait bound reached");
