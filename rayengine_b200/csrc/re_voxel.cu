@@ -45,12 +45,28 @@ __device__ __forceinline__ const float2* voxel_row(const GridDev& g, int y, int 
   return g.v + (size_t)g.dim[0] * ((size_t)y + (size_t)g.dim[1] * z);
 }
 
-__device__ __forceinline__ float bspline(float t) {
-  t = fabsf(t);
-  const float a = 2.0f - t;
-  if (t < 1.0f) return 2.0f / 3.0f - 0.5f * t * t * a;
-  if (t < 2.0f) return a * a * a / 6.0f;
-  return 0.0f;
+// x / 6 for x in [0, 1] (zero or at least 2^-69 here): the product with the
+// rounded reciprocal, corrected once by its exact remainder, is the rounded
+// quotient (Markstein 1990, division by a constant with fused multiply-add;
+// compared with the division over every mantissa).
+__device__ __forceinline__ float sixth(float x) {
+  const float y = 1.0f / 6.0f, q = x * y;
+  return __fmaf_rn(__fmaf_rn(-6.0f, q, x), y, q);
+}
+
+// The cubic B-spline at -1 - f, -f, 1 - f and 2 - f for a fraction f in
+// [0, 1]: with t its argument's magnitude and a = 2 - t, 2/3 - t^2 a / 2
+// below 1 and a^3 / 6 from 1 to 2.  The outer two are always in the second
+// range, the inner two in the first or at t = 1.  A NaN fraction (a lookup
+// at an infinite coordinate) has no weight anywhere.
+__device__ __forceinline__ void bspline4(float f, float (&w)[4]) {
+  const float t0 = fabsf(-1.0f - f), t1 = fabsf(f), t2 = fabsf(1.0f - f), t3 = fabsf(2.0f - f);
+  const float a0 = 2.0f - t0, a1 = 2.0f - t1, a2 = 2.0f - t2, a3 = 2.0f - t3;
+  const bool some = f >= 0.0f;
+  w[0] = some ? sixth(a0 * a0 * a0) : 0.0f;
+  w[1] = some ? (t1 < 1.0f ? 2.0f / 3.0f - 0.5f * t1 * t1 * a1 : 1.0f / 6.0f) : 0.0f;
+  w[2] = some ? (t2 < 1.0f ? 2.0f / 3.0f - 0.5f * t2 * t2 * a2 : 1.0f / 6.0f) : 0.0f;
+  w[3] = some ? sixth(a3 * a3 * a3) : 0.0f;
 }
 
 __device__ __forceinline__ float bilerp(float tx, float ty, float c00, float c10, float c01,
@@ -65,7 +81,7 @@ __device__ __forceinline__ float bilerp(float tx, float ty, float c00, float c10
 // The arithmetic is the plain form's: weights bx (by bz), products added in
 // x, y, z order.
 // Measured on B200 (one edit and the 1280x720 frame of a 192x96x192 grid at
-// HIGH, with k_trace and k_brush below): 2.40 -> 1.03 ms; each of the 64
+// HIGH, with k_trace_high and k_brush below): 2.40 -> 0.81 ms; each of the 64
 // lookups had taken its own three clamps, 64-bit index and three B-spline
 // evaluations.
 template <uint32_t Q>
@@ -99,20 +115,27 @@ __device__ __forceinline__ float sample(const GridDev& g, V3 p) {
   float w[3][4];
   if (Q == RE_VOXEL_HIGH) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) w[k][i] = bspline((float)(i - 1) - fr[k]);
+    for (int k = 0; k < 3; ++k) bspline4(fr[k], w[k]);
   }
   float result = 0.0f, ef[2] = {0.0f, 0.0f};
   auto layer = [&](int z, auto row) {  // row(y, x): voxel (x, y) of layer z
     if (Q == RE_VOXEL_MEDIUM) {
       ef[z] = bilerp(fr[0], fr[1], row(0, 0), row(0, 1), row(1, 0), row(1, 1));
     } else {
+      // rows y and y + 1 in the halves of packed registers, added one after
+      // the other
 #pragma unroll
-      for (int y = 0; y < N; ++y) {
-        const float byz = w[1][y] * w[2][z];
+      for (int y = 0; y < N; y += 2) {
+        const f32x2 byz = mul2(pack2(w[1][y], w[1][y + 1]), pack2(w[2][z], w[2][z]));
+        float lo[N], hi[N];
 #pragma unroll
-        for (int x = 0; x < N; ++x) result += (w[0][x] * byz) * row(y, x);
+        for (int x = 0; x < N; ++x)
+          unpack2(mul2(mul2(pack2(w[0][x], w[0][x]), byz), pack2(row(y, x), row(y + 1, x))), lo[x],
+                  hi[x]);
+#pragma unroll
+        for (int x = 0; x < N; ++x) result = __fadd_rn(result, lo[x]);
+#pragma unroll
+        for (int x = 0; x < N; ++x) result = __fadd_rn(result, hi[x]);
       }
     }
   };
@@ -172,18 +195,89 @@ struct MarchDev {
 // voxel centres, origin .. origin + (dim - 1) spacing): the exact tracer's
 // rule t += step_factor * d, hit when d < eps; normal by central
 // differences with delta = half the smallest spacing.  Output as re_sdf_hit.
-//
-// A per-lane state machine with one lookup per trip (phase 0 marches, phases
-// 1..6 are the normal's taps), as the exact tracer's: a lane whose ray ends
-// takes the next pixel, so rays of few and of many lookups share a warp
-// without waiting for one another.  A block owns the 8x4 pixel tiles
-// blockIdx, blockIdx + gridDim, ...; its warps claim them pixel by pixel
-// from a counter in shared memory.
-constexpr uint32_t kVoxelRefill = 8;
 
+// The ray of pixel (x, y) and its span [t0, t1) in the box.
+__device__ __forceinline__ void grid_ray(const GridDev& g, const MarchDev& m, const CamDev& cam,
+                                         uint32_t w, uint32_t h, uint32_t x, uint32_t y, V3& o,
+                                         V3& d, float& t0, float& t1) {
+  generate_ray(cam, w, h, x, y, o, d);
+  const float o3[3] = {o.x, o.y, o.z}, d3[3] = {d.x, d.y, d.z};
+  t0 = 0.0f;
+  t1 = m.tmax;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    float lo = g.origin[k], hi = __fmaf_rn((float)(g.dim[k] - 1), g.spacing[k], g.origin[k]);
+    float inv = 1.0f / d3[k];
+    float ta = (lo - o3[k]) * inv, tb = (hi - o3[k]) * inv;
+    t0 = fmaxf(t0, fminf(ta, tb));
+    t1 = fminf(t1, fmaxf(ta, tb));
+  }
+}
+
+// n: the differences along the axes (hits only).
+__device__ __forceinline__ void store_record(float4* out, uint32_t pix, V3 p, V3 n,
+                                             uint32_t steps, uint32_t status) {
+  float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
+  if (status == 1) {
+    n = normalize(n);
+    r0 = make_float4(p.x, p.y, p.z, n.x);
+    r1 = make_float4(n.y, n.z, 0.f, 0.f);
+  }
+  r1.z = __uint_as_float(steps);
+  r1.w = __uint_as_float(status);
+  out[2 * (size_t)pix] = r0;
+  out[2 * (size_t)pix + 1] = r1;
+}
+
+// LOW and MEDIUM, a thread per pixel: the march, then the six lookups of the
+// normal side by side (their loads overlap; one after another as below they
+// took a 160x90 frame from 78 to 110 us).
 template <uint32_t Q>
-__global__ void __launch_bounds__(256) k_trace(GridDev g, MarchDev m, CamDev cam, uint32_t w,
-                                               uint32_t h, float4* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_trace_pixel(GridDev g, MarchDev m, CamDev cam, uint32_t w,
+                                                     uint32_t h, float4* __restrict__ out) {
+  const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pix >= w * h) return;
+  V3 o, d, p = {0.f, 0.f, 0.f}, n = p;
+  float t, t1;
+  grid_ray(g, m, cam, w, h, pix % w, pix / w, o, d, t, t1);
+  uint32_t steps = 0, status = 0;
+  if (t < t1) {
+    for (;;) {
+      p = v3(__fmaf_rn(t, d.x, o.x), __fmaf_rn(t, d.y, o.y), __fmaf_rn(t, d.z, o.z));
+      const float v = sample<Q>(g, p);
+      ++steps;
+      if (v < m.eps) {
+        status = 1;
+        break;
+      }
+      t = __fmaf_rn(m.step_factor, v, t);
+      if (t > t1) break;
+      if (steps >= m.max_steps) {
+        status = 2;
+        break;
+      }
+    }
+  }
+  if (status == 1) {
+    const float e = 0.5f * fminf(g.spacing[0], fminf(g.spacing[1], g.spacing[2]));
+    n.x = sample<Q>(g, v3(p.x + e, p.y, p.z)) - sample<Q>(g, v3(p.x - e, p.y, p.z));
+    n.y = sample<Q>(g, v3(p.x, p.y + e, p.z)) - sample<Q>(g, v3(p.x, p.y - e, p.z));
+    n.z = sample<Q>(g, v3(p.x, p.y, p.z + e)) - sample<Q>(g, v3(p.x, p.y, p.z - e));
+  }
+  store_record(out, pix, p, n, steps, status);
+}
+
+// HIGH, a per-lane state machine with one lookup per trip (phase 0 marches,
+// phases 1..6 are the normal's taps), so rays that hit early take their taps
+// while others march, and the long lookup is in the code once.  A warp takes
+// its next 8x4 pixel tile when all its rays have ended: the loads bound it
+// (64 a lookup, L1 74 % busy), and lanes of one tile read the same few
+// voxels, which lanes refilled from another do not (measured, frame above:
+// next pixels at 8 idle lanes 906 us, at 24 861, at 32 808; 2 blocks an SM
+// 803, 4 972).  A block owns the tiles blockIdx, blockIdx + gridDim, ...; its
+// warps claim them from a counter in shared memory.
+__global__ void __launch_bounds__(256) k_trace_high(GridDev g, MarchDev m, CamDev cam, uint32_t w,
+                                                    uint32_t h, float4* __restrict__ out) {
   __shared__ uint32_t cursor;
   if (threadIdx.x == 0) cursor = 0u;
   __syncthreads();
@@ -191,50 +285,27 @@ __global__ void __launch_bounds__(256) k_trace(GridDev g, MarchDev m, CamDev cam
   const uint32_t tiles_x = (w + 7) / 8, tiles = tiles_x * ((h + 3) / 4);
   const uint32_t mine = (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x;  // grid <= tiles
   const float delta = 0.5f * fminf(g.spacing[0], fminf(g.spacing[1], g.spacing[2]));
-  bool live = false, exhausted = false;
+  bool live = false;
   uint32_t pix = 0, steps = 0, phase = 0;
-  V3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 1.f}, p = o;
-  float t = 0.f, t1 = 0.f, nx = 0.f, ny = 0.f, nz = 0.f, plus = 0.f;
+  V3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 1.f}, p = o, n = o;
+  float t = 0.f, t1 = 0.f, plus = 0.f;
   for (;;) {
-    const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !live);
-    const uint32_t nidle = __popc(idle);
-    if (!exhausted && (nidle >= kVoxelRefill || nidle == 32u)) {
-      uint32_t base = 0;
-      if (lane == 0) base = atomicAdd(&cursor, nidle);
-      base = __shfl_sync(0xFFFFFFFFu, base, 0);
-      if (base + nidle >= 32u * mine) exhausted = true;
-      if (!live) {
-        const uint32_t i = base + __popc(idle & ((1u << lane) - 1u));
-        const uint32_t tile = blockIdx.x + (i >> 5) * gridDim.x, l = i & 31u;
-        const uint32_t x = (tile % tiles_x) * 8 + (l & 7u), y = (tile / tiles_x) * 4 + (l >> 3);
-        if ((i >> 5) < mine && x < w && y < h) {
-          generate_ray(cam, w, h, x, y, o, d);
-          pix = y * w + x;
-          const float o3[3] = {o.x, o.y, o.z}, d3[3] = {d.x, d.y, d.z};
-          float t0 = 0.0f;
-          t1 = m.tmax;
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            float lo = g.origin[k], hi = __fmaf_rn((float)(g.dim[k] - 1), g.spacing[k], g.origin[k]);
-            float inv = 1.0f / d3[k];
-            float ta = (lo - o3[k]) * inv, tb = (hi - o3[k]) * inv;
-            t0 = fmaxf(t0, fminf(ta, tb));
-            t1 = fminf(t1, fmaxf(ta, tb));
-          }
-          t = t0;
-          steps = 0;
-          phase = 0;
-          live = t0 < t1;
-          if (!live) {  // the ray passes the grid by
-            out[2 * (size_t)pix] = make_float4(0.f, 0.f, 0.f, 0.f);
-            out[2 * (size_t)pix + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-        }
-      }
-    }
     if (__ballot_sync(0xFFFFFFFFu, live) == 0u) {
-      if (exhausted) break;
-      continue;
+      uint32_t k = 0;
+      if (lane == 0) k = atomicAdd(&cursor, 1u);
+      k = __shfl_sync(0xFFFFFFFFu, k, 0);
+      if (k >= mine) break;
+      const uint32_t tile = blockIdx.x + k * gridDim.x;
+      const uint32_t x = (tile % tiles_x) * 8 + (lane & 7u),
+                     y = (tile / tiles_x) * 4 + (lane >> 3);
+      if (x < w && y < h) {
+        grid_ray(g, m, cam, w, h, x, y, o, d, t, t1);
+        pix = y * w + x;
+        steps = 0;
+        phase = 0;
+        live = t < t1;
+        if (!live) store_record(out, pix, p, n, 0u, 0u);  // the ray passes the grid by
+      }
     }
     if (!live) continue;
     V3 q;
@@ -247,7 +318,7 @@ __global__ void __launch_bounds__(256) k_trace(GridDev g, MarchDev m, CamDev cam
       else if (phase <= 4) q.y = p.y + sd;
       else q.z = p.z + sd;
     }
-    const float v = sample<Q>(g, q);
+    const float v = sample<RE_VOXEL_HIGH>(g, q);
     uint32_t status = 3;  // 3 = keep going
     if (phase == 0) {
       ++steps;
@@ -264,24 +335,15 @@ __global__ void __launch_bounds__(256) k_trace(GridDev g, MarchDev m, CamDev cam
         plus = v;
       } else {
         const float diff = plus - v;
-        if (phase == 2) nx = diff;
-        else if (phase == 4) ny = diff;
-        else nz = diff;
+        if (phase == 2) n.x = diff;
+        else if (phase == 4) n.y = diff;
+        else n.z = diff;
       }
       if (phase == 6) status = 1;
       else ++phase;
     }
     if (status != 3) {
-      float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1;
-      if (status == 1) {
-        V3 n = normalize(v3(nx, ny, nz));
-        r0 = make_float4(p.x, p.y, p.z, n.x);
-        r1 = make_float4(n.y, n.z, __uint_as_float(steps), __uint_as_float(status));
-      } else {
-        r1 = make_float4(0.f, 0.f, __uint_as_float(steps), __uint_as_float(status));
-      }
-      out[2 * (size_t)pix] = r0;
-      out[2 * (size_t)pix + 1] = r1;
+      store_record(out, pix, p, n, steps, status);
       live = false;
     }
   }
@@ -418,17 +480,24 @@ RE_API re_status re_voxel_trace(const float* d_grid, const re_voxel_grid* g, uin
     return re::fail(RE_ERR_INVALID_ARG, "re_voxel_trace: bad arguments");
   if ((uint64_t)w * h > (1ull << 30)) return re::fail(RE_ERR_LIMIT, "re_voxel_trace: image too large");
   re::voxel::MarchDev m{march->step_factor, march->eps, march->tmax, march->max_steps};
-  auto k = quality == RE_VOXEL_LOW      ? re::voxel::k_trace<RE_VOXEL_LOW>
-           : quality == RE_VOXEL_MEDIUM ? re::voxel::k_trace<RE_VOXEL_MEDIUM>
-                                        : re::voxel::k_trace<RE_VOXEL_HIGH>;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 256, 0) != cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
-  const uint32_t tiles = ((w + 7) / 8) * ((h + 3) / 4);
-  k<<<std::min<uint32_t>((uint32_t)(per_sm * re::sm_count()), tiles), 256, 0,
-      (cudaStream_t)stream>>>(re::grid_dev(g, d_grid), m, re::cam_of_voxel(*cam), w, h,
-                              reinterpret_cast<float4*>(d_out));
+  const re::voxel::GridDev gd = re::grid_dev(g, d_grid);
+  const re::CamDev cd = re::cam_of_voxel(*cam);
+  float4* out = reinterpret_cast<float4*>(d_out);
+  cudaStream_t cs = (cudaStream_t)stream;
+  if (quality == RE_VOXEL_HIGH) {
+    auto k = re::voxel::k_trace_high;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 256, 0) != cudaSuccess ||
+        per_sm < 1)
+      per_sm = 1;
+    const uint32_t tiles = ((w + 7) / 8) * ((h + 3) / 4);
+    const uint32_t grid = std::min<uint32_t>((uint32_t)(per_sm * re::sm_count()), tiles);
+    k<<<grid, 256, 0, cs>>>(gd, m, cd, w, h, out);
+  } else {
+    auto k = quality == RE_VOXEL_LOW ? re::voxel::k_trace_pixel<RE_VOXEL_LOW>
+                                     : re::voxel::k_trace_pixel<RE_VOXEL_MEDIUM>;
+    k<<<(w * h + 255) / 256, 256, 0, cs>>>(gd, m, cd, w, h, out);
+  }
   RE_CHECK_LAUNCH("re_voxel_trace: launch");
   return RE_OK;
 }
