@@ -17,19 +17,21 @@
 // last bounce writes 0.  Each pixel is written exactly once.
 //
 // Work distribution (no grid-wide barrier):
-//   * primary rays come from a global pixel cursor over all scenes' pixels;
+//   * the two kinds of scene are two pipelines (a continuation stays in its
+//     scene); a warp works on one kind at a time and changes over when that
+//     kind has nothing for it;
+//   * primary rays come from a global pixel cursor per kind over its scenes'
+//     pixels;
 //   * a ray that continues is appended to the queue of (next bounce, scene
 //     kind): a warp reserves slots with one atomic per distinct queue, writes
 //     the 32-byte records and publishes each slot with a release store of the
 //     frame's epoch into the slot's flag;
-//   * idle lanes refill from the deepest non-empty queue (preferring the kind
-//     the warp is already running, so meshes and terrains rarely share a
-//     warp), claiming only published-or-reserved slots (compare-and-swap up to
-//     the reserved count) and waiting, without blocking the warp, for a
+//   * idle lanes refill from the kind's deepest non-empty queue, claiming
+//     slots with one atomic and waiting, without blocking the warp, for a
 //     claimed slot's flag;
-//   * a warp leaves when the cursor is exhausted and every created ray has
-//     finished (children are counted as created before their parent counts
-//     as finished, so finished == created means nothing is in flight);
+//   * a warp leaves when both kinds' cursors are exhausted and every created
+//     ray has finished (children are counted as created before their parent
+//     counts as finished, so finished == created means nothing is in flight);
 //   * the last block to leave resets the counters and advances the epoch, so
 //     the same launch can be replayed from a CUDA graph.
 // Every wait has an iteration bound after which the kernel sets the error
@@ -64,12 +66,12 @@ constexpr uint32_t kMesh = RE_BATCH_MESH, kTerrain = RE_BATCH_TERRAIN;
 // of bounce b = the reserved counts of bounce b's two queues.
 constexpr uint32_t kLine = 32;
 enum : uint32_t {
-  kCursor = 0 * kLine,
-  kFin = 1 * kLine,  // + bounce * kLine: finished rays of that bounce
-  kEpoch = (1 + kMaxDepth) * kLine,
-  kDone = (2 + kMaxDepth) * kLine,
-  kError = (2 + kMaxDepth) * kLine + 1,
-  kReserved = (3 + kMaxDepth) * kLine,  // + q * kLine
+  kCursor = 0 * kLine,  // + kind * kLine
+  kFin = 2 * kLine,     // + (2 * bounce + kind) * kLine: finished rays of that bounce
+  kEpoch = (2 + 2 * kMaxDepth) * kLine,
+  kDone = (3 + 2 * kMaxDepth) * kLine,
+  kError = (3 + 2 * kMaxDepth) * kLine + 1,
+  kReserved = (4 + 2 * kMaxDepth) * kLine,  // + q * kLine
   kClaimed = kReserved + kMaxQueues * kLine,
   kStats = kClaimed + kMaxQueues * kLine,  // + q
   kStatsPrimary = kStats + kMaxQueues,
@@ -77,7 +79,10 @@ enum : uint32_t {
   kNumCounters = kStats + kLine
 };
 static_assert(kStatsError < kNumCounters, "counter layout");
-__host__ __device__ constexpr uint32_t fin_at(uint32_t b) { return kFin + b * kLine; }
+__host__ __device__ constexpr uint32_t cursor_at(uint32_t kind) { return kCursor + kind * kLine; }
+__host__ __device__ constexpr uint32_t fin_at(uint32_t b, uint32_t kind) {
+  return kFin + (2u * b + kind) * kLine;
+}
 __host__ __device__ constexpr uint32_t reserved_at(uint32_t q) { return kReserved + q * kLine; }
 __host__ __device__ constexpr uint32_t claimed_at(uint32_t q) { return kClaimed + q * kLine; }
 
@@ -92,6 +97,7 @@ struct __align__(16) SceneDev {
   float ceiling;  // terrain: no surface above this height (|fBm| bound)
   CamDev cam;
   uint32_t w, h, kind, pix_off;
+  uint32_t kind_off[2];  // pixels of each kind in the scenes before this one
   float albedo;
   // the mesh's entry table (re_kd.cuh entry_node) for its camera rays
   const uint32_t* entry;
@@ -106,7 +112,8 @@ static_assert(sizeof(SceneDev) % 16 == 0, "SceneDev must keep the staged nodes a
 struct BatchDev {
   const SceneDev* scenes;
   const uint8_t* perms;  // perm_count tables of 512 bytes (words in shared memory)
-  uint32_t num_scenes, perm_count, stage_total, total_pixels;
+  uint32_t num_scenes, perm_count, stage_total;
+  uint32_t kind_pixels[2];
   uint32_t depth, seed, refill_min, steps_per_trip;
   uint32_t pending_bound, loop_bound;  // polls of one slot flag, trips of the loop
   float mesh_bias;
@@ -139,6 +146,19 @@ __device__ __forceinline__ uint32_t scene_of(const SceneDev* sc, uint32_t n, uin
   while (lo < hi) {
     uint32_t mid = (lo + hi + 1) >> 1;
     if (sc[mid].pix_off <= gpix) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+// The scene of pixel i among the pixels of `kind`.
+__device__ __forceinline__ uint32_t scene_of_kind(const SceneDev* sc, uint32_t n, uint32_t kind,
+                                                  uint32_t i) {
+  // the last scene with kind_off <= i: the next one of this kind starts past i
+  uint32_t lo = 0, hi = n - 1;
+  while (lo < hi) {
+    uint32_t mid = (lo + hi + 1) >> 1;
+    if (sc[mid].kind_off[kind] <= i) lo = mid;
     else hi = mid - 1;
   }
   return lo;
@@ -198,104 +218,72 @@ __device__ __forceinline__ float miss_radiance(float albedo, uint32_t bounce, V3
 }
 
 enum : uint32_t { kIdle = 0, kPending = 1, kLive = 2 };
-enum : uint32_t { kMarch = 0, kNormal = 1 };
 // Default wait bounds (re_batch_set_wait_bounds lowers them for tests).
 constexpr uint32_t kPendingBound = 1u << 22;  // polls of one slot flag
 constexpr uint32_t kLoopBound = 1u << 22;     // trips of the persistent loop
 
-// Bounce b's queues are closed (no ray of bounce b can still be created)
-// once the pixel cursor is exhausted and every ray of bounce b - 1 has
-// finished.  Bit b of the result, b = 1 .. depth; bit depth = the frame is
+// Bounce b's queue of a kind is closed (no ray of bounce b can still be
+// created: a ray's continuation stays in its scene, so in its kind) once the
+// kind's pixel cursor is exhausted and every ray of bounce b - 1 has
+// finished.  Bit b of the result, b = 1 .. depth; bit depth = the kind is
 // done.  Each bounce's created count is read only after its predecessor's
 // finished count compared equal (a control dependency orders the loads), so
 // it is final when read: its producers all finished first.
-__device__ __forceinline__ uint32_t closed_mask(const uint32_t* ctr, const BatchDev& B) {
-  uint32_t mask = 0, created = B.total_pixels;
+__device__ __forceinline__ uint32_t closed_mask(const uint32_t* ctr, const BatchDev& B,
+                                                uint32_t kind) {
+  uint32_t mask = 0, created = B.kind_pixels[kind];
   for (uint32_t b = 1; b <= B.depth; ++b) {
-    if (ld_relaxed(&ctr[fin_at(b - 1)]) != created) break;
+    if (ld_relaxed(&ctr[fin_at(b - 1, kind)]) != created) break;
     mask |= 1u << b;
     if (b == B.depth) break;
-    created = ld_relaxed(&ctr[reserved_at(2 * (b - 1))]) + ld_relaxed(&ctr[reserved_at(2 * (b - 1) + 1)]);
+    created = ld_relaxed(&ctr[reserved_at(2 * (b - 1) + kind)]);
   }
   return mask;
 }
 
-// Launch bounds: blocks of up to 256 threads, 4 resident per SM (64
-// registers, 32 warps per SM).  Measured on the 8-scene batch: 22.0 ms
-// against 30.4 ms with 122 registers and 16 warps, despite the spills.
-#ifndef RE_BATCH_MIN_BLOCKS
-#define RE_BATCH_MIN_BLOCKS 4
-#endif
-#ifndef RE_BATCH_MAX_THREADS
-#define RE_BATCH_MAX_THREADS 256
-#endif
-
-// WORDS: the terrain permutation tables in shared memory as perm_word()
-// entries (2 KB per seed), else as bytes (512 B per seed; batches with
-// more than kWordTablesMax seeds, where word tables would cost blocks per SM).
-template <bool COUNT, bool WORDS>
-__global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_batch(BatchDev B) {
-  extern __shared__ uint4 smem_u4[];
-  SceneDev* sc = reinterpret_cast<SceneDev*>(smem_u4);
-  uint8_t* sperm = reinterpret_cast<uint8_t*>(sc + B.num_scenes);
-  uint32_t* sperm_w = reinterpret_cast<uint32_t*>(sperm);
-  uint2* snodes = reinterpret_cast<uint2*>(sperm + (WORDS ? 4u : 1u) * 512u * B.perm_count);
-  uint32_t* sfin = reinterpret_cast<uint32_t*>(snodes + B.stage_total);  // [warp][bounce]
-  {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(B.scenes);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(sc);
-    for (uint32_t i = threadIdx.x; i < B.num_scenes * (uint32_t)(sizeof(SceneDev) / 4); i += blockDim.x)
-      dst[i] = src[i];
-    for (uint32_t i = threadIdx.x; i < 512u * B.perm_count; i += blockDim.x) {
-      if (WORDS)
-        sperm_w[i] = perm_word(B.perms[i]);
-      else
-        sperm[i] = B.perms[i];
-    }
-    for (uint32_t i = threadIdx.x; i < (blockDim.x / 32u) * kMaxDepth; i += blockDim.x) sfin[i] = 0u;
-    __syncthreads();
-    for (uint32_t s = 0; s < B.num_scenes; ++s)
-      for (uint32_t i = threadIdx.x; i < sc[s].stage; i += blockDim.x)
-        snodes[sc[s].stage_off + i] = __ldg(&sc[s].nodes[i]);
-    __syncthreads();
-  }
+// TABLE: the terrain tables in shared memory, by the number of seeds (larger
+// tables would cost blocks per SM): kFieldTables, the paired form's A and G
+// words (4 KB per seed); kWordTables, perm_word() entries (2 KB); kByteTables,
+// bytes (512 B); kNoTables: a batch of meshes alone.
+enum : int { kByteTables = 0, kWordTables = 1, kFieldTables = 2, kNoTables = 3 };
+__host__ __device__ constexpr uint32_t table_bytes(int table) {
+  return table == kFieldTables ? kFieldWordsBytes : table == kWordTables ? 2048u : 512u;
+}
+// One kind's rays on one warp: claims and steps them until the warp holds none
+// and finds none to claim.  Returns whether it held any.
+//
+// The kinds never exchange rays, so a warp works on one at a time and the
+// mesh walk and the terrain march do not share a loop: in one loop for both
+// they shared its registers (284 bytes of spills) and its warps, and a step
+// of either kind waited for the other's.  Measured on B200, six scenes of
+// 864,000 pixels (two terrains): 3.61 -> 2.62 ms, of which the paired field
+// 0.3; meshes alone 1.45 -> 1.26 ms; the 32-scene batch 60.8 -> 56.4.  Three
+// blocks per SM: the six scenes 2.60, the 32 scenes 64.3.
+template <bool COUNT, int TABLE, uint32_t KIND>
+__device__ __forceinline__ bool run_kind(const BatchDev& B, const SceneDev* sc,
+                                         const uint8_t* sperm, const uint2* snodes, uint32_t* wfin,
+                                         uint32_t epoch, uint32_t& trip, Counters& cnt,
+                                         uint32_t& errors) {
+  const uint32_t* sperm_w = reinterpret_cast<const uint32_t*>(sperm);
   uint32_t* ctr = B.ctr;
-  const uint32_t epoch = ld_relaxed(&ctr[kEpoch]);
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt_mask = (1u << lane) - 1u;
-  const uint32_t nq = 2u * (B.depth - 1u);
-  uint32_t* wfin = sfin + (threadIdx.x >> 5) * kMaxDepth;  // this warp's unpublished counts
-
   uint32_t state = kIdle;
-  uint32_t gpix = 0, scene = 0, bounce = 0, kind = kMesh;
+  uint32_t gpix = 0, scene = 0, bounce = 0;
   Trav tr;
   tr.live = false;
-  // Terrain march state, kept in the Trav fields that a terrain ray leaves
-  // unused (its ray is tr.o / tr.d) so that it takes no registers of its
-  // own in this register-bound kernel: nx, ny, nz as float bits, the mode
-  // (bit 3) and the normal tap (bits 0-2) in one word.  Every field is set
-  // by a ray's start (trav_init or the terrain start below) before use.
-  float& t = tr.t_entry;
-  float& v_hit = tr.best_t;
-  float& delta = tr.best_u;
-  float& plus = tr.best_v;
-  V3& p = tr.inv;
-  uint32_t& steps = tr.visits;
-  uint32_t& mode_tap = tr.node;
-  uint32_t& nx_bits = tr.best_ref;
-  uint32_t& ny_bits = tr.best_leaf;
-  int32_t& nz_bits = tr.best_id;
-  // A pending claim (queue, slot, polls so far) likewise: a lane waiting
-  // for its record has no ray yet, and the ray's start overwrites these
-  // fields only after the record has been read.
-  uint32_t& pq = tr.best_ref;
-  uint32_t& pslot = tr.best_leaf;
-  uint32_t& polls = tr.visits;
-  Counters cnt = {0, 0, 0, 0};
-  uint32_t errors = 0;
+  tr.o = tr.d = v3(0.f, 0.f, 0.f);
+  tr.best_ref = tr.best_leaf = tr.visits = 0u;
+  // The march keeps its state in the walk's fields (the other kind's, unused
+  // here), as does a pending claim (queue, slot, polls so far): a lane that
+  // waits for its record has no ray yet, and the ray's start overwrites them.
+  float &t = tr.t_entry, &v_hit = tr.best_t, &plus = tr.best_u;
+  V3& tap_diff = tr.inv;
+  uint32_t &steps = tr.visits, &tap = tr.best_ref;
+  uint32_t &pq = tr.best_ref, &pslot = tr.best_leaf, &polls = tr.visits;
   uint32_t fin_pending = 0;   // lane 0: finished rays in wfin
-  uint32_t backoff = 32;      // lane 0: idle sleep, ns
   bool primary_done = false;  // lane 0: the pixel cursor has passed the end
+  bool any = false;
 
   // publishes this warp's finished counts (after its reservations, which
   // completed when their atomics returned)
@@ -306,7 +294,7 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
       for (uint32_t b = 0; b < B.depth; ++b) {
         uint32_t v = wfin[b];
         if (v) {
-          atomicAdd(&ctr[fin_at(b)], v);
+          atomicAdd(&ctr[fin_at(b, KIND)], v);
           wfin[b] = 0u;
         }
       }
@@ -315,7 +303,6 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
     __syncwarp();
   };
 
-  uint32_t trip = 0;
   for (; trip < B.loop_bound; ++trip) {
     // ---- pending claims: the slot's record is published once its flag holds this epoch
     if (state == kPending) {
@@ -332,16 +319,15 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
         gpix = tag & 0x0FFFFFFFu;
         bounce = tag >> 28;
         scene = scene_of(sc, B.num_scenes, gpix);
-        kind = sc[scene].kind;
         V3 o = v3(A.x, A.y, A.z), d = v3(Bv.x, Bv.y, Bv.z);
-        if (kind == kMesh) {
+        if (KIND == kMesh) {
           trav_init(tr, kd_of(sc[scene]), o, d, K_INF, __float_as_uint(A.w));
         } else {
           tr.o = o;
           tr.d = d;
           t = 0.f;
           steps = 0;
-          mode_tap = kMarch << 3;
+          tap = 0u;
         }
         state = kLive;
       } else {
@@ -356,7 +342,7 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
     // of their slot (checked every 64 unsuccessful polls)
     if (__ballot_sync(0xFFFFFFFFu, state == kPending && polls != 0u && (polls & 63u) == 0u)) {
       uint32_t mask = 0;
-      if (lane == 0) mask = closed_mask(ctr, B);
+      if (lane == 0) mask = closed_mask(ctr, B, KIND);
       mask = __shfl_sync(0xFFFFFFFFu, mask, 0);
       if (state == kPending && ((mask >> (pq / 2u + 1u)) & 1u)) {
         if (pslot >= ld_relaxed(&ctr[reserved_at(pq)])) state = kIdle;  // never filled
@@ -370,34 +356,29 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
     uint32_t idle = __ballot_sync(0xFFFFFFFFu, state == kIdle);
     uint32_t nidle = __popc(idle);
     if (nidle != 0u && (nidle >= B.refill_min || nidle == 32u)) {
-      uint32_t live_mesh = __ballot_sync(0xFFFFFFFFu, state != kIdle && kind == kMesh);
-      uint32_t live_terr = __ballot_sync(0xFFFFFFFFu, state != kIdle && kind == kTerrain);
-      // lane q reads queue q's counters: one round trip for all queues
+      // lane b - 1 reads the counters of bounce b's queue: one round trip
       uint32_t avail = 0;
-      if (lane < nq) {
-        uint32_t r = ld_relaxed(&ctr[reserved_at(lane)]), c = ld_relaxed(&ctr[claimed_at(lane)]);
+      if (lane + 1u < B.depth) {
+        const uint32_t q = 2u * lane + KIND;
+        uint32_t r = ld_relaxed(&ctr[reserved_at(q)]), c = ld_relaxed(&ctr[claimed_at(q)]);
         avail = r > c ? r - c : 0u;
       }
       uint32_t src = 0xFFFFFFFFu, base = 0, k = 0;
-      const uint32_t first = live_terr > live_mesh ? kTerrain : kMesh;
-      for (int b = (int)B.depth - 1; b >= 1 && k == 0; --b) {
-        for (uint32_t j = 0; j < 2 && k == 0; ++j) {
-          uint32_t q = 2u * (uint32_t)(b - 1) + (j == 0 ? first : 1u - first);
-          uint32_t av = __shfl_sync(0xFFFFFFFFu, avail, q);
-          if (av == 0u) continue;
-          // atomicAdd claims pipeline in L2 (a compare-and-swap loop
-          // serialises thousands of warps); a claim that races past the
-          // reserved count waits for its slot or retires when the queue closes
-          k = min(nidle, av);
-          if (lane == 0) base = atomicAdd(&ctr[claimed_at(q)], k);
-          src = q;
-        }
+      const uint32_t some = __ballot_sync(0xFFFFFFFFu, avail != 0u);
+      if (some) {  // the deepest
+        const uint32_t at = 31u - __clz(some), q = 2u * at + KIND;
+        // atomicAdd claims pipeline in L2 (a compare-and-swap loop
+        // serialises thousands of warps); a claim that races past the
+        // reserved count waits for its slot or retires when the queue closes
+        k = min(nidle, __shfl_sync(0xFFFFFFFFu, avail, at));
+        if (lane == 0) base = atomicAdd(&ctr[claimed_at(q)], k);
+        src = q;
       }
       if (k == 0 && lane == 0 && !primary_done) {
-        base = atomicAdd(&ctr[kCursor], nidle);
-        k = base < B.total_pixels ? min(nidle, B.total_pixels - base) : 0u;
+        base = atomicAdd(&ctr[cursor_at(KIND)], nidle);
+        k = base < B.kind_pixels[KIND] ? min(nidle, B.kind_pixels[KIND] - base) : 0u;
         if (k) src = 0xFFFFFFFEu;
-        if (base + nidle >= B.total_pixels) primary_done = true;
+        if (base + nidle >= B.kind_pixels[KIND]) primary_done = true;
       }
       src = __shfl_sync(0xFFFFFFFFu, src, 0);
       base = __shfl_sync(0xFFFFFFFFu, base, 0);
@@ -405,22 +386,21 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
       uint32_t rank = __popc(idle & lt_mask);
       if (state == kIdle && rank < k) {
         if (src == 0xFFFFFFFEu) {
-          gpix = base + rank;
           bounce = 0;
-          scene = scene_of(sc, B.num_scenes, gpix);
-          kind = sc[scene].kind;
+          scene = scene_of_kind(sc, B.num_scenes, KIND, base + rank);
           const SceneDev& S = sc[scene];
-          uint32_t lp = gpix - S.pix_off;
+          const uint32_t lp = base + rank - S.kind_off[KIND];
+          gpix = S.pix_off + lp;
           V3 o, d;
           generate_ray(S.cam, S.w, S.h, lp % S.w, lp / S.w, o, d);
-          if (kind == kMesh) {
+          if (KIND == kMesh) {
             trav_init(tr, COUNT ? kd_of(S) : kd_entry_of(S), o, d, K_INF, 0u);
           } else {
             tr.o = o;
             tr.d = d;
             t = 0.f;
             steps = 0;
-            mode_tap = kMarch << 3;
+            tap = 0u;
           }
           state = kLive;
         } else if (base + rank < B.qcap[src]) {
@@ -431,123 +411,122 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
           pslot = base + rank;
           polls = 0;
           state = kPending;
-          kind = src & 1u;
         }
       }
     }
     if (__ballot_sync(0xFFFFFFFFu, state != kIdle) == 0u) {
-      // nothing in this warp: publish its finished counts, then leave once
-      // every bounce is closed (all created rays have finished)
+      // nothing in this warp: publish its finished counts and leave
       flush();
-      uint32_t leave = 0;
-      if (lane == 0) {
-        if (!primary_done) primary_done = ld_relaxed(&ctr[kCursor]) >= B.total_pixels;
-        if (primary_done) leave = (closed_mask(ctr, B) >> B.depth) & 1u;
-        if (!leave) {
-          __nanosleep(backoff);
-          backoff = min(2u * backoff, 4096u);
-        }
-      }
-      if (__shfl_sync(0xFFFFFFFFu, leave, 0)) break;
-      continue;
+      return any;
     }
-    backoff = 32;
-    // ---- one step of every live ray
+    any = true;
+    // ---- steps of the live rays: up to steps_per_trip leaves or field
+    // evaluations before the bookkeeping runs again, fewer once refill_min
+    // rays have ended (or all)
     bool done = false, hit = false;
+    const uint32_t nlive = __popc(__ballot_sync(0xFFFFFFFFu, state == kLive));
+    const uint32_t enough = min(B.refill_min, nlive);
+    if constexpr (KIND == kMesh) {
+      for (uint32_t it = 0; it < B.steps_per_trip; ++it) {
+        if (state == kLive && !done) {
+          const SceneDev& S = sc[scene];
+          // (a ray that misses the root box has no walk)
+          if (tr.live) trav_step<0, false, COUNT>(tr, kd_of(S), snodes + S.stage_off, cnt);
+          done = !tr.live;
+        }
+        if ((uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, done)) >= enough) break;
+      }
+    } else {
+      for (uint32_t it = 0; it < B.steps_per_trip; ++it) {
+        if (state == kLive && !done) {
+          const SceneDev& S = sc[scene];
+          const auto P = [&] {
+            if constexpr (TABLE == kFieldTables)
+              return FieldWords{(uint32_t)__cvta_generic_to_shared(sperm) +
+                                kFieldWordsBytes * S.perm_slot};
+            else if constexpr (TABLE == kWordTables)
+              return PermWords{sperm_w + 512u * S.perm_slot};
+            else
+              return PermBytes{sperm + 512u * S.perm_slot};
+          }();
+          // tap 0: marching; 1..6: the normal's taps about the hit at t
+          V3 q = v3(__fmaf_rn(t, tr.d.x, tr.o.x), __fmaf_rn(t, tr.d.y, tr.o.y),
+                    __fmaf_rn(t, tr.d.z, tr.o.z));
+          if (tap != 0u) {
+            const float delta = fmaxf(0.002f * t, 1e-3f);
+            const float sd = (tap & 1u) ? delta : -delta;
+            if (tap <= 2u) q.x = q.x + sd;
+            else if (tap <= 4u) q.y = q.y + sd;
+            else q.z = q.z + sd;
+          }
+          float v;
+          if constexpr (TABLE == kFieldTables)
+            v = terrain_density<1>(P, q, S.octaves, S.scale, S.amp);
+          else
+            v = terrain_density(P, q, S.octaves, S.scale, S.amp);
+          if (COUNT) ++cnt.status;  // field evaluations
+          if (tap == 0u) {
+            ++steps;
+            if (v < S.eps) {
+              v_hit = v;
+              tap = 1u;
+            } else {
+              t = __fmaf_rn(S.step_factor, v, t);
+              // going up above the ceiling it can only miss: stop early (the
+              // result, a miss with this direction, is what the march reaches)
+              if (t > S.tmax || steps >= S.max_steps || (tr.d.y >= 0.0f && q.y > S.ceiling))
+                done = true;
+            }
+          } else {
+            if (tap & 1u) {
+              plus = v;
+            } else {
+              const float diff = plus - v;
+              if (tap == 2u) tap_diff.x = diff;
+              else if (tap == 4u) tap_diff.y = diff;
+              else tap_diff.z = diff;
+            }
+            if (tap == 6u) done = hit = true;
+            else ++tap;
+          }
+        }
+        if ((uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, done)) >= enough) break;
+      }
+    }
+    // ---- the hits of the rays that have ended
     V3 n = {0.f, 0.f, 1.f}, hp = {0.f, 0.f, 0.f};
     uint32_t start_leaf = 0;
     float hit_t = 0.f, hit_u = 0.f, hit_v = 0.f;
     int32_t hit_id = -1;
-    if (state == kLive) {
-      const SceneDev& S = sc[scene];
-      if (kind == kMesh) {
-        KdDev kd = kd_of(S);
-        // up to steps_per_trip leaves before the warp's bookkeeping runs again
-        for (uint32_t it = 0; it < B.steps_per_trip && tr.live; ++it)
-          trav_step<0, false, COUNT>(tr, kd, snodes + S.stage_off, cnt);
-        if (!tr.live) {
-          done = true;
-          hit = tr.best_id >= 0;
-          if (hit) {
-            hit_t = tr.best_t;
-            hit_u = tr.best_u;
-            hit_v = tr.best_v;
-            hit_id = tr.best_id;
-            start_leaf = tr.best_leaf;
-            const float4* T = S.tris + 3 * (size_t)tr.best_ref;
-            float4 T1 = __ldg(T + 1), T2 = __ldg(T + 2);
-            n = normalize(cross(v3(T1.x, T1.y, T1.z), v3(T2.x, T2.y, T2.z)));
-            if (dot(n, tr.d) > 0.0f) n = v3(-n.x, -n.y, -n.z);
-            V3 q = v3(__fmaf_rn(hit_t, tr.d.x, tr.o.x), __fmaf_rn(hit_t, tr.d.y, tr.o.y),
-                      __fmaf_rn(hit_t, tr.d.z, tr.o.z));
-            hp = v3(__fmaf_rn(n.x, B.mesh_bias, q.x), __fmaf_rn(n.y, B.mesh_bias, q.y),
-                    __fmaf_rn(n.z, B.mesh_bias, q.z));
-          }
-        }
-      } else {
-        const auto P = [&] {
-          if constexpr (WORDS)
-            return PermWords{sperm_w + 512u * S.perm_slot};
-          else
-            return PermBytes{sperm + 512u * S.perm_slot};
-        }();
-        for (uint32_t it = 0; it < B.steps_per_trip && !done; ++it) {
-        V3 qp;
-        if ((mode_tap >> 3) == kMarch) {
-          qp = v3(__fmaf_rn(t, tr.d.x, tr.o.x), __fmaf_rn(t, tr.d.y, tr.o.y),
-                  __fmaf_rn(t, tr.d.z, tr.o.z));
-        } else {
-          uint32_t tap = mode_tap & 7u;
-          float sd = (tap & 1u) ? -delta : delta;
-          qp = p;
-          if (tap < 2) qp.x = p.x + sd;
-          else if (tap < 4) qp.y = p.y + sd;
-          else qp.z = p.z + sd;
-        }
-        float v = terrain_density(P, qp, S.octaves, S.scale, S.amp);
-        if (COUNT) ++cnt.status;  // field evaluations
-        if ((mode_tap >> 3) == kMarch) {
-          ++steps;
-          if (v < S.eps) {
-            p = qp;
-            v_hit = v;
-            delta = fmaxf(0.002f * t, 1e-3f);
-            mode_tap = kNormal << 3;  // tap 0
-          } else {
-            t = __fmaf_rn(S.step_factor, v, t);
-            // going up above the ceiling it can only miss: stop early (the
-            // result, a miss with this direction, is what the march reaches)
-            if (t > S.tmax || steps >= S.max_steps || (tr.d.y >= 0.0f && qp.y > S.ceiling))
-              done = true;
-          }
-        } else {
-          uint32_t tap = mode_tap & 7u;
-          if ((tap & 1u) == 0u) {
-            plus = v;
-          } else {
-            float diff = plus - v;
-            if (tap == 1) nx_bits = __float_as_uint(diff);
-            else if (tap == 3) ny_bits = __float_as_uint(diff);
-            else nz_bits = __float_as_int(diff);
-          }
-          if (tap == 5) {
-            float nx = __uint_as_float(nx_bits), ny = __uint_as_float(ny_bits),
-                  nz = __int_as_float(nz_bits);
-            done = true;
-            hit = true;
-            hit_t = t;
-            hit_id = 0;
-            float gl = sqrtf(__fmaf_rn(nz, nz, __fmaf_rn(ny, ny, nx * nx)));
-            n = normalize(v3(nx, ny, nz));
-            // leave the surface: the march may stop inside (v_hit < 0)
-            float off = fmaxf(-v_hit, 0.0f) / (gl / (2.0f * delta)) + 2e-3f;
-            hp = v3(__fmaf_rn(n.x, off, p.x), __fmaf_rn(n.y, off, p.y), __fmaf_rn(n.z, off, p.z));
-          } else {
-            ++mode_tap;
-          }
-        }
-        }
+    if constexpr (KIND == kMesh) {
+      hit = done && tr.best_id >= 0;
+      if (hit) {
+        hit_t = tr.best_t;
+        hit_u = tr.best_u;
+        hit_v = tr.best_v;
+        hit_id = tr.best_id;
+        start_leaf = tr.best_leaf;
+        const float4* T = sc[scene].tris + 3 * (size_t)tr.best_ref;
+        float4 T1 = __ldg(T + 1), T2 = __ldg(T + 2);
+        n = normalize(cross(v3(T1.x, T1.y, T1.z), v3(T2.x, T2.y, T2.z)));
+        if (dot(n, tr.d) > 0.0f) n = v3(-n.x, -n.y, -n.z);
+        V3 q = v3(__fmaf_rn(hit_t, tr.d.x, tr.o.x), __fmaf_rn(hit_t, tr.d.y, tr.o.y),
+                  __fmaf_rn(hit_t, tr.d.z, tr.o.z));
+        hp = v3(__fmaf_rn(n.x, B.mesh_bias, q.x), __fmaf_rn(n.y, B.mesh_bias, q.y),
+                __fmaf_rn(n.z, B.mesh_bias, q.z));
       }
+    } else if (hit) {
+      hit_t = t;
+      hit_id = 0;
+      const V3 p = v3(__fmaf_rn(t, tr.d.x, tr.o.x), __fmaf_rn(t, tr.d.y, tr.o.y),
+                      __fmaf_rn(t, tr.d.z, tr.o.z));
+      const float delta = fmaxf(0.002f * t, 1e-3f);
+      const float nx = tap_diff.x, ny = tap_diff.y, nz = tap_diff.z;
+      float gl = sqrtf(__fmaf_rn(nz, nz, __fmaf_rn(ny, ny, nx * nx)));
+      n = normalize(v3(nx, ny, nz));
+      // leave the surface: the march may stop inside (v_hit < 0)
+      float off = fmaxf(-v_hit, 0.0f) / (gl / (2.0f * delta)) + 2e-3f;
+      hp = v3(__fmaf_rn(n.x, off, p.x), __fmaf_rn(n.y, off, p.y), __fmaf_rn(n.z, off, p.z));
     }
     // ---- finished rays: write or continue the path
     bool push = false;
@@ -561,7 +540,7 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
       if (hit && bounce + 1u < B.depth) {
         V3 nd = cosine_dir(n, B.seed, gpix, bounce);
         push = true;
-        qn = 2u * bounce + kind;
+        qn = 2u * bounce + KIND;
         R0 = make_float4(hp.x, hp.y, hp.z, __uint_as_float(start_leaf));
         R1 = make_float4(nd.x, nd.y, nd.z, __uint_as_float(gpix | ((bounce + 1u) << 28)));
       } else {
@@ -597,6 +576,83 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
     if (__shfl_sync(0xFFFFFFFFu, fin_pending, 0) >= 1024u) flush();
   }
   flush();
+  return any;
+}
+
+// Launch bounds: blocks of up to 256 threads, 4 resident per SM (64
+// registers, 32 warps per SM).  Measured on the 8-scene batch: 22.0 ms
+// against 30.4 ms with 122 registers and 16 warps, despite the spills.
+#ifndef RE_BATCH_MIN_BLOCKS
+#define RE_BATCH_MIN_BLOCKS 4
+#endif
+#ifndef RE_BATCH_MAX_THREADS
+#define RE_BATCH_MAX_THREADS 256
+#endif
+
+template <bool COUNT, int TABLE>
+__global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_batch(BatchDev B) {
+  extern __shared__ uint4 smem_u4[];
+  SceneDev* sc = reinterpret_cast<SceneDev*>(smem_u4);
+  uint8_t* sperm = reinterpret_cast<uint8_t*>(sc + B.num_scenes);
+  uint32_t* sperm_w = reinterpret_cast<uint32_t*>(sperm);
+  uint2* snodes = reinterpret_cast<uint2*>(sperm + table_bytes(TABLE) * B.perm_count);
+  uint32_t* sfin = reinterpret_cast<uint32_t*>(snodes + B.stage_total);  // [warp][bounce]
+  {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(B.scenes);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(sc);
+    for (uint32_t i = threadIdx.x; i < B.num_scenes * (uint32_t)(sizeof(SceneDev) / 4); i += blockDim.x)
+      dst[i] = src[i];
+    for (uint32_t i = threadIdx.x; i < 512u * B.perm_count; i += blockDim.x) {
+      if (TABLE == kFieldTables) {
+        const uint32_t j = i & 511u, p = B.perms[i], q = B.perms[i - j + ((j + 1u) & 511u)];
+        uint32_t* t = sperm_w + (i >> 9) * (kFieldWordsBytes / 4u);
+        t[j] = field_a_word<4>(p, q);
+        t[512u + j] = grad_bytes(p);
+      } else if (TABLE == kWordTables) {
+        sperm_w[i] = perm_word(B.perms[i]);
+      } else {
+        sperm[i] = B.perms[i];
+      }
+    }
+    for (uint32_t i = threadIdx.x; i < (blockDim.x / 32u) * kMaxDepth; i += blockDim.x) sfin[i] = 0u;
+    __syncthreads();
+    for (uint32_t s = 0; s < B.num_scenes; ++s)
+      for (uint32_t i = threadIdx.x; i < sc[s].stage; i += blockDim.x)
+        snodes[sc[s].stage_off + i] = __ldg(&sc[s].nodes[i]);
+    __syncthreads();
+  }
+  uint32_t* ctr = B.ctr;
+  const uint32_t epoch = ld_relaxed(&ctr[kEpoch]);
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t nq = 2u * (B.depth - 1u);
+  uint32_t* wfin = sfin + (threadIdx.x >> 5) * kMaxDepth;  // this warp's unpublished counts
+  Counters cnt = {0, 0, 0, 0};
+  uint32_t errors = 0, trip = 0;
+  // Neighbouring warps start on different kinds, so that an SM's walks
+  // (bound by latency) and marches (by the FP32 pipes) run side by side; a
+  // warp that finds nothing to do changes over, and leaves once both are done.
+  uint32_t kind = TABLE == kNoTables ? kMesh : (threadIdx.x >> 5) & 1u;
+  uint32_t backoff = 32, dry = 0;
+  for (; trip < B.loop_bound; ++trip) {
+    bool any;
+    if (TABLE == kNoTables || kind == kMesh)
+      any = run_kind<COUNT, TABLE, kMesh>(B, sc, sperm, snodes, wfin, epoch, trip, cnt, errors);
+    else
+      any = run_kind<COUNT, TABLE, kTerrain>(B, sc, sperm, snodes, wfin, epoch, trip, cnt, errors);
+    if (trip >= B.loop_bound) break;
+    dry = any ? 0u : dry + 1u;
+    if (any) backoff = 32;
+    if (TABLE != kNoTables) kind ^= 1u;
+    if (dry >= 2u) {
+      uint32_t leave = 0;
+      if (lane == 0) {
+        leave = (closed_mask(ctr, B, kMesh) & closed_mask(ctr, B, kTerrain)) >> B.depth & 1u;
+        if (!leave) __nanosleep(backoff);
+      }
+      backoff = min(2u * backoff, 4096u);
+      if (__shfl_sync(0xFFFFFFFFu, leave, 0)) break;
+    }
+  }
   if (trip >= B.loop_bound) errors = 1;
   if (COUNT) {
     uint32_t v4[4] = {cnt.inner, cnt.leaf, cnt.tests, cnt.status};
@@ -619,10 +675,11 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
         ctr[reserved_at(q)] = 0u;
         ctr[claimed_at(q)] = 0u;
       }
-      for (uint32_t b = 0; b < kMaxDepth; ++b) ctr[fin_at(b)] = 0u;
-      ctr[kStatsPrimary] = min(ctr[kCursor], B.total_pixels);
+      for (uint32_t b = 0; b < kMaxDepth; ++b) ctr[fin_at(b, 0)] = ctr[fin_at(b, 1)] = 0u;
+      ctr[kStatsPrimary] = min(ctr[cursor_at(0)], B.kind_pixels[0]) +
+                           min(ctr[cursor_at(1)], B.kind_pixels[1]);
       ctr[kStatsError] = ctr[kError];
-      ctr[kCursor] = 0u;
+      ctr[cursor_at(0)] = ctr[cursor_at(1)] = 0u;
       ctr[kError] = 0u;
       ctr[kDone] = 0u;
       __threadfence();
@@ -705,14 +762,31 @@ uint32_t layout_stage(re_batch* b, uint32_t stage_nodes) {
   return off;
 }
 
-// Word tables while the batch has at most this many terrain seeds (32 KB).
-constexpr uint32_t kWordTablesMax = 16;
+// The largest tables that leave room for four blocks per SM: the paired
+// form's up to 12 seeds (48 KB), words up to 16 (32 KB).
+constexpr uint32_t kFieldTablesMax = 12, kWordTablesMax = 16;
 
-bool word_tables(const re_batch* b) { return b->perms.size() / 512 <= kWordTablesMax; }
+int table_of(const re_batch* b) {
+  const size_t seeds = b->perms.size() / 512;
+  return seeds == 0                 ? kNoTables
+         : seeds <= kFieldTablesMax ? kFieldTables
+         : seeds <= kWordTablesMax  ? kWordTables
+                                    : kByteTables;
+}
 
 size_t smem_bytes(const re_batch* b, uint32_t stage_total, uint32_t block_threads) {
-  return b->num_scenes * sizeof(SceneDev) + (word_tables(b) ? 4u : 1u) * b->perms.size() +
+  return b->num_scenes * sizeof(SceneDev) + b->perms.size() / 512 * table_bytes(table_of(b)) +
          (size_t)stage_total * sizeof(uint2) + (size_t)(block_threads / 32) * kMaxDepth * 4;
+}
+
+using Kernel = void (*)(BatchDev);
+Kernel kernel_of(const re_batch* b, bool count) {
+  switch (table_of(b)) {
+    case kFieldTables: return count ? k_batch<true, kFieldTables> : k_batch<false, kFieldTables>;
+    case kWordTables: return count ? k_batch<true, kWordTables> : k_batch<false, kWordTables>;
+    case kNoTables: return count ? k_batch<true, kNoTables> : k_batch<false, kNoTables>;
+    default: return count ? k_batch<true, kByteTables> : k_batch<false, kByteTables>;
+  }
 }
 
 // Scene table (with this tuning's staging offsets) to the device and the
@@ -723,10 +797,9 @@ re_status prepare(re_batch* b, const re_batch_tuning& tn, cudaStream_t st) {
                           cudaMemcpyHostToDevice, st));
   RE_CUDA(cudaStreamSynchronize(st));
   int bytes = (int)smem_bytes(b, stage_total, 512);
-  RE_CUDA(cudaFuncSetAttribute(k_batch<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  RE_CUDA(cudaFuncSetAttribute(k_batch<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  RE_CUDA(cudaFuncSetAttribute(k_batch<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  RE_CUDA(cudaFuncSetAttribute(k_batch<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  for (bool count : {false, true})
+    RE_CUDA(cudaFuncSetAttribute(kernel_of(b, count), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 bytes));
   return RE_OK;
 }
 
@@ -736,8 +809,7 @@ re_status launch(re_batch* b, float* d_radiance, re_hit* d_primary, cudaStream_t
   uint32_t stage_total = layout_stage(b, tn.stage_nodes);
   size_t smem = smem_bytes(b, stage_total, tn.block_threads);
   int per_sm = 0;
-  auto kern = word_tables(b) ? (totals ? k_batch<true, true> : k_batch<false, true>)
-                             : (totals ? k_batch<true, false> : k_batch<false, false>);
+  const Kernel kern = kernel_of(b, totals != nullptr);
   RE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)tn.block_threads,
                                                         smem));
   if (per_sm < 1) return fail(RE_ERR_LIMIT, "re_batch: tuning does not fit on an SM");
@@ -747,7 +819,7 @@ re_status launch(re_batch* b, float* d_radiance, re_hit* d_primary, cudaStream_t
   B.num_scenes = b->num_scenes;
   B.perm_count = (uint32_t)(b->perms.size() / 512);
   B.stage_total = stage_total;
-  B.total_pixels = (uint32_t)b->total_pixels;
+  for (int k = 0; k < 2; ++k) B.kind_pixels[k] = (uint32_t)b->cap[k];
   B.depth = b->depth;
   B.seed = b->seed;
   B.refill_min = tn.refill_min;
@@ -820,6 +892,7 @@ RE_API re_status re_batch_create(const re_batch_scene* scenes, uint32_t n, const
     d.kind = s.kind;
     d.albedo = s.albedo;
     d.pix_off = (uint32_t)off;
+    for (int k = 0; k < 2; ++k) d.kind_off[k] = (uint32_t)b->cap[k];
     if (s.kind == RE_BATCH_MESH) {
       const re_scene* m = s.mesh;
       int dev = -1;

@@ -197,6 +197,7 @@ __device__ __forceinline__ float terrain_density(const PT& P, V3 p,
 // left (the scalar form of this layout: 29.9 G/s).  Frames, before and after:
 // the 1080p terrain 3.18 -> 2.56 ms, the shaded terrain at 1366x768 2.65 ->
 // 2.10 ms, the 1080p neural tracer 2.27 -> 1.85 ms.
+// FieldTable<STRIDE, G>: rows STRIDE bytes apart, G words G bytes past A words.
 constexpr uint32_t kRowBytes = 256;
 constexpr uint32_t kRowsSmemBytes = 512 * kRowBytes;
 // One block per SM, whose warps share the table.  640 threads: 5 warps per
@@ -205,9 +206,21 @@ constexpr uint32_t kRowsSmemBytes = 512 * kRowBytes;
 // with four pairs unrolled 2.56.
 constexpr uint32_t kRowsThreads = 640;
 
-struct FieldRows {
+template <uint32_t STRIDE, uint32_t G>
+struct FieldTable {
   uint32_t base;  // shared-memory address of this lane's column
 };
+using FieldRows = FieldTable<kRowBytes, 128>;
+
+// One copy of the table per seed, 512 A words then 512 G words (the batched
+// renderer, which holds several seeds; lanes may meet in a bank).
+constexpr uint32_t kFieldWordsBytes = 2 * 512 * 4;
+using FieldWords = FieldTable<4, 2048>;
+
+template <uint32_t STRIDE>
+__host__ __device__ __forceinline__ uint32_t field_a_word(uint32_t p, uint32_t next) {
+  return p * STRIDE | (next * STRIDE) << 16;
+}
 
 __host__ __device__ __forceinline__ uint32_t grad_bytes(uint32_t p) {
   const uint32_t h = perm_word(p) >> 28;  // bit 0: first is y, 1: second is y, 2, 3: negated
@@ -222,7 +235,7 @@ __device__ __forceinline__ FieldRows load_rows(const PermTable& t, uint32_t* sme
   const uint32_t lane = threadIdx.x & 31u;
   for (uint32_t j = threadIdx.x >> 5; j < 512u; j += blockDim.x >> 5) {
     const uint32_t p = t.p[j], q = t.p[(j + 1u) & 511u];
-    smem[64u * j + lane] = (p << 8) | (q << 24);
+    smem[64u * j + lane] = field_a_word<kRowBytes>(p, q);
     smem[64u * j + 32u + lane] = grad_bytes(p);
   }
   __syncthreads();
@@ -274,11 +287,11 @@ __device__ __forceinline__ uint32_t row_word(uint32_t addr) {
 // The 8 corner G words of the cell whose masked indices are the low bytes of
 // x, y and z (corner order a..h: x fastest, then y, z).  Every row index is
 // a sum of two bytes, at most 510, and a corner at z + 1 is the next row.
-__device__ __forceinline__ void cell_words(const FieldRows& R, uint32_t x, uint32_t y, uint32_t z,
-                                           uint32_t (&g)[8]) {
-  constexpr uint32_t G = 128;
-  const uint32_t wx = row_word<0>((x & 255u) * kRowBytes + R.base);
-  const uint32_t ry = (y & 255u) * kRowBytes + R.base, rz = (z & 255u) * kRowBytes + R.base;
+template <uint32_t STRIDE, uint32_t G>
+__device__ __forceinline__ void cell_words(const FieldTable<STRIDE, G>& R, uint32_t x, uint32_t y,
+                                           uint32_t z, uint32_t (&g)[8]) {
+  const uint32_t wx = row_word<0>((x & 255u) * STRIDE + R.base);
+  const uint32_t ry = (y & 255u) * STRIDE + R.base, rz = (z & 255u) * STRIDE + R.base;
   const uint32_t w0 = row_word<0>(__dp2a_lo(wx, 1u, ry)), w1 = row_word<0>((wx >> 16) + ry);
   const uint32_t r00 = __dp2a_lo(w0, 1u, rz), r01 = (w0 >> 16) + rz;
   const uint32_t r10 = __dp2a_lo(w1, 1u, rz), r11 = (w1 >> 16) + rz;
@@ -286,10 +299,10 @@ __device__ __forceinline__ void cell_words(const FieldRows& R, uint32_t x, uint3
   g[1] = row_word<G>(r10);
   g[2] = row_word<G>(r01);
   g[3] = row_word<G>(r11);
-  g[4] = row_word<G + kRowBytes>(r00);
-  g[5] = row_word<G + kRowBytes>(r10);
-  g[6] = row_word<G + kRowBytes>(r01);
-  g[7] = row_word<G + kRowBytes>(r11);
+  g[4] = row_word<G + STRIDE>(r00);
+  g[5] = row_word<G + STRIDE>(r10);
+  g[6] = row_word<G + STRIDE>(r01);
+  g[7] = row_word<G + STRIDE>(r11);
 }
 
 // Twice the corner values of both octaves.
@@ -309,7 +322,8 @@ __device__ __forceinline__ f32x2 quintic2(f32x2 t) {
 }
 
 // Twice the noise of two octaves; every coordinate below 2^22.
-__device__ __forceinline__ f32x2 perlin2(const FieldRows& R, f32x2 x, f32x2 y, f32x2 z) {
+template <class FT>
+__device__ __forceinline__ f32x2 perlin2(const FT& R, f32x2 x, f32x2 y, f32x2 z) {
   const f32x2 kInt = pack2(12582912.0f, 12582912.0f), kOne = pack2(1.0f, 1.0f);
   const f32x2 ix = add2_down(x, kInt), iy = add2_down(y, kInt), iz = add2_down(z, kInt);
   const f32x2 tx = sub2(x, sub2(ix, kInt)), ty = sub2(y, sub2(iy, kInt)),
@@ -337,20 +351,22 @@ __device__ __forceinline__ f32x2 perlin2(const FieldRows& R, f32x2 x, f32x2 y, f
   return fma2(k7, mul2(mul2(u, v), w), r);
 }
 
-// perlin()'s view of the rows.
+// perlin()'s view of the table.
+template <uint32_t STRIDE>
 struct PermRows {
   uint32_t base;
   __device__ __forceinline__ uint32_t idx(uint32_t j) const {
-    return (row_word<0>(base + j * kRowBytes) >> 8) & 255u;
+    return (row_word<0>(base + j * STRIDE) & 0xFFFFu) / STRIDE;
   }
   __device__ __forceinline__ uint32_t grad(uint32_t j) const { return perm_word(idx(j)); }
 };
 
 // fbm() at any coordinates (infinities and NaN among them); out of line, so
 // that the callers' registers are those of the near form.
+template <uint32_t STRIDE>
 static __device__ __noinline__ float field_far(uint32_t base, float x, float y, float z,
                                                uint32_t octaves) {
-  PermRows P{base};
+  PermRows<STRIDE> P{base};
   float sum = 0.0f, amp = 1.0f;
 #pragma unroll 1
   for (uint32_t i = 0; i < octaves; ++i) {
@@ -366,8 +382,10 @@ static __device__ __noinline__ float field_far(uint32_t base, float x, float y, 
 // terrain_density() on the rows.  The near form evaluates octaves in pairs,
 // an odd last one with an octave past it at amplitude zero, so the largest
 // coordinate it meets is below 2^octaves times the first one's.
-__device__ __forceinline__ float terrain_density(const FieldRows& R, V3 p, uint32_t octaves,
-                                                 float scale, float amp) {
+// UNROLL: pairs in the code at once.
+template <int UNROLL = 4, uint32_t STRIDE, uint32_t G>
+__device__ __forceinline__ float terrain_density(const FieldTable<STRIDE, G>& R, V3 p,
+                                                 uint32_t octaves, float scale, float amp) {
   const float x = scale * p.x, y = scale * p.y, z = scale * p.z;
   // 2^(22 - octaves), octaves <= 32
   const float lim = __uint_as_float((127u + 22u - octaves) << 23);
@@ -376,7 +394,7 @@ __device__ __forceinline__ float terrain_density(const FieldRows& R, V3 p, uint3
     const f32x2 kFour = pack2(4.0f, 4.0f);
     f32x2 X = pack2(x, 2.0f * x), Y = pack2(y, 2.0f * y), Z = pack2(z, 2.0f * z);
     float a = 0.5f;
-#pragma unroll 4
+#pragma unroll UNROLL
     for (uint32_t i = 0; i < octaves; i += 2) {
       float r0, r1;
       unpack2(perlin2(R, X, Y, Z), r0, r1);
@@ -388,7 +406,7 @@ __device__ __forceinline__ float terrain_density(const FieldRows& R, V3 p, uint3
       Z = mul2(Z, kFour);
     }
   } else {
-    sum = field_far(R.base, x, y, z, octaves);
+    sum = field_far<STRIDE>(R.base, x, y, z, octaves);
   }
   return __fmaf_rn(-amp, sum, p.y);
 }
