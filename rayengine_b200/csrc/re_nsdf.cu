@@ -1487,8 +1487,8 @@ constexpr uint32_t kRefineSmemBytes = kRowsSmemBytes + (kRowsThreads / 32) * 64 
 // the analytic-gradient form (1) carries no stencil state.
 template <uint32_t NT>
 __global__ void __launch_bounds__(kRowsThreads) k_sdf_refine(
-    PermTable perm, FieldDev f, RefineDev rd, CamDev cam, uint32_t w, uint32_t h, int direct,
-    const uint4* __restrict__ queue, uint32_t* __restrict__ counters,
+    PermTable perm, FieldDev f, RefineDev rd, CamDev cam, uint32_t w, uint32_t h, RowsSpread spread,
+    int direct, const uint4* __restrict__ queue, uint32_t* __restrict__ counters,
     unsigned long long* __restrict__ totals, float4* __restrict__ out) {
   extern __shared__ uint32_t rows_smem[];
   // Per-warp ring of set-up rays (64 entries): the warp claims 32 work
@@ -1502,10 +1502,12 @@ __global__ void __launch_bounds__(kRowsThreads) k_sdf_refine(
   uint4(*ring_b)[64] = reinterpret_cast<uint4(*)[64]>(ring_a + kRowsThreads / 32);
   const FieldRows P = load_rows(perm, rows_smem);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  if (warp >= spread.warps) return;
   // direct mode claims pixels in 8x4 tiles (claim i = lane i & 31 of tile
   // i >> 5), so a warp's rays start close together
   const uint32_t dtiles_x = (w + 7) / 8;
   const uint32_t total = direct ? dtiles_x * ((h + 3) / 4) * 32u : counters[1];
+  const bool holds = lane < spread.rays;  // may hold a ray
   bool live = false, claimed_all = false, have_lo = false, restarted = false;
   uint32_t head = 0, tail = 0;  // ring positions (warp-uniform)
   uint32_t pix = 0, steps = 0, base_steps = 0, mode = kMarch, tap = 0, iters = 0;
@@ -1515,15 +1517,15 @@ __global__ void __launch_bounds__(kRowsThreads) k_sdf_refine(
   float nx = 0.f, ny = 0.f, nz = 0.f, plus = 0.f;
   uint32_t n_exact = 0, n_normal = 0;  // evaluations: march/probe/root, normal taps
   for (;;) {
-    uint32_t idle = __ballot_sync(0xFFFFFFFFu, !live);
+    uint32_t idle = __ballot_sync(0xFFFFFFFFu, holds && !live);
     uint32_t nidle = __popc(idle);
     if (nidle >= 4u && (!claimed_all || head != tail)) {
       if (tail - head < nidle && !claimed_all) {
         uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(&counters[2], 32u);
+        if (lane == 0) base = atomicAdd(&counters[2], spread.rays);
         base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base + 32u >= total) claimed_all = true;
-        const uint32_t i = base + lane;
+        if (base + spread.rays >= total) claimed_all = true;
+        const uint32_t i = lane < spread.rays ? base + lane : total;
         uint32_t dx = 0, dy = 0;
         if (direct) {
           dx = ((i >> 5) % dtiles_x) * 8 + (i & 7u);
@@ -1546,10 +1548,10 @@ __global__ void __launch_bounds__(kRowsThreads) k_sdf_refine(
         ring_a[warp][(tail + lane) & 63u] = ea;
         ring_b[warp][(tail + lane) & 63u] = eb;
         __syncwarp();
-        tail += 32u;
+        tail += spread.rays;
       }
       const uint32_t avail = tail - head;
-      if (!live) {
+      if ((idle >> lane) & 1u) {
         const uint32_t r = __popc(idle & ((1u << lane) - 1u));
         if (r < avail) {
           const float4 ea = ring_a[warp][(head + r) & 63u];
@@ -1575,7 +1577,6 @@ __global__ void __launch_bounds__(kRowsThreads) k_sdf_refine(
       if (claimed_all && head == tail) break;
       continue;
     }
-    if (!live) continue;
     V3 qp;
     if (mode == kMarch) {
       qp = v3(__fmaf_rn(t, d.x, o.x), __fmaf_rn(t, d.y, o.y), __fmaf_rn(t, d.z, o.z));
@@ -1593,7 +1594,8 @@ __global__ void __launch_bounds__(kRowsThreads) k_sdf_refine(
       else if (tap < 4) qp.y = p.y + sd;
       else qp.z = p.z + sd;
     }
-    float v = terrain_density(P, qp, f.octaves, f.scale, f.amp);
+    float v = warp_density(P, qp, live, f.octaves, f.scale, f.amp);
+    if (!live) continue;
     if (NT != 1u && mode == kNormal) ++n_normal;
     else ++n_exact;
     uint32_t status = 3;  // 3 = still running
@@ -2447,6 +2449,7 @@ RE_API re_status re_nsdf_trace_exact(re_nsdf* s, const re_sdf_params* field,
   rd.cone_tiles_x = cone ? s->cone_tiles_x : 0u;
   kr<<<re::sm_count(), re::kRowsThreads, re::nsdf::kRefineSmemBytes, cs>>>(
       re::perm_of(field->seed), re::field_of(*field), rd, re::cam_dev(*cam), w, h,
+      re::rows_spread((uint64_t)w * h, (uint32_t)re::sm_count()),
       exact_only || cone ? 1 : 0, s->queue, s->counters, totals, reinterpret_cast<float4*>(d_out));
   RE_CHECK_LAUNCH("re_nsdf_trace_exact: refine launch");
   if (rd.normal_taps == 1u) {

@@ -124,24 +124,25 @@ __device__ __forceinline__ void light_setup(const ShadeDev& S, V3 p, V3& L, floa
   ldz = ld.z;
 }
 
-// One step: returns false when the march is over (step bound, range, or the
-// ray is occluded: prel = 0).  The march starts with t = shadow_tmin,
-// prel = 1, i = 0.
-template <class PT>
-__device__ __forceinline__ bool shadow_step(const PT& P, const ShadeDev& S, V3 p, V3 L, float& t,
-                                            float& prel, uint32_t& i, uint32_t& evals) {
-  if (!(i < S.shadow_max_steps && t < S.shadow_tmax)) return false;
+// One step of a live lane's march; all 32 lanes call it.  live turns false
+// when the march is over (step bound, range, or the ray is occluded: prel =
+// 0).  The march starts with t = shadow_tmin, prel = 1, i = 0.
+__device__ __forceinline__ void shadow_step(const FieldRows& P, const ShadeDev& S, V3 p, V3 L,
+                                            bool& live, float& t, float& prel, uint32_t& i,
+                                            uint32_t& evals) {
+  live = live && i < S.shadow_max_steps && t < S.shadow_tmax;
   V3 q = {__fmaf_rn(t, L.x, p.x), __fmaf_rn(t, L.y, p.y), __fmaf_rn(t, L.z, p.z)};
-  float dd = terrain_density(P, q, S.octaves, S.scale, S.amp);
+  float dd = warp_density(P, q, live, S.octaves, S.scale, S.amp);
+  if (!live) return;
   ++evals;
   ++i;
   if (prel < kEps || dd <= 1e-5f) {
     prel = 0.0f;
-    return false;
+    live = false;
+    return;
   }
   prel = fminf(prel, (S.soft_k * dd) / t);
   t = __fmaf_rn(S.step_factor, dd, t);
-  return true;
 }
 
 __device__ __forceinline__ V3 light_terms(const ShadeDev& S, float prel, V3 n, V3 L, float ldx,
@@ -302,11 +303,12 @@ __device__ __forceinline__ uint32_t finish_pixel(const ShadeDev& S, V3 col, V3 o
 constexpr uint32_t kShadeRefill = 4;
 
 __global__ void __launch_bounds__(kRowsThreads) k_sdf_shadow(
-    PermTable perm, ShadeDev S, uint32_t w, uint32_t h, const float4* __restrict__ hits,
-    uint32_t* __restrict__ rgba, uint32_t* __restrict__ cursor,
+    PermTable perm, ShadeDev S, uint32_t w, uint32_t h, RowsSpread spread,
+    const float4* __restrict__ hits, uint32_t* __restrict__ rgba, uint32_t* __restrict__ cursor,
     unsigned long long* __restrict__ evals_out) {
   extern __shared__ uint32_t rows_smem[];
   const FieldRows P = load_rows(perm, rows_smem);
+  if ((threadIdx.x >> 5) >= spread.warps) return;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t tiles_x = (w + 7) / 8;
   const uint32_t total = tiles_x * ((h + 3) / 4) * 32u;
@@ -316,14 +318,14 @@ __global__ void __launch_bounds__(kRowsThreads) k_sdf_shadow(
   V3 p = {0.f, 0.f, 0.f}, L = p;
   float ldx = 0.f, ldz = 0.f, t = 0.f, prel = 0.f;
   for (;;) {
-    uint32_t idle = __ballot_sync(0xFFFFFFFFu, !live);
+    uint32_t idle = __ballot_sync(0xFFFFFFFFu, !live && lane < spread.rays);
     uint32_t nidle = __popc(idle);
-    if (!exhausted && (nidle >= kShadeRefill || nidle == 32u)) {
+    if (!exhausted && nidle >= kShadeRefill) {
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(cursor, nidle);
       base = __shfl_sync(0xFFFFFFFFu, base, 0);
       if (base + nidle >= total) exhausted = true;
-      if (!live) {
+      if ((idle >> lane) & 1u) {
         uint32_t k = base + __popc(idle & ((1u << lane) - 1u));
         uint32_t tile = k >> 5, l = k & 31u;
         uint32_t x = (tile % tiles_x) * 8 + (l & 7u), y = (tile / tiles_x) * 4 + (l >> 3);
@@ -346,10 +348,9 @@ __global__ void __launch_bounds__(kRowsThreads) k_sdf_shadow(
       if (exhausted) break;
       continue;
     }
-    if (live && !shadow_step(P, S, p, L, t, prel, i, evals)) {
-      rgba[pix] = __float_as_uint(prel);
-      live = false;
-    }
+    const bool was = live;
+    shadow_step(P, S, p, L, live, t, prel, i, evals);
+    if (was && !live) rgba[pix] = __float_as_uint(prel);
   }
   if (evals_out) {
     uint32_t s = __reduce_add_sync(0xFFFFFFFFu, evals);
@@ -476,8 +477,10 @@ re_status shade(const re_sdf_params& f, const re_sdf_shade_params& s, const re_c
     RE_CUDA(cudaFuncSetAttribute(k_sdf_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kRowsSmemBytes));
     k_sdf_shadow<<<sm_count(), kRowsThreads, kRowsSmemBytes, st>>>(
-        perm_table(f.seed), shade_dev(f, s), w, h, reinterpret_cast<const float4*>(d_hits),
-        d_rgba, ctr, reinterpret_cast<unsigned long long*>(d_evals));
+        perm_table(f.seed), shade_dev(f, s), w, h,
+        rows_spread((uint64_t)w * h, (uint32_t)sm_count()),
+        reinterpret_cast<const float4*>(d_hits), d_rgba, ctr,
+        reinterpret_cast<unsigned long long*>(d_evals));
     RE_CHECK_LAUNCH("re_render_sdf_frame: shadow launch");
   }
   int fin_sm = 0;

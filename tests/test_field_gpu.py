@@ -4,6 +4,7 @@ coordinates below, across and beyond the range of the paired form (the
 largest |scale * p| times 2^octaves below 2^22) on both sides of zero."""
 import numpy as np
 import pytest
+import torch
 
 import rayengine_b200 as rb
 from oracle import pyoracle as po
@@ -40,3 +41,24 @@ def test_across_the_paired_range(cuda, octaves, axis, sign):
 
 def test_far_from_the_origin(cuda):
     _bake(8, 1.0, (3.0, 1024.0, 513.0), (3.0e6, -3.0, -7.0e8))
+
+
+# pixels at and past 8 and 16 rays for each of 148 x 20 warps, where a frame's
+# rays go from four lanes each to two and one, and frames of a few rays
+@pytest.mark.parametrize("w,h,octaves", [(2, 2, 8), (37, 5, 9), (64, 36, 7), (160, 148, 8),
+                                         (161, 148, 8), (320, 148, 8), (321, 148, 8)])
+def test_frames_of_few_rays(cuda, w, h, octaves):
+    cfg = rb.configs.TerrainConfig(width=w, height=h, octaves=octaves)
+    shade = rb.sdf_shade_params()
+    img, hits = rb.render_sdf_frame(cfg.params(), shade, cfg.camera(), w, h)
+    plain = rb.sphere_trace(cfg.params(), cfg.camera(), w, h)
+    assert torch.equal(plain, hits)
+    ref = po.sdf_image(po.perm(cfg.seed), cfg.camera(), w, h, octaves=octaves)
+    u = plain.cpu().numpy().view(np.uint32).reshape(-1, 8)
+    assert np.array_equal(u[:, 6], ref["steps"])
+    assert np.array_equal(u[:, 7], ref["status"])
+    hit = ref["status"] == 1
+    assert np.array_equal(u[hit, 0:3], ref["pos"][hit].view(np.uint32))
+    assert np.array_equal(u[hit, 3:6], ref["normal"][hit].view(np.uint32))
+    want = po.sdf_frame(po.perm(cfg.seed), cfg.camera(), w, h, cfg.params(), shade)
+    assert np.array_equal(img.cpu().numpy().view(np.uint32), want)
