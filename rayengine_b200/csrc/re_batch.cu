@@ -438,32 +438,34 @@ __device__ __forceinline__ bool run_kind(const BatchDev& B, const SceneDev* sc,
       }
     } else {
       for (uint32_t it = 0; it < B.steps_per_trip; ++it) {
-        if (state == kLive && !done) {
-          const SceneDev& S = sc[scene];
-          const auto P = [&] {
-            if constexpr (TABLE == kFieldTables)
-              return FieldWords{(uint32_t)__cvta_generic_to_shared(sperm) +
-                                kFieldWordsBytes * S.perm_slot};
-            else if constexpr (TABLE == kWordTables)
-              return PermWords{sperm_w + 512u * S.perm_slot};
-            else
-              return PermBytes{sperm + 512u * S.perm_slot};
-          }();
-          // tap 0: marching; 1..6: the normal's taps about the hit at t
-          V3 q = v3(__fmaf_rn(t, tr.d.x, tr.o.x), __fmaf_rn(t, tr.d.y, tr.o.y),
-                    __fmaf_rn(t, tr.d.z, tr.o.z));
-          if (tap != 0u) {
-            const float delta = fmaxf(0.002f * t, 1e-3f);
-            const float sd = (tap & 1u) ? delta : -delta;
-            if (tap <= 2u) q.x = q.x + sd;
-            else if (tap <= 4u) q.y = q.y + sd;
-            else q.z = q.z + sd;
-          }
-          float v;
-          if constexpr (TABLE == kFieldTables)
-            v = terrain_density<1>(P, q, S.octaves, S.scale, S.amp);
+        const bool runs = state == kLive && !done;
+        const SceneDev& S = sc[scene];
+        // tap 0: marching; 1..6: the normal's taps about the hit at t
+        V3 q = v3(__fmaf_rn(t, tr.d.x, tr.o.x), __fmaf_rn(t, tr.d.y, tr.o.y),
+                  __fmaf_rn(t, tr.d.z, tr.o.z));
+        if (runs && tap != 0u) {
+          const float delta = fmaxf(0.002f * t, 1e-3f);
+          const float sd = (tap & 1u) ? delta : -delta;
+          q.x = tap - 1u < 2u ? q.x + sd : q.x;
+          q.y = tap - 3u < 2u ? q.y + sd : q.y;
+          q.z = tap - 5u < 2u ? q.z + sd : q.z;
+        }
+        float v = 0.f;
+        if constexpr (TABLE == kFieldTables) {
+          const FieldWords P{(uint32_t)__cvta_generic_to_shared(sperm) +
+                             kFieldWordsBytes * S.perm_slot};
+          // with two lanes to a point as well, six scenes took 3.08 ms against
+          // 2.62: the mesh walk's code runs beside this on every SM
+          v = warp_density<1, false>(P, q, runs, S.octaves, S.scale, S.amp);
+        } else if (runs) {
+          if constexpr (TABLE == kWordTables)
+            v = terrain_density(PermWords{sperm_w + 512u * S.perm_slot}, q, S.octaves, S.scale,
+                                S.amp);
           else
-            v = terrain_density(P, q, S.octaves, S.scale, S.amp);
+            v = terrain_density(PermBytes{sperm + 512u * S.perm_slot}, q, S.octaves, S.scale,
+                                S.amp);
+        }
+        if (runs) {
           if (COUNT) ++cnt.status;  // field evaluations
           if (tap == 0u) {
             ++steps;

@@ -442,31 +442,41 @@ __device__ __forceinline__ uint32_t nth_set(uint32_t m, uint32_t n) {
 // live lanes get their value.  For frames with fewer rays than lanes and for
 // the end of any frame, when what is left is the chain of the longest rays:
 // an evaluation takes a warp alone 1.2 us, with 4 lanes to the point 0.8.
-template <uint32_t L>
-__device__ __forceinline__ float terrain_density_shared(const FieldRows& R, V3 p, uint32_t live,
-                                                        uint32_t octaves, float scale, float amp) {
+// The field may differ between the lanes (FieldWords: and its table with it;
+// FieldRows: one table, every lane its own copy).
+template <uint32_t L, uint32_t STRIDE, uint32_t G>
+__device__ __forceinline__ float terrain_density_shared(const FieldTable<STRIDE, G>& R, V3 p,
+                                                        uint32_t live, uint32_t octaves,
+                                                        float scale, float amp) {
   const uint32_t lane = threadIdx.x & 31u;
   const float x = scale * p.x, y = scale * p.y, z = scale * p.z;
   const float lim = __uint_as_float((127u + 22u - octaves) << 23);
   const bool mine = (live >> lane) & 1u;
   float sum = 0.0f;
   if (__any_sync(0xFFFFFFFFu, mine && !(fabsf(x) < lim && fabsf(y) < lim && fabsf(z) < lim))) {
-    if (mine) sum = field_far<kRowBytes>(R.base, x, y, z, octaves);
+    if (mine) sum = field_far<STRIDE>(R.base, x, y, z, octaves);
     return __fmaf_rn(-amp, sum, p.y);
   }
   const uint32_t src = nth_set(live, lane / L);  // past the last point: lane 31's, unused
   const float sx = __shfl_sync(0xFFFFFFFFu, x, src), sy = __shfl_sync(0xFFFFFFFFu, y, src),
               sz = __shfl_sync(0xFFFFFFFFu, z, src);
+  FieldTable<STRIDE, G> T = R;
+  uint32_t oct = octaves, most = octaves;  // of the point this lane helps with; of any
+  if (STRIDE != kRowBytes) {
+    T.base = __shfl_sync(0xFFFFFFFFu, R.base, src);
+    oct = __shfl_sync(0xFFFFFFFFu, octaves, src);
+    most = __reduce_max_sync(0xFFFFFFFFu, mine ? octaves : 0u);
+  }
   const bool helps = lane / L < (uint32_t)__popc(live);
   const uint32_t from = L * (uint32_t)__popc(live & ((1u << lane) - 1u));  // this point's helpers
   float a = 1.0f;
 #pragma unroll 1
-  for (uint32_t c = 0; c < octaves; c += 2u * L) {
+  for (uint32_t c = 0; c < most; c += 2u * L) {
     const uint32_t k = c + 2u * (lane & (L - 1u));
     float r0 = 0.0f, r1 = 0.0f;
-    if (helps && k < octaves) {
+    if (helps && k < oct) {
       const float f = __uint_as_float((127u + k) << 23);  // 2^k
-      unpack2(perlin2(R, pack2(f * sx, 2.0f * (f * sx)), pack2(f * sy, 2.0f * (f * sy)),
+      unpack2(perlin2(T, pack2(f * sx, 2.0f * (f * sx)), pack2(f * sy, 2.0f * (f * sy)),
                       pack2(f * sz, 2.0f * (f * sz))),
               r0, r1);
     }
@@ -485,13 +495,15 @@ __device__ __forceinline__ float terrain_density_shared(const FieldRows& R, V3 p
 
 // terrain_density() at the points of the live lanes, with more lanes to a
 // point where they are few.  All 32 lanes call it.
-__device__ __forceinline__ float warp_density(const FieldRows& R, V3 p, bool live,
+// SHARED2: two lanes to a point as well as four (a third copy of the code).
+template <int UNROLL = 2, bool SHARED2 = true, uint32_t STRIDE, uint32_t G>
+__device__ __forceinline__ float warp_density(const FieldTable<STRIDE, G>& R, V3 p, bool live,
                                               uint32_t octaves, float scale, float amp) {
   const uint32_t mask = __ballot_sync(0xFFFFFFFFu, live);
   const uint32_t n = __popc(mask);
   if (n <= 8u) return terrain_density_shared<4>(R, p, mask, octaves, scale, amp);
-  if (n <= 16u) return terrain_density_shared<2>(R, p, mask, octaves, scale, amp);
-  return live ? terrain_density<2>(R, p, octaves, scale, amp) : 0.0f;
+  if (SHARED2 && n <= 16u) return terrain_density_shared<2>(R, p, mask, octaves, scale, amp);
+  return live ? terrain_density<UNROLL>(R, p, octaves, scale, amp) : 0.0f;
 }
 
 // Gradient of perlin() at (x, y, z), from the same lattice, fade and blend
