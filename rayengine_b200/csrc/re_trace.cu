@@ -80,7 +80,7 @@ __device__ __forceinline__ void refill_walk(const KdDev& kd, const uint2* snodes
       continue;
     }
     if (s.live) {
-      trav_step<MODE, ANYHIT, COUNT>(s, kd, snodes, c);
+      trav_step<MODE, ANYHIT, COUNT, 1, kRefillDescent>(s, kd, snodes, c);
       if (!s.live) done(cur, s, c);
     }
   }
@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(256, 5) k_ao_secondary(KdDev kd, AoDev ao, AoQ
       continue;
     }
     if (s.live) {
-      trav_step<0, true, COUNT>(s, kd, snodes, c);
+      trav_step<0, true, COUNT, 1, kAoDescent>(s, kd, snodes, c);
       if (!s.live && !COUNT) {
         uint32_t bits = (s.best_id < 0 ? 1u << (tag & 7u) : 0u) |
                         (trav_truncated(s) ? kMaskTruncated : 0u);
