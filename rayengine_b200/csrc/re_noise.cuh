@@ -565,20 +565,122 @@ __device__ __forceinline__ V3 perlin_grad(const PT& P, float x, float y, float z
   return r;
 }
 
-// Gradient of terrain_density: (0, 1, 0) - amp * scale * sum_i gain^i
-// lacunarity^i grad perlin(lacunarity^i scale p), lacunarity 2, gain 0.5
-// (each octave's amplitude x frequency is 1).
-template <class PT>
-__device__ __forceinline__ V3 terrain_gradient(const PT& P, V3 p, uint32_t octaves, float scale,
-                                               float amp) {
-  float x = scale * p.x, y = scale * p.y, z = scale * p.z;
+// The octaves' gradients at any coordinates, summed (out of line, as
+// field_far is).
+template <uint32_t STRIDE>
+static __device__ __noinline__ V3 gradient_far(uint32_t base, float x, float y, float z,
+                                               uint32_t octaves) {
+  PermRows<STRIDE> P{base};
   V3 s = v3(0.f, 0.f, 0.f);
+#pragma unroll 1
   for (uint32_t i = 0; i < octaves; ++i) {
     V3 gi = perlin_grad(P, x, y, z);
     s = v3(s.x + gi.x, s.y + gi.y, s.z + gi.z);
     x *= 2.0f;
     y *= 2.0f;
     z *= 2.0f;
+  }
+  return s;
+}
+
+// a + b and a - b where one of them may be a product: as a product with one,
+// so that the two roundings stay two.  (A packed product feeding a packed
+// addition is contracted, a product with a one known to the compiler too;
+// `one` comes from the caller's arguments.)
+__device__ __forceinline__ f32x2 plus2(f32x2 a, f32x2 b, float one) {
+  return fma2(b, pack2(one, one), a);
+}
+__device__ __forceinline__ f32x2 minus2(f32x2 a, f32x2 b, float one) {
+  return fma2(b, pack2(-one, -one), a);
+}
+
+// Twice perlin_grad() of two octaves; every coordinate below 2^22.  The
+// corners' gradient bytes are +2, -2 and 0, so perlin_grad's selections by
+// gradient case are products here, exact ones, and every value is twice
+// perlin_grad's.
+template <class FT>
+__device__ __forceinline__ void perlin_grad2(const FT& R, f32x2 x, f32x2 y, f32x2 z, float one,
+                                             f32x2& rx, f32x2& ry, f32x2& rz) {
+  const f32x2 kInt = pack2(12582912.0f, 12582912.0f), kOne = pack2(1.0f, 1.0f);
+  const f32x2 k30 = pack2(30.0f, 30.0f);
+  const f32x2 ix = add2_down(x, kInt), iy = add2_down(y, kInt), iz = add2_down(z, kInt);
+  const f32x2 tx = sub2(x, sub2(ix, kInt)), ty = sub2(y, sub2(iy, kInt)),
+              tz = sub2(z, sub2(iz, kInt));
+  uint32_t lo[8], hi[8];
+  cell_words(R, (uint32_t)ix, (uint32_t)iy, (uint32_t)iz, lo);
+  cell_words(R, (uint32_t)(ix >> 32), (uint32_t)(iy >> 32), (uint32_t)(iz >> 32), hi);
+  const f32x2 x1 = sub2(tx, kOne), y1 = sub2(ty, kOne), z1 = sub2(tz, kOne);
+  const f32x2 u = quintic2(tx), v = quintic2(ty), w = quintic2(tz);
+  const f32x2 uv = mul2(u, v), uw = mul2(u, w), vw = mul2(v, w), uvw = mul2(uv, w);
+  const auto plus = [one](f32x2 a, f32x2 b) { return plus2(a, b, one); };
+  const auto minus = [one](f32x2 a, f32x2 b) { return minus2(a, b, one); };
+  // trilinear weights of the corners (order a..h: x fastest, then y, z)
+  const f32x2 cw[8] = {
+      minus(plus(plus(plus(minus(minus(minus(kOne, u), v), w), uv), uw), vw), uvw),
+      plus(minus(minus(u, uv), uw), uvw),
+      plus(minus(minus(v, uv), vw), uvw),
+      minus(uv, uvw),
+      plus(minus(minus(w, uw), vw), uvw),
+      minus(uw, uvw),
+      minus(vw, uvw),
+      uvw};
+  f32x2 c[8], sx = 0ull, sy = 0ull, sz = 0ull;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const f32x2 gx =
+        pack2(__uint_as_float(lo[k] & 0xFF000000u), __uint_as_float(hi[k] & 0xFF000000u));
+    const f32x2 gy = pack2(__uint_as_float(__byte_perm(lo[k], 0u, 0x2444)),
+                           __uint_as_float(__byte_perm(hi[k], 0u, 0x2444)));
+    const f32x2 gz = pack2(__uint_as_float(lo[k] << 24), __uint_as_float(hi[k] << 24));
+    c[k] = fma2(gz, k & 4 ? z1 : tz, fma2(gy, k & 2 ? y1 : ty, mul2(gx, k & 1 ? x1 : tx)));
+    sx = fma2(cw[k], gx, sx);
+    sy = fma2(cw[k], gy, sy);
+    sz = fma2(cw[k], gz, sz);
+  }
+  const f32x2 k1 = sub2(c[1], c[0]), k2 = sub2(c[2], c[0]), k3 = sub2(c[4], c[0]);
+  const f32x2 k4 = sub2(sub2(add2(c[0], c[3]), c[1]), c[2]);
+  const f32x2 k5 = sub2(sub2(add2(c[0], c[5]), c[1]), c[4]);
+  const f32x2 k6 = sub2(sub2(add2(c[0], c[6]), c[2]), c[4]);
+  const f32x2 k7 =
+      sub2(sub2(sub2(sub2(add2(add2(add2(c[1], c[2]), c[4]), c[7]), c[0]), c[3]), c[5]), c[6]);
+  const f32x2 du = mul2(mul2(k30, mul2(tx, tx)), mul2(x1, x1));
+  const f32x2 dv = mul2(mul2(k30, mul2(ty, ty)), mul2(y1, y1));
+  const f32x2 dw = mul2(mul2(k30, mul2(tz, tz)), mul2(z1, z1));
+  rx = plus(sx, mul2(du, plus(plus(plus(k1, mul2(k4, v)), mul2(k5, w)), mul2(k7, vw))));
+  ry = plus(sy, mul2(dv, plus(plus(plus(k2, mul2(k4, u)), mul2(k6, w)), mul2(k7, uw))));
+  rz = plus(sz, mul2(dw, plus(plus(plus(k3, mul2(k5, u)), mul2(k6, v)), mul2(k7, uv))));
+}
+
+// Gradient of terrain_density: (0, 1, 0) - amp * scale * sum_i gain^i
+// lacunarity^i grad perlin(lacunarity^i scale p), lacunarity 2, gain 0.5
+// (each octave's amplitude x frequency is 1).  Octaves in pairs, as
+// terrain_density() evaluates them.  one: 1.0f (plus2).
+template <uint32_t STRIDE, uint32_t G>
+__device__ __forceinline__ V3 terrain_gradient(const FieldTable<STRIDE, G>& R, V3 p,
+                                               uint32_t octaves, float scale, float amp,
+                                               float one) {
+  const float x = scale * p.x, y = scale * p.y, z = scale * p.z;
+  const float lim = __uint_as_float((127u + 22u - octaves) << 23);
+  V3 s = v3(0.f, 0.f, 0.f);
+  if (fabsf(x) < lim && fabsf(y) < lim && fabsf(z) < lim) {
+    const f32x2 kFour = pack2(4.0f, 4.0f);
+    f32x2 X = pack2(x, 2.0f * x), Y = pack2(y, 2.0f * y), Z = pack2(z, 2.0f * z);
+#pragma unroll 1
+    for (uint32_t i = 0; i < octaves; i += 2) {
+      f32x2 gx, gy, gz;
+      perlin_grad2(R, X, Y, Z, one, gx, gy, gz);
+      float x0, x1, y0, y1, z0, z1;
+      unpack2(gx, x0, x1);
+      unpack2(gy, y0, y1);
+      unpack2(gz, z0, z1);
+      s = v3(s.x + 0.5f * x0, s.y + 0.5f * y0, s.z + 0.5f * z0);
+      if (i + 1u < octaves) s = v3(s.x + 0.5f * x1, s.y + 0.5f * y1, s.z + 0.5f * z1);
+      X = mul2(X, kFour);
+      Y = mul2(Y, kFour);
+      Z = mul2(Z, kFour);
+    }
+  } else {
+    s = gradient_far<STRIDE>(R.base, x, y, z, octaves);
   }
   const float k = -amp * scale;
   return v3(k * s.x, __fmaf_rn(k, s.y, 1.0f), k * s.z);

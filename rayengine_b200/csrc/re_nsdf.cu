@@ -1742,18 +1742,21 @@ __global__ void __launch_bounds__(kRowsThreads) k_sdf_refine(
 // which at radius 0.002 t are coarse estimates of this gradient).  A
 // separate pass, so that the exact phase's state machine keeps a single
 // field call site and the gradient's lanes do not diverge from the march.
-__global__ void __launch_bounds__(256) k_sdf_grad_normal(PermTable perm, FieldDev f, uint32_t n,
-                                                         float4* __restrict__ out,
-                                                         unsigned long long* __restrict__ totals) {
-  extern __shared__ uint32_t perm_smem[];
-  load_perm(perm, perm_smem);
-  Perm P = perm_view(perm_smem);
+// Bound by instructions: octaves in pairs on the rows' table take 116 us of a
+// 1080p frame, one octave at a time on 16 copies of the permutation took 169.
+__global__ void __launch_bounds__(kRowsThreads, 1)
+k_sdf_grad_normal(PermTable perm, FieldDev f, uint32_t n, float one, float4* __restrict__ out,
+                  unsigned long long* __restrict__ totals) {
+  extern __shared__ uint32_t rows_smem[];
+  const FieldRows R = load_rows(perm, rows_smem);
   uint32_t count = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  // the warps of all blocks in turn, so that a small frame spreads over the SMs
+  const uint32_t first = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32u + (threadIdx.x & 31u);
+  for (uint32_t i = first; i < n; i += gridDim.x * blockDim.x) {
     float4 r1 = out[2 * (size_t)i + 1];
     if (__float_as_uint(r1.w) != 1u) continue;
     float4 r0 = out[2 * (size_t)i];
-    V3 nn = normalize(terrain_gradient(P, v3(r0.x, r0.y, r0.z), f.octaves, f.scale, f.amp));
+    V3 nn = normalize(terrain_gradient(R, v3(r0.x, r0.y, r0.z), f.octaves, f.scale, f.amp, one));
     r0.w = nn.x;
     r1.x = nn.y;
     r1.y = nn.z;
@@ -2453,15 +2456,12 @@ RE_API re_status re_nsdf_trace_exact(re_nsdf* s, const re_sdf_params* field,
       exact_only || cone ? 1 : 0, s->queue, s->counters, totals, reinterpret_cast<float4*>(d_out));
   RE_CHECK_LAUNCH("re_nsdf_trace_exact: refine launch");
   if (rd.normal_taps == 1u) {
-    auto kg = re::nsdf::k_sdf_grad_normal;
-    int gper_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&gper_sm, kg, 256, re::kPermSmemBytes) !=
-            cudaSuccess ||
-        gper_sm < 1)
-      gper_sm = 1;
-    kg<<<gper_sm * re::sm_count(), 256, re::kPermSmemBytes, cs>>>(
-        re::perm_of(field->seed), re::field_of(*field), w * h, reinterpret_cast<float4*>(d_out),
-        totals);
+    RE_CUDA(cudaFuncSetAttribute(re::nsdf::k_sdf_grad_normal,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)re::kRowsSmemBytes));
+    re::nsdf::k_sdf_grad_normal<<<re::sm_count(), re::kRowsThreads, re::kRowsSmemBytes, cs>>>(
+        re::perm_of(field->seed), re::field_of(*field), w * h, 1.0f,
+        reinterpret_cast<float4*>(d_out), totals);
     RE_CHECK_LAUNCH("re_nsdf_trace_exact: normal launch");
   }
   return RE_OK;

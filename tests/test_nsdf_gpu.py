@@ -280,3 +280,29 @@ def test_training_steps_follow_one_another(cuda):
             out.append((losses, m.get_params()))
     assert np.array_equal(out[0][0], out[1][0])
     assert np.array_equal(out[0][1], out[1][1])
+
+
+# octave counts around the pairs, a frame of fewer rays than a warp, and a
+# camera past the paired form's range (|0.25 x| times 2^8 above 2^22)
+@pytest.mark.parametrize("octaves,w,h,x", [(1, 64, 36, 0.0), (2, 33, 7, 0.0), (7, 64, 36, -3.0),
+                                           (8, 5, 4, 0.0), (9, 161, 45, 0.0),
+                                           (8, 64, 36, 65537.0), (8, 64, 36, -70000.0)])
+def test_gradient_of_octave_pairs(cuda, octaves, w, h, x):
+    """The normals of normal_taps 1 against the FP64 gradient at the returned
+    positions (scale 0.25 is a power of two, so FP32 coordinates are exact).
+    A component of an octave's gradient is a sum of about 20 roundings of
+    values up to 4, 5e-6; amplitude x scale = 0.75 of octaves of these, over
+    the gradient's length; 1e-5 more for the central differences and the
+    normalisation."""
+    tc = rb.configs.TerrainConfig(width=w, height=h, octaves=octaves,
+                                  campos=(x, 6.0, -20.0), lookat=(x, 0.0, 0.0))
+    with _model() as m:
+        out = m.trace(tc.params(), rb.nsdf_trace_params(exact_only=True, normal_taps=1),
+                      tc.camera(), w, h).cpu().numpy().reshape(-1, 8)
+    hit = out[out[:, 7] == 1].view(np.float32)
+    assert len(hit) > 0
+    P, p = po.perm(tc.seed), hit[:, 0:3].astype(np.float64)
+    g = np.stack([(po.density_d(P, p + e, octaves) - po.density_d(P, p - e, octaves)) / 2e-5
+                  for e in 1e-5 * np.eye(3)], axis=1)
+    length = np.linalg.norm(g, axis=1, keepdims=True)
+    assert np.all(np.abs(hit[:, 3:6] - g / length) <= 0.75 * octaves * 5e-6 / length + 1e-5)
