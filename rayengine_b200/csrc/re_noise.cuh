@@ -19,12 +19,12 @@ struct PermTable {
   uint8_t p[512];
 };
 
-// The table lives in shared memory in 16 interleaved copies: entry j of
-// lane c is the word 16*j + (c & 15), so of a warp's 32 divergent lookups
+// One octave at a time (the caller-point fBm and the heightfield; the terrain
+// field reads FieldTable below): the table in 16 interleaved copies, entry j
+// of lane c at word 16*j + (c & 15), so that of a warp's 32 divergent lookups
 // only lanes c and c + 16 can meet in a bank (when their entries have the
-// same parity).  512 entries x 16 copies x 4 B = 32 KB; measured on B200 2 %
-// faster on the SDF march than 32 conflict-free copies (64 KB), which allow
-// one block per SM fewer.  Each
+// same parity).  512 entries x 16 copies x 4 B = 32 KB, four blocks to an SM;
+// 32 conflict-free copies (64 KB) allow one block fewer.  Each
 // word holds P[j] in bits 0-7 and the gradient case h = P[j] & 15 decoded
 // for grad_dot in bits 28-31: bit 28 set when its first operand is y (else
 // x), bit 29 when its second operand is y (else z), bit 30 when the second
@@ -194,16 +194,19 @@ __device__ __forceinline__ float terrain_density(const PT& P, V3 p,
 // Measured on B200 (a march of 8-octave evaluations, no other work): 33.3 G
 // evaluations/s against 26.3 of perlin() on 16 copies.  Per octave 99
 // instructions against 147; the multiply-add pipes, 73 % busy, are what is
-// left (the scalar form of this layout: 29.9 G/s).  Frames, before and after:
-// the 1080p terrain 3.18 -> 2.56 ms, the shaded terrain at 1366x768 2.65 ->
-// 2.10 ms, the 1080p neural tracer 2.27 -> 1.85 ms.
+// left (the scalar form of this layout: 29.9 G/s).  Frames, one octave at a
+// time on 16 copies against this form alone: the 1080p terrain 3.18 -> 2.56
+// ms, the shaded terrain at 1366x768 2.65 -> 2.10 ms (1.95 with several lanes
+// to a ray, terrain_density_shared), the 1080p neural tracer 2.27 -> 1.85 ms
+// (1.77 with the normals' gradient in this form too, perlin_grad2).
 // FieldTable<STRIDE, G>: rows STRIDE bytes apart, G words G bytes past A words.
 constexpr uint32_t kRowBytes = 256;
 constexpr uint32_t kRowsSmemBytes = 512 * kRowBytes;
 // One block per SM, whose warps share the table.  640 threads: 5 warps per
 // sub-partition with 96 registers to keep both cells' lookups in flight
-// (1080p terrain frame 2.62 ms; 512 threads 2.75, 768 2.69, 1024 2.74), and
-// with four pairs unrolled 2.56.
+// (1080p terrain frame 2.62 ms; 512 threads 2.75, 768 2.69, 1024 2.74).  One,
+// two and four pairs of octaves unrolled: 2.62, 2.58, 2.56; kernels that hold
+// the forms with several lanes to a ray as well unroll two (warp_density).
 constexpr uint32_t kRowsThreads = 640;
 
 // How a frame of n rays spreads over `blocks` blocks of kRowsThreads: the rays
