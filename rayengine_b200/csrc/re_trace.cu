@@ -90,7 +90,7 @@ __device__ __forceinline__ void refill_walk(const KdDev& kd, const uint2* snodes
 // blocks of 256 threads per SM (40 registers, a few dozen bytes of spills):
 // the 2^20-triangle soup's primary pass is 3 % faster than at 5 blocks (48
 // registers) and 9 % faster than at 4; the AO frame's kernels keep 5 blocks
-// (at 6 its secondary pass is 2.6 % slower).
+// (at 6 the frame is 9 % slower).
 //
 // Primary rays, persistent warps over 8x4 pixel tiles, each lane running its
 // ray to the end (ray_refill_min 32: no per-leaf bookkeeping; fastest when
