@@ -691,6 +691,10 @@ RE_API re_status re_batch_render_graph(re_batch* b, float* d_radiance,
  * primary rays under kind 0), 2 * max_depth values; error = 1 if a wait
  * bound was reached (rays dropped). */
 RE_API re_status re_batch_stats_get(re_batch* b, uint64_t* rays, int* error);
+/* For checking: pixels asked for in the last frame, of mesh scenes and of
+ * terrains.  Each is at least the kind's pixels and exceeds them by at most
+ * one claim of 32 per warp of the launch. */
+RE_API re_status re_batch_claims_get(re_batch* b, uint32_t* claims);
 /* Bounds of the persistent kernel's waits: polls of one queue slot's flag
  * before a claim is dropped, and trips of the kernel's loop (0 = the
  * defaults, 2^22 each).  Reaching either sets the frame's error flag

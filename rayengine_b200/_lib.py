@@ -302,6 +302,7 @@ _SIGS = {
     "re_batch_stats_get": (ctypes.c_int, [_P, _P, ctypes.POINTER(ctypes.c_int)]),
     "re_batch_set_wait_bounds": (ctypes.c_int, [_P, _U32, _U32]),
     "re_batch_counts": (ctypes.c_int, [_P, _P, _P, _P]),
+    "re_batch_claims_get": (ctypes.c_int, [_P, _P]),
     "re_batch_get_tuning": (ctypes.c_int, [_P, ctypes.POINTER(re_batch_tuning)]),
     "re_batch_set_tuning": (ctypes.c_int, [_P, ctypes.POINTER(re_batch_tuning)]),
     "re_batch_autotune": (ctypes.c_int, [_P, _P, _P, ctypes.POINTER(re_batch_tuning), ctypes.POINTER(_F)]),

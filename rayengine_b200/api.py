@@ -697,6 +697,13 @@ class Batch:
         call("re_batch_stats_get", self._h, rays.ctypes.data, ctypes.byref(err))
         return {"rays": rays.reshape(self.max_depth, 2).astype(np.int64), "error": int(err.value)}
 
+    def claims(self) -> np.ndarray:
+        """Pixels asked for in the last frame, of mesh scenes and of terrains
+        (re_batch_claims_get)."""
+        v = np.zeros(2, np.uint32)
+        call("re_batch_claims_get", self._h, v.ctypes.data)
+        return v.astype(np.int64)
+
     def set_wait_bounds(self, pending_polls: int = 0, loop_trips: int = 0) -> None:
         """Lower the kernel's wait bounds (0 = defaults); for error-path tests."""
         call("re_batch_set_wait_bounds", self._h, pending_polls, loop_trips)

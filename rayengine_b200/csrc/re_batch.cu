@@ -76,9 +76,10 @@ enum : uint32_t {
   kStats = kClaimed + kMaxQueues * kLine,  // + q
   kStatsPrimary = kStats + kMaxQueues,
   kStatsError = kStatsPrimary + 1,
+  kStatsCursor = kStatsError + 1,  // + kind
   kNumCounters = kStats + kLine
 };
-static_assert(kStatsError < kNumCounters, "counter layout");
+static_assert(kStatsCursor + 1 < kNumCounters, "counter layout");
 __host__ __device__ constexpr uint32_t cursor_at(uint32_t kind) { return kCursor + kind * kLine; }
 __host__ __device__ constexpr uint32_t fin_at(uint32_t b, uint32_t kind) {
   return kFin + (2u * b + kind) * kLine;
@@ -250,7 +251,8 @@ __host__ __device__ constexpr uint32_t table_bytes(int table) {
   return table == kFieldTables ? kFieldWordsBytes : table == kWordTables ? 2048u : 512u;
 }
 // One kind's rays on one warp: claims and steps them until the warp holds none
-// and finds none to claim.  Returns whether it held any.
+// and finds none to claim.  Returns whether it held any.  primary_done (lane 0):
+// whether the kind's pixel cursor has passed its end.
 //
 // The kinds never exchange rays, so a warp works on one at a time and the
 // mesh walk and the terrain march do not share a loop: in one loop for both
@@ -263,7 +265,7 @@ template <bool COUNT, int TABLE, uint32_t KIND>
 __device__ __forceinline__ bool run_kind(const BatchDev& B, const SceneDev* sc,
                                          const uint8_t* sperm, const uint2* snodes, uint32_t* wfin,
                                          uint32_t epoch, uint32_t& trip, Counters& cnt,
-                                         uint32_t& errors) {
+                                         uint32_t& errors, bool& primary_done) {
   const uint32_t* sperm_w = reinterpret_cast<const uint32_t*>(sperm);
   uint32_t* ctr = B.ctr;
   const uint32_t lane = threadIdx.x & 31u;
@@ -282,7 +284,6 @@ __device__ __forceinline__ bool run_kind(const BatchDev& B, const SceneDev* sc,
   uint32_t &steps = tr.visits, &tap = tr.best_ref;
   uint32_t &pq = tr.best_ref, &pslot = tr.best_leaf, &polls = tr.visits;
   uint32_t fin_pending = 0;   // lane 0: finished rays in wfin
-  bool primary_done = false;  // lane 0: the pixel cursor has passed the end
   bool any = false;
 
   // publishes this warp's finished counts (after its reservations, which
@@ -561,11 +562,13 @@ __device__ __forceinline__ bool run_kind(const BatchDev& B, const SceneDev* sc,
         if (lane == leader) b0 = atomicAdd(&ctr[reserved_at(qn)], (uint32_t)__popc(peers));
         b0 = __shfl_sync(peers, b0, leader);
         slot = b0 + __popc(peers & lt_mask);
-        float4* rec = B.queue + 2 * (B.qoff[qn] + slot);
-        __stcg(rec, R0);
-        __stcg(rec + 1, R1);
-        // the release store orders this lane's record before its flag
-        st_release(&B.flags[B.qoff[qn] + slot], epoch);
+        if (slot < B.qcap[qn]) {
+          float4* rec = B.queue + 2 * (B.qoff[qn] + slot);
+          __stcg(rec, R0);
+          __stcg(rec + 1, R1);
+          // the release store orders this lane's record before its flag
+          st_release(&B.flags[B.qoff[qn] + slot], epoch);
+        }  // else never written: the last block reports it
       }
     }
     // finished rays are counted per warp and bounce in shared memory and
@@ -630,6 +633,12 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
   uint32_t* wfin = sfin + (threadIdx.x >> 5) * kMaxDepth;  // this warp's unpublished counts
   Counters cnt = {0, 0, 0, 0};
   uint32_t errors = 0, trip = 0;
+  // primary_done of the two kinds.  They outlive a call of run_kind: a warp
+  // without work comes back to both kinds until the frame is over, and may
+  // advance each cursor past its end once (one that waiting warps went on
+  // advancing would wrap its 32 bits within half a second and hand pixels out
+  // again).
+  bool mesh_done = false, terrain_done = false;
   // Neighbouring warps start on different kinds, so that an SM's walks
   // (bound by latency) and marches (by the FP32 pipes) run side by side; a
   // warp that finds nothing to do changes over, and leaves once both are done.
@@ -638,9 +647,11 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
   for (; trip < B.loop_bound; ++trip) {
     bool any;
     if (TABLE == kNoTables || kind == kMesh)
-      any = run_kind<COUNT, TABLE, kMesh>(B, sc, sperm, snodes, wfin, epoch, trip, cnt, errors);
+      any = run_kind<COUNT, TABLE, kMesh>(B, sc, sperm, snodes, wfin, epoch, trip, cnt, errors,
+                                          mesh_done);
     else
-      any = run_kind<COUNT, TABLE, kTerrain>(B, sc, sperm, snodes, wfin, epoch, trip, cnt, errors);
+      any = run_kind<COUNT, TABLE, kTerrain>(B, sc, sperm, snodes, wfin, epoch, trip, cnt, errors,
+                                             terrain_done);
     if (trip >= B.loop_bound) break;
     dry = any ? 0u : dry + 1u;
     if (any) backoff = 32;
@@ -674,6 +685,7 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
       __threadfence();
       for (uint32_t q = 0; q < nq; ++q) {
         ctr[kStats + q] = ctr[reserved_at(q)];
+        if (ctr[reserved_at(q)] > B.qcap[q]) ctr[kError] = 1u;  // dropped continuations
         ctr[reserved_at(q)] = 0u;
         ctr[claimed_at(q)] = 0u;
       }
@@ -681,6 +693,8 @@ __global__ void __launch_bounds__(RE_BATCH_MAX_THREADS, RE_BATCH_MIN_BLOCKS) k_b
       ctr[kStatsPrimary] = min(ctr[cursor_at(0)], B.kind_pixels[0]) +
                            min(ctr[cursor_at(1)], B.kind_pixels[1]);
       ctr[kStatsError] = ctr[kError];
+      ctr[kStatsCursor] = ctr[cursor_at(0)];
+      ctr[kStatsCursor + 1u] = ctr[cursor_at(1)];
       ctr[cursor_at(0)] = ctr[cursor_at(1)] = 0u;
       ctr[kError] = 0u;
       ctr[kDone] = 0u;
@@ -1085,6 +1099,14 @@ RE_API re_status re_batch_stats_get(re_batch* b, uint64_t* rays, int* error) {
   rays[0] = c[kStatsPrimary];
   for (uint32_t q = 0; q < 2 * (b->depth - 1); ++q) rays[2 + q] = c[kStats + q];
   if (error) *error = (int)c[kStatsError];
+  return RE_OK;
+}
+
+RE_API re_status re_batch_claims_get(re_batch* b, uint32_t* claims) {
+  using namespace re::batch;
+  if (!b || !claims) return re::fail(RE_ERR_INVALID_ARG, "re_batch_claims_get: bad arguments");
+  RE_CUDA(cudaMemcpy(claims, b->d_ctr + kStatsCursor, 2 * sizeof(uint32_t),
+                     cudaMemcpyDeviceToHost));
   return RE_OK;
 }
 
