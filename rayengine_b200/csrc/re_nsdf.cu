@@ -1833,11 +1833,18 @@ namespace {
 
 using namespace nsdf;
 
-void free_train(re_nsdf* s) {
+// Forgets the captured training step.  It holds the model's input map, the
+// training points' address and number, the loss history's address, the batch
+// and the learning rate: whatever changes one of them calls this.
+void drop_graph(re_nsdf* s) {
   if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
   if (s->graph) cudaGraphDestroy(s->graph);
   s->graph_exec = nullptr;
   s->graph = nullptr;
+}
+
+void free_train(re_nsdf* s) {
+  drop_graph(s);
   cudaFree(s->part);
   s->part = nullptr;
   s->batch = 0;
@@ -2097,6 +2104,7 @@ RE_API re_status re_nsdf_generate(re_nsdf* s, const re_sdf_params* field, const 
   cudaStream_t cs = (cudaStream_t)stream;
   if (s->npts != num_points) {
     RE_CUDA(cudaStreamSynchronize(cs));
+    re::drop_graph(s);
     cudaFree(s->data);
     s->data = nullptr;
     s->npts = 0;
@@ -2152,16 +2160,10 @@ RE_API re_status re_nsdf_train(re_nsdf* s, uint32_t steps, uint32_t batch, float
     }
     s->loss_hist = nh;
     s->loss_cap = cap;
-    if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
-    if (s->graph) cudaGraphDestroy(s->graph);
-    s->graph_exec = nullptr;
-    s->graph = nullptr;
+    re::drop_graph(s);
   }
   if (!s->graph_exec || s->graph_lr != lr) {
-    if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
-    if (s->graph) cudaGraphDestroy(s->graph);
-    s->graph_exec = nullptr;
-    s->graph = nullptr;
+    re::drop_graph(s);
     cudaStream_t cap_stream;
     RE_CUDA(cudaStreamCreateWithFlags(&cap_stream, cudaStreamNonBlocking));
     cudaError_t e = cudaStreamBeginCapture(cap_stream, cudaStreamCaptureModeThreadLocal);
@@ -2529,6 +2531,7 @@ RE_API re_status re_nsdf_load(re_nsdf* s, const char* path) {
   RE_CUDA(cudaMemcpy(s->adam_m, buf.data() + kNumParams, kNumParams * 4, cudaMemcpyHostToDevice));
   RE_CUDA(cudaMemcpy(s->adam_v, buf.data() + 2 * kNumParams, kNumParams * 4, cudaMemcpyHostToDevice));
   RE_CUDA(cudaMemcpy(s->step_ctr, &hdr[3], 4, cudaMemcpyHostToDevice));
+  re::drop_graph(s);
   s->map = m;
   s->total_steps_done = hdr[3];
   s->pack_valid = false;

@@ -1,0 +1,52 @@
+"""Calls on a NeuralSDF after its state has changed under it: a captured
+training step must not outlive the points and the input map it was made for."""
+import numpy as np
+import pytest
+
+import rayengine_b200 as rb
+
+pytestmark = pytest.mark.gpu
+
+BOX = ([-40.0, -6.0, -20.0], [40.0, 11.0, 60.0])
+OTHER = ([-20.0, -5.0, -10.0], [30.0, 9.0, 50.0])
+
+
+def _generate(net, points):
+    t = rb.configs.TerrainConfig(width=64, height=36)
+    net.generate(t.params(), t.camera(), t.width, t.height, points, seed=4)
+
+
+def _captured(points, steps=(8, 2)):
+    """A model whose captured step has room left in its loss history (the
+    first call allocates 8 entries, the second grows them to 16)."""
+    net = rb.NeuralSDF(*BOX, 0.5, 3)
+    _generate(net, points)
+    for n in steps:
+        net.train(n, batch=512)
+    return net
+
+
+@pytest.mark.parametrize("points", [700, 40000])
+def test_train_after_generate(cuda, tmp_path, points):
+    with _captured(5000) as net, rb.NeuralSDF(*BOX, 0.5, 3) as fresh:
+        ck = str(tmp_path / "state.rnsdf")
+        net.save(ck)
+        fresh.load(ck)
+        for m in (net, fresh):
+            _generate(m, points)
+        assert np.array_equal(net.train(4, batch=512), fresh.train(4, batch=512))
+        assert np.array_equal(net.get_params(), fresh.get_params())
+
+
+def test_train_after_load(cuda, tmp_path):
+    ck = str(tmp_path / "other.rnsdf")
+    with rb.NeuralSDF(*OTHER, 0.7, 3) as other:
+        _generate(other, 5000)
+        other.train(10, batch=512)
+        other.save(ck)
+    with _captured(5000) as net, rb.NeuralSDF(*BOX, 0.5, 3) as fresh:
+        _generate(fresh, 5000)
+        for m in (net, fresh):
+            m.load(ck)
+        assert np.array_equal(net.train(4, batch=512), fresh.train(4, batch=512))
+        assert np.array_equal(net.get_params(), fresh.get_params())
