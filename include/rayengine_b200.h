@@ -473,6 +473,10 @@ RE_API re_status re_nsdf_eval(re_nsdf* s, const float* d_pts, uint32_t n,
 /* The same with the training arithmetic (SIMT FP32, BF16-rounded). */
 RE_API re_status re_nsdf_eval_reference(re_nsdf* s, const float* d_pts,
                                         uint32_t n, float* d_out, void* stream);
+/* For checking: whether the end of the evaluation and training kernels
+ * reports a wait that ran out in the given one of a block's 1024 threads
+ * (1024 and above: in none). */
+RE_API re_status re_nsdf_check_report(re_nsdf* s, uint32_t thread, int* reported);
 /* Gradient-norm bound: the `quantile` (0 < q <= 1; 1 = the largest) of
  * the forward-difference gradient norms at `samples` training points. */
 RE_API re_status re_nsdf_lipschitz(re_nsdf* s, uint32_t samples, float h,

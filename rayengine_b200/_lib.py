@@ -272,6 +272,7 @@ _SIGS = {
     "re_nsdf_train": (ctypes.c_int, [_P, _U32, _U32, _F, _P, _P]),
     "re_nsdf_loss_grad": (ctypes.c_int, [_P, _P, _U32, _P, _P, _P]),
     "re_nsdf_eval": (ctypes.c_int, [_P, _P, _U32, _P, _P]),
+    "re_nsdf_check_report": (ctypes.c_int, [_P, _U32, ctypes.POINTER(ctypes.c_int)]),
     "re_nsdf_eval_reference": (ctypes.c_int, [_P, _P, _U32, _P, _P]),
     "re_nsdf_lipschitz": (ctypes.c_int, [_P, _U32, _F, _F, ctypes.POINTER(_F), _P]),
     "re_nsdf_trace": (ctypes.c_int, [_P, ctypes.POINTER(re_sdf_params), ctypes.POINTER(re_nsdf_trace_params), ctypes.POINTER(re_camera), _U32, _U32, _P, _P]),

@@ -290,6 +290,14 @@ __device__ __forceinline__ void report(int* word) {
   __threadfence_system();
 }
 
+// The end of a kernel whose threads each kept whether their own waits came
+// through: all of them call it, and one that ran out, whichever thread's it
+// was, is reported.
+__device__ __forceinline__ void report_block(bool ok, int* word) {
+  ok = __syncthreads_and(ok);
+  if (!ok && threadIdx.x == 0) report(word);
+}
+
 __device__ __forceinline__ void fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -936,10 +944,9 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_tc_train(
       s.red[row >> 5][kHidden + 1] = loss;
     }
   }
-  ok = __syncthreads_and(ok);
+  report_block(ok, err);
   if (tid < kHidden + 2)
     pp[OFF_W5 + tid] = (s.red[0][tid] + s.red[1][tid]) + (s.red[2][tid] + s.red[3][tid]);
-  if (!ok && tid == 0) report(err);
   fence_before();
   __syncthreads();
   fence_after();
@@ -1105,13 +1112,17 @@ __global__ void __launch_bounds__(kEvalThreads, 1) k_tc_eval(InputMap m,
     }
     if (live) out[i] = d + s.b5;
   }
-  if (!ok && row == 0) report(err);
   fence_before();
-  __syncthreads();
+  report_block(ok, err);
   fence_after();
   if (tid < 32)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem),
                  "r"(kEvalCols));
+}
+
+// report_block() with one thread whose wait ran out, for checking it.
+__global__ void __launch_bounds__(kEvalThreads) k_check_report(uint32_t thread, int* err) {
+  report_block(threadIdx.x != thread, err);
 }
 
 // ------------------------------------------------------------- tracing
@@ -2231,6 +2242,18 @@ RE_API re_status re_nsdf_eval(re_nsdf* s, const float* d_pts, uint32_t n, float*
   RE_CHECK_LAUNCH("re_nsdf_eval: launch");
   RE_CUDA(cudaStreamSynchronize(cs));
   if (*s->sync_err) return re::fail(RE_ERR_INTERNAL, "re_nsdf_eval: tensor-core wait bound reached");
+  return RE_OK;
+}
+
+RE_API re_status re_nsdf_check_report(re_nsdf* s, uint32_t thread, int* reported) {
+  re_status st = re::check(s, "re_nsdf_check_report");
+  if (st != RE_OK) return st;
+  if (!reported) return re::fail(RE_ERR_INVALID_ARG, "re_nsdf_check_report: null output");
+  *s->sync_err = 0;
+  re::nsdf::k_check_report<<<1, re::nsdf::kEvalThreads>>>(thread, s->sync_err_dev);
+  RE_CHECK_LAUNCH("re_nsdf_check_report: launch");
+  RE_CUDA(cudaStreamSynchronize(nullptr));
+  *reported = *s->sync_err;
   return RE_OK;
 }
 

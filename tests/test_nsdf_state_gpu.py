@@ -1,5 +1,8 @@
 """Calls on a NeuralSDF after its state has changed under it: a captured
-training step must not outlive the points and the input map it was made for."""
+training step must not outlive the points and the input map it was made for,
+and a wait that ran out must not go unreported."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -50,3 +53,13 @@ def test_train_after_load(cuda, tmp_path):
             m.load(ck)
         assert np.array_equal(net.train(4, batch=512), fresh.train(4, batch=512))
         assert np.array_equal(net.get_params(), fresh.get_params())
+
+
+@pytest.mark.parametrize("thread", [0, 1, 127, 128, 600, 1023, 1024])
+def test_any_threads_failed_wait_is_reported(cuda, thread):
+    """The evaluation kernel's 1024 threads wait each for itself: one whose
+    wait ran out (1024: none) is reported, whichever row it holds."""
+    with rb.NeuralSDF(*BOX, 0.5, 3) as net:
+        got = ctypes.c_int(-1)
+        rb.api.call("re_nsdf_check_report", net._h, thread, ctypes.byref(got))
+        assert got.value == (1 if thread < 1024 else 0)
