@@ -2209,6 +2209,13 @@ RE_API re_status re_nsdf_loss_grad(re_nsdf* s, const float* d_xyzl, uint32_t n, 
   if (!d_xyzl || !d_grad || n == 0 || n % re::nsdf::kRowsBwd != 0)
     return re::fail(RE_ERR_INVALID_ARG, "re_nsdf_loss_grad: n must be a positive multiple of %d",
                     re::nsdf::kRowsBwd);
+  // a kernel writes the gradient: an address the device cannot reach is
+  // refused here, as a copy to it would be
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, d_grad) != cudaSuccess || !at.devicePointer) {
+    cudaGetLastError();
+    return re::fail(RE_ERR_INVALID_ARG, "re_nsdf_loss_grad: d_grad is not device memory");
+  }
   cudaStream_t cs = (cudaStream_t)stream;
   st = re::alloc_train(s, n);
   if (st != RE_OK) return st;

@@ -5,6 +5,7 @@ import ctypes
 
 import numpy as np
 import pytest
+import torch
 
 import rayengine_b200 as rb
 
@@ -63,3 +64,19 @@ def test_any_threads_failed_wait_is_reported(cuda, thread):
         got = ctypes.c_int(-1)
         rb.api.call("re_nsdf_check_report", net._h, thread, ctypes.byref(got))
         assert got.value == (1 if thread < 1024 else 0)
+
+
+def test_loss_gradient_refuses_host_memory(cuda):
+    with rb.NeuralSDF(*BOX, 0.5, 3) as net:
+        _generate(net, 512)
+        xyzl = torch.from_numpy(net.data(512)).cuda()
+        want, _ = net.loss_grad(xyzl)
+        host = np.zeros(net.num_params, np.float32)
+        with pytest.raises(rb.RayEngineError) as e:
+            rb.api.call("re_nsdf_loss_grad", net._h, xyzl.data_ptr(), 512, host.ctypes.data, None,
+                        None)
+        assert e.value.status == 1 and not host.any()
+        pinned = torch.zeros(net.num_params).pin_memory()  # the device reaches it
+        rb.api.call("re_nsdf_loss_grad", net._h, xyzl.data_ptr(), 512, pinned.data_ptr(), None,
+                    None)
+        assert torch.equal(pinned, want.cpu())
