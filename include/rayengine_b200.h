@@ -7,6 +7,12 @@
  * re_status; nothing calls exit().  The last error message of the calling
  * thread is available from re_last_error().
  *
+ * Streams and threads: calls that take no re_scene, re_nsdf or re_batch may
+ * run on any streams and threads at once.  Such an object owns the scratch of
+ * its calls, so calls on one object that could run side by side must be
+ * serialised by the caller; different objects are independent
+ * (re_render_ao_noalloc excepted, see there).
+ *
  * Reference interface each entry replaces (hadalhw17/RayEngine, paths
  * relative to its repository root, "RE/" = RayEngine/src/):
  *

@@ -4,7 +4,11 @@
 
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <new>
 #include <random>
+#include <utility>
+#include <vector>
 
 namespace re {
 
@@ -93,6 +97,149 @@ int sm_count() {
       return 148;
   }
   return cached;
+}
+
+namespace {
+
+// One slab of slots at a time; slots of streams that may be gone are taken
+// back, after the device is idle, when this many streams have come by.
+constexpr size_t kSlots = 1024;
+
+struct WordPool {
+  std::mutex mu;
+  std::vector<uint32_t*> free;
+  std::map<unsigned long long, uint32_t*> streams;  // by stream id
+  // by capture id and stream handle
+  std::map<std::pair<unsigned long long, unsigned long long>, uint32_t*> captures;
+};
+
+// Never destroyed: graphs may outlive the library's static objects.
+WordPool& word_pool(int dev) {
+  static WordPool* pools = new WordPool[64];
+  return pools[dev];
+}
+
+// Calls that a capture elsewhere in the process would otherwise forbid.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+cudaError_t take_slot(WordPool& p, uint32_t** out) {
+  if (p.free.empty()) {
+    RelaxedCapture relaxed;
+    uint32_t* slab = nullptr;
+    cudaError_t e = cudaMalloc(&slab, kSlots * kLaunchWords * sizeof(uint32_t));
+    if (e != cudaSuccess) return e;
+    for (size_t i = 0; i < kSlots; ++i) p.free.push_back(slab + i * kLaunchWords);
+  }
+  *out = p.free.back();
+  p.free.pop_back();
+  return cudaSuccess;
+}
+
+struct CapturedSlot {
+  WordPool* pool;
+  std::pair<unsigned long long, unsigned long long> key;
+};
+
+void release_captured(void* arg) {
+  CapturedSlot* c = static_cast<CapturedSlot*>(arg);
+  {
+    std::lock_guard<std::mutex> lk(c->pool->mu);
+    auto it = c->pool->captures.find(c->key);
+    if (it != c->pool->captures.end()) {
+      c->pool->free.push_back(it->second);
+      c->pool->captures.erase(it);
+    }
+  }
+  delete c;
+}
+
+}  // namespace
+
+namespace {
+LaunchWords find_words(cudaStream_t st) {
+  LaunchWords w;
+  auto failed = [&w](cudaError_t e) {
+    w.error = e;
+    if (w.lock.owns_lock()) w.lock.unlock();
+    return std::move(w);
+  };
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && (dev < 0 || dev >= 64)) e = cudaErrorInvalidDevice;
+  if (e != cudaSuccess) return failed(e);
+  unsigned long long id = 0, capture = 0;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(st, &status, &capture, &graph) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream beside a capture: the launch itself will say
+    status = cudaStreamCaptureStatusNone;
+  }
+  if (status == cudaStreamCaptureStatusActive)
+    id = reinterpret_cast<unsigned long long>(st);  // alive while it captures; has no id then
+  else
+    e = cudaStreamGetId(st, &id);
+  if (e != cudaSuccess) return failed(e);
+  WordPool& p = word_pool(dev);
+  w.lock = std::unique_lock<std::mutex>(p.mu);
+  if (status != cudaStreamCaptureStatusActive) {
+    auto it = p.streams.find(id);
+    if (it == p.streams.end()) {
+      if (p.streams.size() >= kSlots) {
+        RelaxedCapture relaxed;
+        if (cudaDeviceSynchronize() == cudaSuccess) {
+          for (auto& s : p.streams) p.free.push_back(s.second);
+          p.streams.clear();
+        } else {
+          cudaGetLastError();
+        }
+      }
+      uint32_t* slot = nullptr;
+      e = take_slot(p, &slot);
+      if (e != cudaSuccess) return failed(e);
+      it = p.streams.emplace(id, slot).first;
+    }
+    w.words = it->second;
+    return w;
+  }
+  const auto key = std::make_pair(capture, id);
+  auto it = p.captures.find(key);
+  if (it == p.captures.end()) {
+    uint32_t* slot = nullptr;
+    e = take_slot(p, &slot);
+    if (e != cudaSuccess) return failed(e);
+    CapturedSlot* c = new CapturedSlot{&p, key};
+    cudaUserObject_t obj = nullptr;
+    e = cudaUserObjectCreate(&obj, c, release_captured, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+      delete c;
+      p.free.push_back(slot);
+      return failed(e);
+    }
+    it = p.captures.emplace(key, slot).first;
+    e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) {
+      w.lock.unlock();
+      cudaUserObjectRelease(obj, 1);  // gives the slot back
+      return failed(e);
+    }
+  }
+  w.words = it->second;
+  return w;
+}
+}  // namespace
+
+LaunchWords launch_words(cudaStream_t st) {
+  try {
+    return find_words(st);
+  } catch (const std::bad_alloc&) {
+    LaunchWords w;
+    w.error = cudaErrorMemoryAllocation;
+    return w;
+  }
 }
 
 }  // namespace re

@@ -4,6 +4,7 @@
 
 #include <cstdarg>
 #include <cstdio>
+#include <mutex>
 #include <string>
 
 #include "../../include/rayengine_b200.h"
@@ -44,5 +45,19 @@ void camera_basis(const re_camera& cam, CamBasis& out);
 void perlin_permutation(uint32_t seed, uint32_t out[512]);
 
 int sm_count();
+
+// Device memory for the claim cursor of a launch on `st` (kLaunchWords words)
+// that no launch which may run beside it uses: every stream has its own, and
+// every graph that is being captured has one per stream of the capture, until
+// the graph and what was instantiated from it are gone.  The caller sets it
+// and launches on `st` before it lets go of the lock.  words null: `error`
+// says why.
+constexpr unsigned kLaunchWords = 8;
+struct LaunchWords {
+  std::unique_lock<std::mutex> lock;
+  uint32_t* words = nullptr;
+  cudaError_t error = cudaSuccess;
+};
+LaunchWords launch_words(cudaStream_t st);
 
 }  // namespace re

@@ -178,15 +178,6 @@ int blocks_for(uint64_t n) {
   uint64_t cap = (uint64_t)sm_count() * 8;
   return (int)(b < cap ? (b ? b : 1) : cap);
 }
-
-// Claim cursor of the SDF kernel, one per device.
-uint32_t* sdf_counter() {
-  static uint32_t* ptrs[64] = {nullptr};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  if (!ptrs[dev] && cudaMalloc(&ptrs[dev], 16) != cudaSuccess) return nullptr;
-  return ptrs[dev];
-}
 }  // namespace
 
 }  // namespace re
@@ -232,8 +223,6 @@ RE_API re_status re_sdf_trace(const re_sdf_params* p, const re_camera* cam, uint
   if (p->octaves > 32) return re::fail(RE_ERR_LIMIT, "re_sdf_trace: octaves > 32");
   if (p->max_steps == 0 || p->max_steps > (1u << 20))
     return re::fail(RE_ERR_LIMIT, "re_sdf_trace: max_steps must be in [1, 2^20]");
-  uint32_t* counter = re::sdf_counter();
-  if (!counter) return re::fail(RE_ERR_CUDA, "re_sdf_trace: counter allocation failed");
   re::PermTable t = re::make_perm(p->seed);
   re::SdfDev sp;
   sp.octaves = p->octaves;
@@ -252,12 +241,14 @@ RE_API re_status re_sdf_trace(const re_sdf_params* p, const re_camera* cam, uint
   cd.vertical = {b.vertical[0], b.vertical[1], b.vertical[2]};
   cd.focal = b.focal;
   cudaStream_t st = (cudaStream_t)stream;
-  RE_CUDA(cudaMemsetAsync(counter, 0, 4, st));
+  const re::LaunchWords cursor = re::launch_words(st);
+  if (!cursor.words) return re::cuda_fail(cursor.error, "re_sdf_trace: claim cursor");
+  RE_CUDA(cudaMemsetAsync(cursor.words, 0, 4, st));
   RE_CUDA(cudaFuncSetAttribute(re::k_sdf, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)re::kRowsSmemBytes));
   re::k_sdf<<<re::sm_count(), re::kRowsThreads, re::kRowsSmemBytes, st>>>(
       t, sp, cd, w, h, re::rows_spread((uint64_t)w * h, (uint32_t)re::sm_count()),
-      reinterpret_cast<float4*>(d_out), counter);
+      reinterpret_cast<float4*>(d_out), cursor.words);
   RE_CHECK_LAUNCH("re_sdf_trace: launch");
   return RE_OK;
 }

@@ -408,18 +408,6 @@ PermTable perm_table(uint32_t seed) {
   return t;
 }
 
-// Per-device scratch of the shading kernel: the tile cursor and the
-// shadow-march evaluation count.
-uint32_t* counters() {
-  static uint32_t* ptrs[64] = {nullptr};
-  static std::mutex mu;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lk(mu);
-  if (!ptrs[dev] && cudaMalloc(&ptrs[dev], 64) != cudaSuccess) return nullptr;
-  return ptrs[dev];
-}
-
 re_status check_shade(const re_sdf_shade_params* s, const char* fn) {
   if (!s) return fail(RE_ERR_INVALID_ARG, "%s: null shade parameters", fn);
   if (s->flags & ~(uint32_t)(RE_SDF_SHADE | RE_SDF_FOG | RE_SDF_GAMMA | RE_SDF_VIGNETTING))
@@ -462,8 +450,6 @@ ShadeDev shade_dev(const re_sdf_params& f, const re_sdf_shade_params& s) {
 re_status shade(const re_sdf_params& f, const re_sdf_shade_params& s, const re_camera& cam,
                 uint32_t w, uint32_t h, const re_sdf_hit* d_hits, uint32_t* d_rgba,
                 cudaStream_t st, uint64_t* d_evals) {
-  uint32_t* ctr = counters();
-  if (!ctr) return fail(RE_ERR_CUDA, "re_render_sdf_frame: counter allocation failed");
   CamBasis b;
   camera_basis(cam, b);
   CamDev cd;
@@ -473,13 +459,15 @@ re_status shade(const re_sdf_params& f, const re_sdf_shade_params& s, const re_c
   cd.vertical = {b.vertical[0], b.vertical[1], b.vertical[2]};
   cd.focal = b.focal;
   if (s.flags & RE_SDF_SHADE) {
-    RE_CUDA(cudaMemsetAsync(ctr, 0, 4, st));
+    const LaunchWords cursor = launch_words(st);
+    if (!cursor.words) return cuda_fail(cursor.error, "re_render_sdf_frame: claim cursor");
+    RE_CUDA(cudaMemsetAsync(cursor.words, 0, 4, st));
     RE_CUDA(cudaFuncSetAttribute(k_sdf_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kRowsSmemBytes));
     k_sdf_shadow<<<sm_count(), kRowsThreads, kRowsSmemBytes, st>>>(
         perm_table(f.seed), shade_dev(f, s), w, h,
         rows_spread((uint64_t)w * h, (uint32_t)sm_count()),
-        reinterpret_cast<const float4*>(d_hits), d_rgba, ctr,
+        reinterpret_cast<const float4*>(d_hits), d_rgba, cursor.words,
         reinterpret_cast<unsigned long long*>(d_evals));
     RE_CHECK_LAUNCH("re_render_sdf_frame: shadow launch");
   }
