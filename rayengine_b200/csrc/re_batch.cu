@@ -267,6 +267,7 @@ __device__ __forceinline__ bool run_kind(const BatchDev& B, const SceneDev* sc,
                                          uint32_t epoch, uint32_t& trip, Counters& cnt,
                                          uint32_t& errors, bool& primary_done) {
   const uint32_t* sperm_w = reinterpret_cast<const uint32_t*>(sperm);
+  const uint32_t field = after_barrier((uint32_t)__cvta_generic_to_shared(sperm));
   uint32_t* ctr = B.ctr;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt_mask = (1u << lane) - 1u;
@@ -453,8 +454,7 @@ __device__ __forceinline__ bool run_kind(const BatchDev& B, const SceneDev* sc,
         }
         float v = 0.f;
         if constexpr (TABLE == kFieldTables) {
-          const FieldWords P{(uint32_t)__cvta_generic_to_shared(sperm) +
-                             kFieldWordsBytes * S.perm_slot};
+          const FieldWords P{field + kFieldWordsBytes * S.perm_slot};
           // with two lanes to a point as well, six scenes took 3.08 ms against
           // 2.62: the mesh walk's code runs beside this on every SM
           v = warp_density<1, false>(P, q, runs, S.octaves, S.scale, S.amp);

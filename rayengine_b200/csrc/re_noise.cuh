@@ -248,6 +248,14 @@ __host__ __device__ __forceinline__ uint32_t grad_bytes(uint32_t p) {
   return (gx << 24) | (gy << 16) | gz;
 }
 
+// A table's base address, for row_word(), whose loads the compiler takes for
+// functions of the address alone: they depend on this value, and it comes
+// from behind the barrier that publishes the table.
+__device__ __forceinline__ uint32_t after_barrier(uint32_t base) {
+  asm volatile("" : "+r"(base) : : "memory");
+  return base;
+}
+
 // smem: kRowsSmemBytes; every thread of the block calls it.
 __device__ __forceinline__ FieldRows load_rows(const PermTable& t, uint32_t* smem) {
   const uint32_t lane = threadIdx.x & 31u;
@@ -257,7 +265,7 @@ __device__ __forceinline__ FieldRows load_rows(const PermTable& t, uint32_t* sme
     smem[64u * j + 32u + lane] = grad_bytes(p);
   }
   __syncthreads();
-  return FieldRows{(uint32_t)__cvta_generic_to_shared(smem) + 4u * lane};
+  return FieldRows{after_barrier((uint32_t)__cvta_generic_to_shared(smem) + 4u * lane)};
 }
 
 typedef unsigned long long f32x2;
@@ -295,6 +303,7 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   return r;
 }
 
+// A word of a table whose base went through after_barrier().
 template <uint32_t OFF>
 __device__ __forceinline__ uint32_t row_word(uint32_t addr) {
   uint32_t r;
