@@ -242,10 +242,9 @@ __device__ __forceinline__ uint32_t closed_mask(const uint32_t* ctr, const Batch
   return mask;
 }
 
-// TABLE: the terrain tables in shared memory, by the number of seeds (larger
-// tables would cost blocks per SM): kFieldTables, the paired form's A and G
-// words (4 KB per seed); kWordTables, perm_word() entries (2 KB); kByteTables,
-// bytes (512 B); kNoTables: a batch of meshes alone.
+// TABLE: the terrain tables in shared memory (table_of chooses): kFieldTables,
+// the paired form's A and G words (4 KB per seed); kWordTables, perm_word()
+// entries (2 KB); kByteTables, bytes (512 B); kNoTables: a batch of meshes alone.
 enum : int { kByteTables = 0, kWordTables = 1, kFieldTables = 2, kNoTables = 3 };
 __host__ __device__ constexpr uint32_t table_bytes(int table) {
   return table == kFieldTables ? kFieldWordsBytes : table == kWordTables ? 2048u : 512u;
@@ -778,26 +777,47 @@ uint32_t layout_stage(re_batch* b, uint32_t stage_nodes) {
   return off;
 }
 
-// The largest tables that leave room for four blocks per SM: the paired
-// form's up to 12 seeds (48 KB), words up to 16 (32 KB).
-constexpr uint32_t kFieldTablesMax = 12, kWordTablesMax = 16;
-
-int table_of(const re_batch* b) {
-  const size_t seeds = b->perms.size() / 512;
-  return seeds == 0                 ? kNoTables
-         : seeds <= kFieldTablesMax ? kFieldTables
-         : seeds <= kWordTablesMax  ? kWordTables
-                                    : kByteTables;
-}
-
-size_t smem_bytes(const re_batch* b, uint32_t stage_total, uint32_t block_threads) {
-  return b->num_scenes * sizeof(SceneDev) + b->perms.size() / 512 * table_bytes(table_of(b)) +
+size_t smem_bytes(const re_batch* b, int table, uint32_t stage_total, uint32_t block_threads) {
+  return b->num_scenes * sizeof(SceneDev) + b->perms.size() / 512 * table_bytes(table) +
          (size_t)stage_total * sizeof(uint2) + (size_t)(block_threads / 32) * kMaxDepth * 4;
 }
 
+// Blocks that an SM holds: 64 registers a thread of 65,536 (__launch_bounds__),
+// and 228 KB of shared memory, of which a block takes 1 KB for itself.
+uint32_t blocks_per_sm(size_t smem, uint32_t block_threads) {
+  return std::min<uint32_t>(1024u / block_threads, 233472u / (uint32_t)(smem + 1024u));
+}
+
+// The terrain tables.  Beside them a block holds 192 bytes a scene and the
+// staged nodes, so the paired form's 4 KB a seed are taken (up to 12 seeds)
+// where they leave as many blocks on an SM as the words' 2 KB do, or, in a
+// batch that is mostly terrain, half as many: fewer warps slow the mesh walks,
+// which wait for memory, more than the paired form gains.  Measured on B200,
+// 160x90 a scene, 12 seeds, words against the paired form: 2 meshes 4 | 4
+// blocks 1896 -> 1490 us, 512 nodes staged 4 | 3 1917 -> 1287, blocks of 128
+// threads 8 | 4 1903 -> 1578; 20 meshes, 512 nodes 2 | 1 2476 -> 3136; 44
+// meshes, 128 threads 6 | 3 3111 -> 3775.  Words up to 16 seeds, then bytes.
+constexpr uint32_t kFieldTablesMax = 12, kWordTablesMax = 16;
+constexpr size_t kMaxSmem = 232448;
+
+int table_of(const re_batch* b, uint32_t stage_total, uint32_t block_threads) {
+  const size_t seeds = b->perms.size() / 512;
+  if (seeds == 0) return kNoTables;
+  if (seeds > kWordTablesMax) return kByteTables;
+  if (seeds > kFieldTablesMax ||
+      smem_bytes(b, kFieldTables, stage_total, 512) > kMaxSmem)
+    return kWordTables;
+  const uint32_t field =
+      blocks_per_sm(smem_bytes(b, kFieldTables, stage_total, block_threads), block_threads);
+  const uint32_t word =
+      blocks_per_sm(smem_bytes(b, kWordTables, stage_total, block_threads), block_threads);
+  const bool terrain = b->cap[kTerrain] >= b->cap[kMesh];
+  return (terrain ? 2u : 1u) * field >= word ? kFieldTables : kWordTables;
+}
+
 using Kernel = void (*)(BatchDev);
-Kernel kernel_of(const re_batch* b, bool count) {
-  switch (table_of(b)) {
+Kernel kernel_of(int table, bool count) {
+  switch (table) {
     case kFieldTables: return count ? k_batch<true, kFieldTables> : k_batch<false, kFieldTables>;
     case kWordTables: return count ? k_batch<true, kWordTables> : k_batch<false, kWordTables>;
     case kNoTables: return count ? k_batch<true, kNoTables> : k_batch<false, kNoTables>;
@@ -812,10 +832,11 @@ re_status prepare(re_batch* b, const re_batch_tuning& tn, cudaStream_t st) {
   RE_CUDA(cudaMemcpyAsync(b->d_scenes, b->host_scenes.data(), b->num_scenes * sizeof(SceneDev),
                           cudaMemcpyHostToDevice, st));
   RE_CUDA(cudaStreamSynchronize(st));
-  int bytes = (int)smem_bytes(b, stage_total, 512);
+  const int table = table_of(b, stage_total, tn.block_threads);
+  int bytes = (int)smem_bytes(b, table, stage_total, 512);
   for (bool count : {false, true})
-    RE_CUDA(cudaFuncSetAttribute(kernel_of(b, count), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 bytes));
+    RE_CUDA(cudaFuncSetAttribute(kernel_of(table, count),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   return RE_OK;
 }
 
@@ -823,9 +844,10 @@ re_status prepare(re_batch* b, const re_batch_tuning& tn, cudaStream_t st) {
 re_status launch(re_batch* b, float* d_radiance, re_hit* d_primary, cudaStream_t st,
                  const re_batch_tuning& tn, unsigned long long* totals = nullptr) {
   uint32_t stage_total = layout_stage(b, tn.stage_nodes);
-  size_t smem = smem_bytes(b, stage_total, tn.block_threads);
+  const int table = table_of(b, stage_total, tn.block_threads);
+  size_t smem = smem_bytes(b, table, stage_total, tn.block_threads);
   int per_sm = 0;
-  const Kernel kern = kernel_of(b, totals != nullptr);
+  const Kernel kern = kernel_of(table, totals != nullptr);
   RE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)tn.block_threads,
                                                         smem));
   if (per_sm < 1) return fail(RE_ERR_LIMIT, "re_batch: tuning does not fit on an SM");
@@ -1146,7 +1168,8 @@ RE_API re_status re_batch_autotune(re_batch* b, float* d_radiance, void* stream,
       for (uint32_t sg : stages)
         for (uint32_t tp : trips) {
         re_batch_tuning t = {bt, rf, sg, tp};
-        size_t smem = re::smem_bytes(b, re::layout_stage(b, sg), bt);
+        const uint32_t staged = re::layout_stage(b, sg);
+        size_t smem = re::smem_bytes(b, re::table_of(b, staged, bt), staged, bt);
         if (smem > 200 * 1024) continue;
         s = re::prepare(b, t, st);
         if (s != RE_OK) break;

@@ -1,4 +1,5 @@
-"""The batched renderer at its limits: claims of waiting warps."""
+"""The batched renderer at its limits: claims of waiting warps, and shared
+memory nearly full of staged nodes and terrain tables."""
 import numpy as np
 import pytest
 import torch
@@ -33,4 +34,32 @@ def test_waiting_warps_claim_once(cuda, order):
         assert (claims >= pixels).all()
         assert (claims <= pixels + 32 * warps).all(), claims
         assert np.array_equal(b.render(graph=True).cpu().numpy(), rad)
+    mesh.close()
+
+
+# scenes, block size, staged nodes per mesh: the paired tables of 12 seeds (48
+# KB) do not fit beside the staged nodes, fit with fewer blocks per SM than the
+# words (24 KB) in a batch of meshes and in one of terrains, and fit as often
+@pytest.mark.parametrize("order,threads,stage", [
+    ("m" * 6 + "t" * 12, 256, 4096), ("m" * 20 + "t" * 12, 256, 512),
+    ("mm" + "t" * 12, 128, 0), ("m" * 44 + "t" * 12, 128, 0), ("mm" + "t" * 12, 256, 0)])
+def test_tables_beside_staged_nodes(cuda, order, threads, stage):
+    cfg = rb.configs.SoupConfig(num_tris=16384)
+    mesh = rb.KDScene.from_packed(cfg.packed(), cfg.kd_params())
+    assert mesh.stats()["num_nodes"] >= 4096
+    specs = []
+    for i, k in enumerate(order):
+        if k == "m":
+            specs.append(dict(mesh=mesh, camera=_cam(24, 18), width=24, height=18, albedo=0.7))
+        else:
+            tc = rb.configs.TerrainConfig(seed=900 + i, width=14, height=9)
+            specs.append(dict(terrain=tc.params(), camera=tc.camera(), width=14, height=9,
+                              albedo=0.6))
+    with rb.Batch(specs, max_depth=3, seed=2, mesh_bias=1e-4) as b:
+        want = b.render().cpu().numpy()  # the default tuning stages nothing
+        counts = b.counts()
+        b.set_tuning(threads, 8, stage, 8)
+        for graph in (False, True):
+            assert np.array_equal(b.render(graph=graph).cpu().numpy(), want)
+        assert b.stats()["error"] == 0 and b.counts() == counts
     mesh.close()
