@@ -769,7 +769,7 @@ uint32_t layout_stage(re_batch* b, uint32_t stage_nodes) {
       s.stage_off = 0;
       continue;
     }
-    uint32_t n = (uint32_t)std::min<size_t>(stage_nodes, b->meshes[i]->host.nodes.size());
+    uint32_t n = std::min(stage_nodes, b->meshes[i]->host.num_nodes);
     s.stage = n;
     s.stage_off = off;
     off += n;

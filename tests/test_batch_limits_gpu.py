@@ -63,3 +63,17 @@ def test_tables_beside_staged_nodes(cuda, order, threads, stage):
             assert np.array_equal(b.render(graph=graph).cpu().numpy(), want)
         assert b.stats()["error"] == 0 and b.counts() == counts
     mesh.close()
+
+
+def test_no_more_nodes_staged_than_there_are(cuda):
+    """Eight trees of some 2200 nodes fit in shared memory; the 4096 asked for
+    of each would not."""
+    cfg = rb.configs.SoupConfig(num_tris=5000)
+    mesh = rb.KDScene.from_packed(cfg.packed(), cfg.kd_params())
+    assert 2048 < mesh.stats()["num_nodes"] < 3000
+    scene = dict(mesh=mesh, camera=_cam(24, 18), width=24, height=18, albedo=0.7)
+    with rb.Batch([scene] * 8, max_depth=3, seed=2, mesh_bias=1e-4) as b:
+        want = b.render().cpu().numpy()
+        b.set_tuning(256, 8, 4096, 8)
+        assert np.array_equal(b.render().cpu().numpy(), want)
+    mesh.close()
