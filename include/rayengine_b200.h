@@ -105,6 +105,9 @@ typedef struct re_kd_params {
 
 typedef struct re_scene re_scene;
 
+/* re_tuning.ray_refill_min: more idle lanes than a warp has, so never refilled. */
+#define RE_RAY_NO_REFILL 33u
+
 /* Launch tuning of a scene (see re_autotune_ao, re_autotune_primary). */
 typedef struct re_tuning {
   uint32_t stage_nodes;      /* top nodes staged in shared memory per block (<= 8192) */
@@ -112,16 +115,16 @@ typedef struct re_tuning {
                                 2 shadow rays first, then each pixel's AO rays    */
   uint32_t refill_min;       /* idle lanes before a warp claims new secondary rays, 1..32 */
   uint32_t ray_refill_min;   /* the same for primary and caller rays (re_trace_primary,
-                                re_count_primary, re_trace_rays), 1..32; 32 (default):
-                                chosen by the number of rays */
+                                re_count_primary, re_trace_rays), 1..31; 32 (default): how
+                                rays are walked is chosen by their number and the tree;
+                                RE_RAY_NO_REFILL: each lane runs its ray to the end */
   uint32_t ray_lanes;        /* lanes per primary ray in re_trace_primary: 1 (default; 0
-                                reads as 1; with ray_refill_min 32: chosen by the number of
-                                rays and the tree's leaves), 2, 4 or 8.  Above 1 the lanes of a ray split
-                                each leaf's triangle tests (same hits); it shortens the
-                                longest walks of frames too small to fill the GPU.  32:
-                                one ray per lane, and the warp tests the triangles of all
-                                its lanes' leaves together (finished lanes help; same
-                                hits) */
+                                reads as 1; with ray_refill_min 32 the choice above), 2, 4
+                                or 8.  Above 1 the lanes of a ray split each leaf's
+                                triangle tests (same hits); it shortens the longest walks
+                                of frames too small to fill the GPU.  32: one ray per
+                                lane, and the warp tests the triangles of all its lanes'
+                                leaves together (finished lanes help; same hits) */
 } re_tuning;
 
 typedef struct re_scene_stats {

@@ -34,6 +34,7 @@ from ._lib import RayEngineError, call, lib  # noqa: F401
 TRACE_TWO_SIDED = 0
 TRACE_ONE_SIDED = 1
 TRACE_ANY_HIT = 2
+RAY_NO_REFILL = 33  # set_tuning's ray_refill_min: each lane runs its ray to the end
 
 HIT_DTYPE = np.dtype([("id", "<i4"), ("t", "<f4"), ("u", "<f4"), ("v", "<f4")])
 SDF_HIT_DTYPE = np.dtype(

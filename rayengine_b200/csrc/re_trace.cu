@@ -731,8 +731,9 @@ namespace {
 
 // The form of a ray pass: lanes per ray (1, 2, 4, 8 or kWholeWarp), or 32
 // for one ray per lane with the warp's tests together.  A tuning other than
-// the default says which (caller rays: ray_refill_min only).  By default it
-// follows the number of rays and the tree; every form finds the same hits.
+// the default says which (caller rays: ray_refill_min only; RE_RAY_NO_REFILL
+// with one lane: the plain walk).  By default it follows the number of rays
+// and the tree; every form finds the same hits.
 //   Few rays leave the GPU idle and their time is that of the longest walk,
 // which the other rays of its warp stretch (their descents and tests take
 // turns): give each more lanes.  Measured on B200, one lane per ray against
@@ -750,7 +751,7 @@ namespace {
 // the plain walk stays (2048x2048 489 us against 544).
 constexpr uint32_t kWholeWarp = 64;
 uint32_t ray_form(const re_scene* s, uint32_t n, bool frame) {
-  const bool by_size = s->tune.ray_refill_min >= 32u && (!frame || s->tune.ray_lanes <= 1u);
+  const bool by_size = s->tune.ray_refill_min == 32u && (!frame || s->tune.ray_lanes <= 1u);
   if (!by_size) return frame ? s->tune.ray_lanes : 1u;
   if (n <= 4096u) return kWholeWarp;
   if (n <= 40960u) return 8u;
@@ -1200,9 +1201,10 @@ RE_API re_status re_scene_get_tuning(const re_scene* s, re_tuning* out) {
 
 RE_API re_status re_scene_set_tuning(re_scene* s, const re_tuning* t) {
   if (!s || !t) return re::fail(RE_ERR_INVALID_ARG, "re_scene_set_tuning: null argument");
-  if (t->refill_min < 1 || t->refill_min > 32 || t->ray_refill_min < 1 || t->ray_refill_min > 32)
+  if (t->refill_min < 1 || t->refill_min > 32 || t->ray_refill_min < 1 ||
+      t->ray_refill_min > RE_RAY_NO_REFILL)
     return re::fail(RE_ERR_INVALID_ARG,
-                    "re_scene_set_tuning: refill_min and ray_refill_min must be in [1, 32]");
+                    "re_scene_set_tuning: refill_min must be in [1, 32], ray_refill_min in [1, 33]");
   if (t->queue_kind_major > 2)
     return re::fail(RE_ERR_INVALID_ARG, "re_scene_set_tuning: queue_kind_major must be 0, 1 or 2");
   if ((t->ray_lanes > 8 && t->ray_lanes != 32) || (t->ray_lanes & (t->ray_lanes - 1u)))
@@ -1286,8 +1288,9 @@ RE_API re_status re_autotune_ao(re_scene* s, const re_camera* cam, uint32_t w, u
 }
 
 // Times the primary pass (re_trace_primary with `flags`) for every
-// combination of staging depth and walk form (one lane per ray with each
-// refill threshold, or 2, 4 or 8 lanes per ray; one warm-up and three timed
+// combination of staging depth and walk form (the one that the frame's size
+// and the tree choose by default, refill thresholds of 4, 8 and 16, 2, 4 or 8
+// lanes per ray, or the warp's tests together; one warm-up and three timed
 // passes each, CUDA events on the caller's stream) and keeps the fastest on
 // the scene.  Each timed pass follows a write of twice the L2 size, so the
 // forms are compared on a frame whose tree is not cached (as after other

@@ -130,3 +130,19 @@ def test_measurement_probes_reject_bad_sizes():
     for iters in (0, 1000, (1 << 20) + 1):
         assert _lib.lib.re_measure_fp32_fma(iters, ctypes.byref(v), None) == 1
     assert _lib.lib.re_measure_fp32_fma(1 << 16, None, None) == 1
+
+
+def test_plain_walk_can_be_asked_for():
+    """ray_refill_min above a warp's 32 lanes: no refill, whatever the number
+    of rays (32, the default, lets the library choose)."""
+    packed = rb.configs.SoupConfig(num_tris=64).packed()
+    with rb.KDScene.build_host(packed) as sc:
+        t = sc.tuning()
+        sc.set_tuning(t["stage_nodes"], 0, 8, rb.RAY_NO_REFILL, 1)
+        assert sc.tuning()["ray_refill_min"] == rb.RAY_NO_REFILL == 33
+        for bad in (0, 34, 64):
+            with pytest.raises(rb.RayEngineError) as e:
+                sc.set_tuning(t["stage_nodes"], 0, 8, bad, 1)
+            assert e.value.status == 1
+        with pytest.raises(rb.RayEngineError):
+            sc.set_tuning(t["stage_nodes"], 0, rb.RAY_NO_REFILL, 32, 1)

@@ -92,3 +92,23 @@ def test_visit_cap(cuda, n):
         assert sc.truncated() == cut > n // 20
         assert torch.equal(sc.trace_rays(dr, rb.TRACE_ANY_HIT), hit)
         assert sc.truncated() == any_cut > 0
+
+
+@pytest.mark.parametrize("long_leaves", [False, True])
+def test_plain_walk(cuda, long_leaves):
+    """The walk without refill or shared lanes, where the default chooses
+    another form: the same hits."""
+    rays = _rays(50001)
+    with _scene(long_leaves) as sc:
+        dr = torch.from_numpy(rays).cuda()
+        cam = rb.build_camera((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), (60.0, 50.0))
+        t = sc.tuning()
+        want = [[sc.trace_primary(cam, w, h) for w, h in SIZES],
+                [sc.trace_rays(dr[:n].contiguous(), f) for n in (1000, 20000, 50001)
+                 for f in (0, rb.TRACE_ANY_HIT)]]
+        sc.set_tuning(t["stage_nodes"], t["queue_kind_major"], t["refill_min"], rb.RAY_NO_REFILL)
+        got = [[sc.trace_primary(cam, w, h) for w, h in SIZES],
+               [sc.trace_rays(dr[:n].contiguous(), f) for n in (1000, 20000, 50001)
+                for f in (0, rb.TRACE_ANY_HIT)]]
+        for a, b in zip(want[0] + want[1], got[0] + got[1]):
+            assert torch.equal(a, b)
