@@ -52,15 +52,27 @@ __device__ __forceinline__ void ldg_pair(const float4* p, float4& a, float4& b) 
 // Inner nodes a step descends before it is put off to the next one (trav_step's
 // DESCENT).  A rope leads 1.7 nodes above its leaf on average, but the longest
 // of a warp's 28 descents took 9, with 5 lanes at work: lanes at their leaf
-// now go on while the others finish their descent beside the next ones.
-// Measured on B200 (heightfield of 2.1M triangles): AO pass 2.30 -> 1.89 ms at
-// 3 (2: 2.00, 4: 1.90, 6: 2.00); primary tiles 624 -> 603 us at 6 (3: 617);
-// refilled random rays 338 -> 311 at 4.  Where the warp's lanes walk together
-// to share a leaf's tests, and in the batch renderer (at its register limit),
-// a whole descent stays the faster (2048x2048 soup 634 us against 654 to 679;
-// six scenes 2.65 ms against 2.80 to 3.05).
+// now go on while the others finish their descent beside the next ones.  In
+// trees of long leaves (launch code: three references or more) a step's tests
+// outlast its descents, and few descents are worth cutting short.
+// Measured on B200, 1920x1080, a whole descent against the limit taken, in
+// trees of short and of long leaves (the 2.1M-triangle heightfield of 1.3
+// references a leaf, soup of 262,144 triangles of 5.6):
+//   AO frame               2919 -> 2510 us at 3 (6: 2615)     2287 -> 2307 at 8 (3: 2544)
+//   AO frame, refill 32    3624 -> 3430 at 6 (3: 3456)        3392 -> 3430 at 8 (3: 3830)
+//   primary tiles          624 -> 603 at 6 (3: 617)           whole
+//   frame, refill 8        778 -> 753 at 6 (4: 759)           486 -> 477 at 12 (4: 508)
+//   random rays, refill 8  1200 -> 1105 at 6 (4: 1145)        786 -> 763 at 12 (4: 774)
+// (the other trees of long leaves, 3.2 to 7 references: AO frames 1 to 3 %
+// faster at 8 than whole).  A whole descent stays the faster where the warp's
+// lanes walk together to share a leaf's tests, in the batch renderer (at its
+// register limit), in the counting passes, and for caller rays walked in
+// chunks to the closest hit (2,073,600 random rays 1395 us against 1442 at 6;
+// any hit 1434 against 1336).
 constexpr uint32_t kWholeDescent = 0xFFFFFFFFu;
-constexpr uint32_t kTileDescent = 6, kAoDescent = 3, kRefillDescent = 4;
+constexpr uint32_t kTileDescent = 6;
+constexpr uint32_t kAoDescent = 3, kAoNoRefillDescent = 6, kAoLongDescent = 8;
+constexpr uint32_t kRefillDescent = 6, kRefillLongDescent = 12;
 
 // Trav::visits of a walk that stopped at the leaf-visit cap.
 constexpr uint32_t kTruncated = 0xFFFFFFFFu;
@@ -560,12 +572,12 @@ __device__ __forceinline__ void trav_result(const Trav& s, HitState& hs) {
 }
 
 // Runs one ray to the end; returns true when it stopped at the leaf-visit cap.
-template <int MODE, bool ANYHIT, bool COUNT>
+template <int MODE, bool ANYHIT, bool COUNT, uint32_t DESCENT = kTileDescent>
 __device__ __forceinline__ bool traverse(const KdDev& kd, const uint2* snodes, V3 o, V3 d,
                                          float tmax, uint32_t start, HitState& hs, Counters& c) {
   Trav s;
   trav_init(s, kd, o, d, tmax, start);
-  while (s.live) trav_step<MODE, ANYHIT, COUNT, 1, kTileDescent>(s, kd, snodes, c);
+  while (s.live) trav_step<MODE, ANYHIT, COUNT, 1, DESCENT>(s, kd, snodes, c);
   trav_result(s, hs);
   return trav_truncated(s);
 }

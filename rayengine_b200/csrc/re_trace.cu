@@ -45,7 +45,7 @@ namespace re {
 // frame has no warp-sized tail.  gen(i, o, d, tmax) -> false for an index
 // without a ray; done(i, s, c) gets the finished walk (c: the ray's own
 // counters when COUNT).
-template <int MODE, bool ANYHIT, bool COUNT, class Gen, class Done>
+template <int MODE, bool ANYHIT, bool COUNT, uint32_t DESCENT, class Gen, class Done>
 __device__ __forceinline__ void refill_walk(const KdDev& kd, const uint2* snodes, uint32_t n,
                                             uint32_t refill_min, uint32_t* counter, Gen gen,
                                             Done done) {
@@ -80,7 +80,7 @@ __device__ __forceinline__ void refill_walk(const KdDev& kd, const uint2* snodes
       continue;
     }
     if (s.live) {
-      trav_step<MODE, ANYHIT, COUNT, 1, kRefillDescent>(s, kd, snodes, c);
+      trav_step<MODE, ANYHIT, COUNT, 1, DESCENT>(s, kd, snodes, c);
       if (!s.live) done(cur, s, c);
     }
   }
@@ -95,7 +95,7 @@ __device__ __forceinline__ void refill_walk(const KdDev& kd, const uint2* snodes
 // Primary rays, persistent warps over 8x4 pixel tiles, each lane running its
 // ray to the end (ray_refill_min 32: no per-leaf bookkeeping; fastest when
 // rays of a tile take similar work).
-template <int MODE, bool COUNT>
+template <int MODE, bool COUNT, uint32_t DESCENT>
 __global__ void __launch_bounds__(256, 6) k_primary_tiles(KdDev kd, CamDev cam, uint32_t w,
                                                        uint32_t h, re_hit* __restrict__ out,
                                                        uint4* __restrict__ counts,
@@ -115,7 +115,8 @@ __global__ void __launch_bounds__(256, 6) k_primary_tiles(KdDev kd, CamDev cam, 
     generate_ray(cam, w, h, x, y, o, d);
     HitState hs;
     Counters c = {0, 0, 0, 0};
-    traverse<MODE, false, COUNT>(kd, snodes, o, d, __int_as_float(0x7f800000), 0u, hs, c);
+    traverse<MODE, false, COUNT, DESCENT>(kd, snodes, o, d, __int_as_float(0x7f800000), 0u, hs,
+                                          c);
     size_t pix = (size_t)y * w + x;
     if (COUNT)
       counts[pix] = make_uint4(c.inner, c.leaf, c.tests, c.status);
@@ -200,7 +201,7 @@ __global__ void __launch_bounds__(256, 4) k_primary_warp(KdDev kd, CamDev cam, u
 // Primary rays with lane refill (ray_refill_min < 32).  Work index i is lane
 // i % 32 of 8x4 pixel tile i / 32, so a warp's claims stay in one screen
 // region.
-template <int MODE, bool COUNT>
+template <int MODE, bool COUNT, uint32_t DESCENT>
 __global__ void __launch_bounds__(256, 6) k_primary(KdDev kd, CamDev cam, uint32_t w, uint32_t h,
                                                  re_hit* __restrict__ out,
                                                  uint4* __restrict__ counts,
@@ -231,12 +232,12 @@ __global__ void __launch_bounds__(256, 6) k_primary(KdDev kd, CamDev cam, uint32
       store_hit(out, pix, hs);
     }
   };
-  refill_walk<MODE, false, COUNT>(kd, snodes, tiles * 32u, refill_min, tile_counter, gen, done);
+  refill_walk<MODE, false, COUNT, DESCENT>(kd, snodes, tiles * 32u, refill_min, tile_counter, gen, done);
 }
 
 // Caller rays (re_ray), persistent warps over 32-ray chunks, each lane
 // running its ray to the end (ray_refill_min 32).
-template <int MODE, bool ANYHIT>
+template <int MODE, bool ANYHIT, uint32_t DESCENT>
 __global__ void __launch_bounds__(256, 6) k_rays_chunks(KdDev kd, const float4* __restrict__ rays,
                                                      uint32_t n, re_hit* __restrict__ out,
                                                      uint32_t* __restrict__ counter, uint32_t) {
@@ -252,13 +253,13 @@ __global__ void __launch_bounds__(256, 6) k_rays_chunks(KdDev kd, const float4* 
     V3 o = {R0.x, R0.y, R0.z}, d = {R1.x, R1.y, R1.z};
     HitState hs;
     Counters c = {0, 0, 0, 0};
-    traverse<MODE, ANYHIT, false>(kd, snodes, o, d, R0.w, 0u, hs, c);
+    traverse<MODE, ANYHIT, false, DESCENT>(kd, snodes, o, d, R0.w, 0u, hs, c);
     store_hit(out, i, hs);
   }
 }
 
 // Caller rays (re_ray), lane refill over ray indices (ray_refill_min < 32).
-template <int MODE, bool ANYHIT>
+template <int MODE, bool ANYHIT, uint32_t DESCENT>
 __global__ void __launch_bounds__(256, 6) k_rays(KdDev kd, const float4* __restrict__ rays,
                                               uint32_t n, re_hit* __restrict__ out,
                                               uint32_t* __restrict__ counter,
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(256, 6) k_rays(KdDev kd, const float4* __restr
     trav_result(s, hs);
     store_hit(out, i, hs);
   };
-  refill_walk<MODE, ANYHIT, false>(kd, snodes, n, refill_min, counter, gen, done);
+  refill_walk<MODE, ANYHIT, false, DESCENT>(kd, snodes, n, refill_min, counter, gen, done);
 }
 
 // Caller rays with G lanes per ray, 32 / G rays to a warp (as
@@ -416,7 +417,7 @@ __device__ __forceinline__ void flush_counts(const Counters& c, uint32_t rays,
 // (ballot + popc) assigns hit ranks.  counters: [0] tile cursor, [1] hits,
 // [2] secondary cursor, [3] secondary rays.  COUNT: also sum the traversal
 // work into totals[0..3].
-template <bool COUNT>
+template <bool COUNT, uint32_t DESCENT>
 __global__ void __launch_bounds__(256, 5) k_ao_primary(KdDev kd, CamDev cam, AoDev ao, uint32_t w,
                                                     uint32_t h, re_hit* __restrict__ out,
                                                     uint32_t* __restrict__ mask,
@@ -439,8 +440,8 @@ __global__ void __launch_bounds__(256, 5) k_ao_primary(KdDev kd, CamDev cam, AoD
     V3 o = {0, 0, 0}, d = {0, 0, 1};
     if (valid) {
       generate_ray(cam, w, h, x, y, o, d);
-      bool cut = traverse<0, false, COUNT>(kd, snodes, o, d, __int_as_float(0x7f800000), 0u,
-                                           hs, c);
+      bool cut = traverse<0, false, COUNT, DESCENT>(kd, snodes, o, d, __int_as_float(0x7f800000),
+                                                    0u, hs, c);
       ++rays;
       size_t pix = (size_t)y * w + x;
       if (!COUNT) {
@@ -513,7 +514,7 @@ __global__ void __launch_bounds__(256, 5) k_ao_primary(KdDev kd, CamDev cam, AoD
 // least aq.refill_min lanes of a warp are idle the warp claims that many new
 // rays with one atomic, so lanes need not wait for the slowest ray of the
 // warp.  The number of hits is read on the device.
-template <bool COUNT>
+template <bool COUNT, uint32_t DESCENT>
 __global__ void __launch_bounds__(256, 5) k_ao_secondary(KdDev kd, AoDev ao, AoQueue aq,
                                                       uint32_t* __restrict__ mask,
                                                       uint32_t* __restrict__ counters,
@@ -568,7 +569,7 @@ __global__ void __launch_bounds__(256, 5) k_ao_secondary(KdDev kd, AoDev ao, AoQ
       continue;
     }
     if (s.live) {
-      trav_step<0, true, COUNT, 1, kAoDescent>(s, kd, snodes, c);
+      trav_step<0, true, COUNT, 1, DESCENT>(s, kd, snodes, c);
       if (!s.live && !COUNT) {
         uint32_t bits = (s.best_id < 0 ? 1u << (tag & 7u) : 0u) |
                         (trav_truncated(s) ? kMaskTruncated : 0u);
@@ -638,6 +639,10 @@ re_status check_scene(const re_scene* s, const char* fn) {
                 s->device, dev);
   return RE_OK;
 }
+
+// Trees of long leaves: three references or more in each (the random soups
+// hold 5.3 to 5.6 in leaves of up to 8, the heightfield's default tree 1.3).
+bool long_leaves(const re_scene* s) { return s->host.num_refs >= 3ull * s->host.num_leaves; }
 
 template <typename K>
 int grid_for(K kernel, size_t smem) {
@@ -756,7 +761,7 @@ uint32_t ray_form(const re_scene* s, uint32_t n, bool frame) {
   if (n <= 4096u) return kWholeWarp;
   if (n <= 40960u) return 8u;
   if (frame && n <= 81920u) return 4u;
-  return s->host.num_refs >= 3ull * s->host.num_leaves ? 32u : 1u;
+  return long_leaves(s) ? 32u : 1u;
 }
 
 int blocks_for(int grid, uint32_t rays, uint32_t rays_per_warp) {
@@ -776,13 +781,16 @@ re_status launch_primary(re_scene* s, const re_camera& cam, uint32_t w, uint32_t
   CamDev cd = cam_view(cam);
   size_t smem = kd.stage * sizeof(uint2);
   uint32_t refill = s->tune.ray_refill_min, lanes = COUNT ? 1u : ray_form(s, w * h, true);
+  const bool long_tree = long_leaves(s);
   auto k = lanes == 2u    ? k_primary_lanes<MODE, 2>
            : lanes == 4u  ? k_primary_lanes<MODE, 4>
            : lanes == 8u  ? k_primary_lanes<MODE, 8>
            : lanes == kWholeWarp ? k_primary_lanes<MODE, 32>
            : lanes == 32u ? k_primary_warp<MODE>
-           : refill >= 32u ? k_primary_tiles<MODE, COUNT>
-                           : k_primary<MODE, COUNT>;
+           : refill >= 32u ? (long_tree || COUNT ? k_primary_tiles<MODE, COUNT, kWholeDescent>
+                                                 : k_primary_tiles<MODE, COUNT, kTileDescent>)
+           : long_tree     ? k_primary<MODE, COUNT, kRefillLongDescent>
+                           : k_primary<MODE, COUNT, kRefillDescent>;
   RE_CUDA(cudaMemsetAsync(s->d_counters, 0, RE_SCENE_RESET_BYTES, st));
   RE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // no more blocks than warps with work: few tiles spread over the SMs
@@ -800,12 +808,15 @@ re_status launch_rays(re_scene* s, const float4* rays, uint32_t n, re_hit* out, 
   uint32_t refill = s->tune.ray_refill_min;
   // refill thresholds of 4 to 16 idle lanes measured within 2 %; 8
   const uint32_t lanes = ray_form(s, n, false);
+  const bool long_tree = long_leaves(s);
   if (lanes == 32u) refill = std::min(refill, 8u);
   auto k = lanes == kWholeWarp ? k_rays_lanes<MODE, ANYHIT, 32>
            : lanes == 8u       ? k_rays_lanes<MODE, ANYHIT, 8>
            : lanes == 32u      ? k_rays_warp<MODE, ANYHIT>
-           : refill >= 32u     ? k_rays_chunks<MODE, ANYHIT>
-                               : k_rays<MODE, ANYHIT>;
+           : refill >= 32u     ? (long_tree || !ANYHIT ? k_rays_chunks<MODE, ANYHIT, kWholeDescent>
+                                                      : k_rays_chunks<MODE, ANYHIT, kTileDescent>)
+           : long_tree         ? k_rays<MODE, ANYHIT, kRefillLongDescent>
+                               : k_rays<MODE, ANYHIT, kRefillDescent>;
   RE_CUDA(cudaMemsetAsync(s->d_counters, 0, RE_SCENE_RESET_BYTES, st));
   RE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const uint32_t per_warp = lanes == kWholeWarp ? 1u : 32u / (lanes < 32u ? lanes : 1u);
@@ -1016,6 +1027,18 @@ re_status ao_prepare(re_scene* s, const re_camera* cam, uint32_t w, uint32_t h,
 }
 
 template <bool COUNT>
+auto ao_primary_kernel(const re_scene* s) {
+  return long_leaves(s) ? k_ao_primary<COUNT, kWholeDescent> : k_ao_primary<COUNT, kTileDescent>;
+}
+
+template <bool COUNT>
+auto ao_secondary_kernel(const re_scene* s) {
+  return long_leaves(s)              ? k_ao_secondary<COUNT, kAoLongDescent>
+         : s->tune.refill_min >= 32u ? k_ao_secondary<COUNT, kAoNoRefillDescent>
+                                     : k_ao_secondary<COUNT, kAoDescent>;
+}
+
+template <bool COUNT>
 re_status ao_primary(re_scene* s, const CamDev& cd, const AoDev& ao, uint32_t w, uint32_t h,
                      re_hit* d_primary, uint32_t* d_mask, unsigned long long* totals,
                      cudaStream_t st) {
@@ -1024,7 +1047,7 @@ re_status ao_primary(re_scene* s, const CamDev& cd, const AoDev& ao, uint32_t w,
   if (COUNT) kd.entry = nullptr;
   size_t smem = kd.stage * sizeof(uint2);
   RE_CUDA(cudaMemsetAsync(s->d_counters, 0, RE_SCENE_RESET_BYTES, st));
-  auto k = k_ao_primary<COUNT>;
+  auto k = ao_primary_kernel<COUNT>(s);
   RE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k<<<grid_for(k, smem), 256, smem, st>>>(kd, cd, ao, w, h, d_primary, d_mask,
                                           ao_queue(s, s->d_queue, s->queue_stride), s->d_counters,
@@ -1040,7 +1063,7 @@ re_status ao_secondary(re_scene* s, uint32_t* d_mask, unsigned long long* totals
   AoDev ao{};
   ao.ao_length = s->ao_length;
   size_t smem = kd.stage * sizeof(uint2);
-  auto k = k_ao_secondary<COUNT>;
+  auto k = ao_secondary_kernel<COUNT>(s);
   RE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k<<<grid_for(k, smem), 256, smem, st>>>(kd, ao, ao_queue(s, s->d_queue, s->queue_stride),
                                           d_mask, s->d_counters, totals);
@@ -1170,14 +1193,14 @@ RE_API re_status re_render_ao_noalloc(re_scene* s, const re_camera* cam, uint32_
   // the array keeps the previous call's contents: the cursors must restart at zero
   RE_CUDA(cudaMemsetAsync(counters, 0, RE_SCENE_RESET_BYTES, st));
   {
-    auto k = re::k_ao_primary<false>;
+    auto k = re::ao_primary_kernel<false>(s);
     RE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k<<<re::grid_for(k, smem), 256, smem, st>>>(kd, cd, ao, w, h, d_primary, d_mask,
                                                 re::ao_queue(s, queue, w * h), counters, nullptr);
     RE_CHECK_LAUNCH("re_render_ao_noalloc: primary launch");
   }
   {
-    auto k = re::k_ao_secondary<false>;
+    auto k = re::ao_secondary_kernel<false>(s);
     RE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k<<<re::grid_for(k, smem), 256, smem, st>>>(kd, ao, re::ao_queue(s, queue, w * h), d_mask,
                                                 counters, nullptr);

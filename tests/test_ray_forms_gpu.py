@@ -112,3 +112,25 @@ def test_plain_walk(cuda, long_leaves):
                 for f in (0, rb.TRACE_ANY_HIT)]]
         for a, b in zip(want[0] + want[1], got[0] + got[1]):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("refill", [1, 8, 32])
+@pytest.mark.parametrize("long_leaves", [False, True])
+def test_ao_frames(cuda, long_leaves, refill):
+    """The AO frame's passes bound their descents by the tree and the refill
+    threshold: hits, masks and work counts as the oracle's."""
+    cfg = rb.configs.SoupConfig(num_tris=6000)
+    packed, light = cfg.packed(), rb.unit((0.3, 1.0, 0.2))
+    w, h = 131, 67
+    cam = rb.build_camera((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), (60.0, 50.0))
+    with _scene(long_leaves) as sc:
+        st, kd = _kd(sc)
+        sc.set_tuning(sc.tuning()["stage_nodes"], 0, refill)
+        hits, mask, nsec = sc.render_ao(cam, w, h, light, 0.3, 1e-4, 5)
+        rh, rm, rn = po.frame_ao(kd, packed, cam, w, h, light, 0.3, 1e-4, 5)
+        assert np.array_equal(hits.cpu().numpy(), rh.view(np.int32).reshape(-1, 4))
+        assert np.array_equal(mask.cpu().numpy().view(np.uint32), rm)
+        assert int(nsec.item()) == rn > 0
+        want = sc.render_ao_counts(cam, w, h, rb.ao_params(light, 0.3, 1e-4, 5))
+        sc.set_tuning(0, 2, 8)
+        assert sc.render_ao_counts(cam, w, h, rb.ao_params(light, 0.3, 1e-4, 5)) == want
