@@ -10,6 +10,7 @@
 // 16 32-bit counters per scene (64 bytes)
 #define RE_SCENE_TRUNC_SLOT 8
 #define RE_SCENE_RESET_BYTES (4 * (RE_SCENE_TRUNC_SLOT + 1))
+#define RE_SCENE_ORDER_SLOT 10
 
 struct re_scene {
   int device = 0;

@@ -134,3 +134,42 @@ def test_ao_frames(cuda, long_leaves, refill):
         want = sc.render_ao_counts(cam, w, h, rb.ao_params(light, 0.3, 1e-4, 5))
         sc.set_tuning(0, 2, 8)
         assert sc.render_ao_counts(cam, w, h, rb.ao_params(light, 0.3, 1e-4, 5)) == want
+
+
+def _camera_rows(w, h):
+    """A camera's rays in row order, from (0, 0, 3) to the origin, 60 degrees
+    wide."""
+    t = np.tan(np.radians(30.0))
+    x, y = np.meshgrid(np.linspace(-t, t, w), np.linspace(t, -t, h) * h / w)
+    d = np.stack([x, y, -np.ones_like(x)], -1).reshape(-1, 3)
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = np.zeros((w * h, 8), np.float32)
+    rays[:, 2], rays[:, 3], rays[:, 4:7] = 3.0, 1e20, d
+    return rays
+
+
+# 1,500,000 rays: from here on their order decides between the forms
+@pytest.mark.parametrize("n", [1499999, 1500000, 1500013])
+@pytest.mark.parametrize("order", ["rows", "shuffled", "rows, then shuffled", "not finite"])
+def test_many_caller_rays(cuda, order, n):
+    rays = torch.from_numpy(_camera_rows(1600, 938)[:n]).cuda()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    mixed = rays[torch.randperm(n, generator=g, device="cuda")]
+    if order == "shuffled":
+        rays = mixed
+    elif order != "rows":
+        rays = torch.cat([rays[: n // 2], mixed[n // 2:]])
+    if order == "not finite":
+        rays[::33, 4] = float("nan")
+        rays[5::33, 0] = float("inf")
+    rays = rays.contiguous()
+    with _scene(True, max_leaf_visits=3) as sc:
+        t = sc.tuning()
+        for flags in (0, 1, rb.TRACE_ANY_HIT, 1 | rb.TRACE_ANY_HIT):
+            got, cut = sc.trace_rays(rays, flags), sc.truncated()
+            sc.set_tuning(t["stage_nodes"], t["queue_kind_major"], t["refill_min"],
+                          rb.RAY_NO_REFILL)
+            assert torch.equal(got, sc.trace_rays(rays, flags)), flags
+            assert sc.truncated() == cut
+            sc.set_tuning(t["stage_nodes"], t["queue_kind_major"], t["refill_min"], 32)
+        assert (got[:, 0] >= 0).sum() > n // 50
