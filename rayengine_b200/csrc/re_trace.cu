@@ -798,7 +798,10 @@ namespace {
 // (8 lanes); 256x256 69, 172, 140, 118 -> 50, 109, 93, 97 (4 lanes).  Random
 // rays: 1000 121, 180, 141, 110 -> 38, 65, 56, 57 (32 lanes), 20,000 150,
 // 266, 190, 145 -> 71, 125, 92, 105 (8 lanes); at 60,000 four lanes are level
-// with the shared tests.
+// with the shared tests.  Caller rays in trees of short leaves, which have no
+// shared tests to go to: 8 and 4 lanes while all rays are resident at once
+// (31,866 random rays in the heightfield plain 159, 8 lanes 156, 4 lanes 125;
+// 39,816 167, 176, 137; 55,913 171, -, 143; past them plain again).
 //   More rays in a tree of long leaves share their tests (the soups hold 5.3
 // to 5.6 references per leaf; 2048x2048 481, 882, 673 -> 450, 750, 635 us,
 // 300,007 random rays 349, 509, 319 -> 235, 299, 204); where leaves are short
@@ -813,6 +816,10 @@ uint32_t ray_form(const re_scene* s, uint32_t n, bool frame) {
   const bool by_size = s->tune.ray_refill_min == 32u && (!frame || s->tune.ray_lanes <= 1u);
   if (!by_size) return frame ? s->tune.ray_lanes : 1u;
   if (n <= 4096u) return kWholeWarp;
+  if (!frame && !long_leaves(s)) {
+    const uint32_t warps = 48u * (uint32_t)sm_count();  // resident
+    return n <= 4u * warps ? 8u : n <= 8u * warps ? 4u : 1u;
+  }
   if (n <= 40960u) return 8u;
   if (frame && n <= 81920u) return 4u;
   return long_leaves(s) ? 32u : 1u;
@@ -866,6 +873,7 @@ re_status launch_rays(re_scene* s, const float4* rays, uint32_t n, re_hit* out, 
   if (lanes == 32u) refill = std::min(refill, 8u);
   auto k = lanes == kWholeWarp ? k_rays_lanes<MODE, ANYHIT, 32>
            : lanes == 8u       ? k_rays_lanes<MODE, ANYHIT, 8>
+           : lanes == 4u       ? k_rays_lanes<MODE, ANYHIT, 4>
            : lanes == 32u      ? k_rays_warp<MODE, ANYHIT>
            : refill >= 32u     ? (long_tree || !ANYHIT ? k_rays_chunks<MODE, ANYHIT, kWholeDescent>
                                                       : k_rays_chunks<MODE, ANYHIT, kTileDescent>)

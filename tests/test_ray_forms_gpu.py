@@ -173,3 +173,18 @@ def test_many_caller_rays(cuda, order, n):
             assert sc.truncated() == cut
             sc.set_tuning(t["stage_nodes"], t["queue_kind_major"], t["refill_min"], 32)
         assert (got[:, 0] >= 0).sum() > n // 50
+
+
+@pytest.mark.parametrize("flags", [0, 1, rb.TRACE_ANY_HIT])
+def test_caller_rays_fill_the_gpu(cuda, flags):
+    """At and past the numbers of rays that are resident at once with 8 and
+    with 4 lanes each."""
+    warps = 48 * torch.cuda.get_device_properties(0).multi_processor_count
+    with _scene(False) as sc:
+        dr = torch.from_numpy(_rays(8 * warps + 1)).cuda()
+        t = sc.tuning()
+        sc.set_tuning(t["stage_nodes"], t["queue_kind_major"], t["refill_min"], rb.RAY_NO_REFILL)
+        want = sc.trace_rays(dr, flags)
+        sc.set_tuning(t["stage_nodes"], t["queue_kind_major"], t["refill_min"], 32)
+        for n in (4 * warps, 4 * warps + 1, 8 * warps - 3, 8 * warps, 8 * warps + 1):
+            assert torch.equal(sc.trace_rays(dr[:n].contiguous(), flags), want[:n]), n
