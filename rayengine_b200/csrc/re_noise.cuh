@@ -189,7 +189,7 @@ __device__ __forceinline__ float terrain_density(const PT& P, V3 p,
 // The lattice cell comes from one addition rounded down to a multiple of 1:
 // 1.5 * 2^23 + floor(x), its low byte the masked index, where floor and a
 // conversion run on the quarter-rate unit.  That holds for |x| < 2^22;
-// beyond, field_far() evaluates perlin() on the same table.
+// beyond, field_far() finds the cells as perlin() does.
 //
 // Measured on B200 (a march of 8-octave evaluations, no other work): 33.3 G
 // evaluations/s against 26.3 of perlin() on 16 copies.  Per octave 99
@@ -348,16 +348,35 @@ __device__ __forceinline__ f32x2 quintic2(f32x2 t) {
   return mul2(mul2(mul2(t, t), t), in);
 }
 
-// Twice the noise of two octaves; every coordinate below 2^22.
-template <class FT>
+// The cells (lattice indices, of which the low bytes count) and the fractions
+// of two coordinates.  FAR: as perlin() takes them, at any magnitude; otherwise
+// below 2^22, from one addition rounded down.
+template <bool FAR>
+__device__ __forceinline__ f32x2 lattice2(f32x2 x, uint32_t& lo, uint32_t& hi) {
+  if (FAR) {
+    float x0, x1;
+    unpack2(x, x0, x1);
+    const float f0 = floorf(x0), f1 = floorf(x1);
+    lo = (uint32_t)(int)f0;
+    hi = (uint32_t)(int)f1;
+    return sub2(x, pack2(f0, f1));
+  }
+  const f32x2 kInt = pack2(12582912.0f, 12582912.0f), i = add2_down(x, kInt);
+  lo = (uint32_t)i;
+  hi = (uint32_t)(i >> 32);
+  return sub2(x, sub2(i, kInt));
+}
+
+// Twice the noise of two octaves; unless FAR every coordinate below 2^22.
+template <bool FAR = false, class FT>
 __device__ __forceinline__ f32x2 perlin2(const FT& R, f32x2 x, f32x2 y, f32x2 z) {
-  const f32x2 kInt = pack2(12582912.0f, 12582912.0f), kOne = pack2(1.0f, 1.0f);
-  const f32x2 ix = add2_down(x, kInt), iy = add2_down(y, kInt), iz = add2_down(z, kInt);
-  const f32x2 tx = sub2(x, sub2(ix, kInt)), ty = sub2(y, sub2(iy, kInt)),
-              tz = sub2(z, sub2(iz, kInt));
+  const f32x2 kOne = pack2(1.0f, 1.0f);
+  uint32_t xl, xh, yl, yh, zl, zh;
+  const f32x2 tx = lattice2<FAR>(x, xl, xh), ty = lattice2<FAR>(y, yl, yh),
+              tz = lattice2<FAR>(z, zl, zh);
   uint32_t lo[8], hi[8];
-  cell_words(R, (uint32_t)ix, (uint32_t)iy, (uint32_t)iz, lo);
-  cell_words(R, (uint32_t)(ix >> 32), (uint32_t)(iy >> 32), (uint32_t)(iz >> 32), hi);
+  cell_words(R, xl, yl, zl, lo);
+  cell_words(R, xh, yh, zh, hi);
   const f32x2 x1 = sub2(tx, kOne), y1 = sub2(ty, kOne), z1 = sub2(tz, kOne);
   const f32x2 u = quintic2(tx), v = quintic2(ty), w = quintic2(tz);
   const f32x2 a = corner2(lo[0], hi[0], tx, ty, tz), b = corner2(lo[1], hi[1], x1, ty, tz);
@@ -388,53 +407,85 @@ struct PermRows {
   __device__ __forceinline__ uint32_t grad(uint32_t j) const { return perm_word(idx(j)); }
 };
 
-// fbm() at any coordinates (infinities and NaN among them); out of line, so
-// that the callers' registers are those of the near form.
-template <uint32_t STRIDE>
+// The octaves' sum at any coordinates (infinities and NaN among them); out of
+// line, so that the callers' registers are those of the near form.  In pairs
+// on the rows; an octave at a time on FieldWords, for the registers of the
+// batched renderer (which takes other tables for such fields).  Measured on
+// B200, 480x270 frames whose rays are all or mostly past the near form's
+// range, an octave at a time | in pairs: 8 octaves at scale 1000 674 | 408 us
+// (one octave at a time on 16 copies, four times the warps: 366), 20 octaves
+// 1892 | 1116 (1157); 1920x1080 at scale 1000: 2176 (2644).
+template <uint32_t STRIDE, uint32_t G>
 static __device__ __noinline__ float field_far(uint32_t base, float x, float y, float z,
                                                uint32_t octaves) {
-  PermRows<STRIDE> P{base};
-  float sum = 0.0f, amp = 1.0f;
+  float sum = 0.0f, a = 1.0f;
+  if (STRIDE != kRowBytes) {
+    PermRows<STRIDE> P{base};
 #pragma unroll 1
-  for (uint32_t i = 0; i < octaves; ++i) {
-    sum = __fmaf_rn(amp, perlin(P, x, y, z), sum);
-    x *= 2.0f;
-    y *= 2.0f;
-    z *= 2.0f;
-    amp *= 0.5f;
+    for (uint32_t i = 0; i < octaves; ++i) {
+      sum = __fmaf_rn(a, perlin(P, x, y, z), sum);
+      x *= 2.0f;
+      y *= 2.0f;
+      z *= 2.0f;
+      a *= 0.5f;
+    }
+    return sum;
+  }
+  const FieldTable<STRIDE, G> R{base};
+  const f32x2 kFour = pack2(4.0f, 4.0f);
+  f32x2 X = pack2(x, 2.0f * x), Y = pack2(y, 2.0f * y), Z = pack2(z, 2.0f * z);
+#pragma unroll 1
+  for (uint32_t i = 0; i < octaves; i += 2) {
+    float r0, r1;
+    unpack2(perlin2<true>(R, X, Y, Z), r0, r1);
+    sum = __fmaf_rn(0.5f * a, r0, sum);
+    // the octave past an odd last one may be infinite or NaN
+    if (i + 1u < octaves) sum = __fmaf_rn(0.25f * a, r1, sum);
+    a *= 0.25f;
+    X = mul2(X, kFour);
+    Y = mul2(Y, kFour);
+    Z = mul2(Z, kFour);
   }
   return sum;
 }
 
-// terrain_density() on the rows.  The near form evaluates octaves in pairs,
+// The octaves' sum on a field table.  The near form evaluates octaves in pairs,
 // an odd last one with an octave past it at amplitude zero, so the largest
 // coordinate it meets is below 2^octaves times the first one's.
 // UNROLL: pairs in the code at once.
+template <int UNROLL, uint32_t STRIDE, uint32_t G>
+__device__ __forceinline__ float field_near(const FieldTable<STRIDE, G>& R, float x, float y,
+                                            float z, uint32_t octaves) {
+  const f32x2 kFour = pack2(4.0f, 4.0f);
+  f32x2 X = pack2(x, 2.0f * x), Y = pack2(y, 2.0f * y), Z = pack2(z, 2.0f * z);
+  float sum = 0.0f, a = 0.5f;
+#pragma unroll UNROLL
+  for (uint32_t i = 0; i < octaves; i += 2) {
+    float r0, r1;
+    unpack2(perlin2(R, X, Y, Z), r0, r1);
+    sum = __fmaf_rn(a, r0, sum);
+    sum = __fmaf_rn(i + 1u < octaves ? 0.5f * a : 0.0f, r1, sum);
+    a *= 0.25f;
+    X = mul2(X, kFour);
+    Y = mul2(Y, kFour);
+    Z = mul2(Z, kFour);
+  }
+  return sum;
+}
+
+// Whether the near form holds: coordinates below 2^(22 - octaves), octaves <= 32.
+__device__ __forceinline__ bool is_near(float x, float y, float z, uint32_t octaves) {
+  const float lim = __uint_as_float((127u + 22u - octaves) << 23);
+  return fabsf(x) < lim && fabsf(y) < lim && fabsf(z) < lim;
+}
+
+// terrain_density() on a field table.
 template <int UNROLL = 4, uint32_t STRIDE, uint32_t G>
 __device__ __forceinline__ float terrain_density(const FieldTable<STRIDE, G>& R, V3 p,
                                                  uint32_t octaves, float scale, float amp) {
   const float x = scale * p.x, y = scale * p.y, z = scale * p.z;
-  // 2^(22 - octaves), octaves <= 32
-  const float lim = __uint_as_float((127u + 22u - octaves) << 23);
-  float sum = 0.0f;
-  if (fabsf(x) < lim && fabsf(y) < lim && fabsf(z) < lim) {
-    const f32x2 kFour = pack2(4.0f, 4.0f);
-    f32x2 X = pack2(x, 2.0f * x), Y = pack2(y, 2.0f * y), Z = pack2(z, 2.0f * z);
-    float a = 0.5f;
-#pragma unroll UNROLL
-    for (uint32_t i = 0; i < octaves; i += 2) {
-      float r0, r1;
-      unpack2(perlin2(R, X, Y, Z), r0, r1);
-      sum = __fmaf_rn(a, r0, sum);
-      sum = __fmaf_rn(i + 1u < octaves ? 0.5f * a : 0.0f, r1, sum);
-      a *= 0.25f;
-      X = mul2(X, kFour);
-      Y = mul2(Y, kFour);
-      Z = mul2(Z, kFour);
-    }
-  } else {
-    sum = field_far<STRIDE>(R.base, x, y, z, octaves);
-  }
+  const float sum = is_near(x, y, z, octaves) ? field_near<UNROLL>(R, x, y, z, octaves)
+                                              : field_far<STRIDE, G>(R.base, x, y, z, octaves);
   return __fmaf_rn(-amp, sum, p.y);
 }
 
@@ -462,11 +513,10 @@ __device__ __forceinline__ float terrain_density_shared(const FieldTable<STRIDE,
                                                         float scale, float amp) {
   const uint32_t lane = threadIdx.x & 31u;
   const float x = scale * p.x, y = scale * p.y, z = scale * p.z;
-  const float lim = __uint_as_float((127u + 22u - octaves) << 23);
   const bool mine = (live >> lane) & 1u;
   float sum = 0.0f;
-  if (__any_sync(0xFFFFFFFFu, mine && !(fabsf(x) < lim && fabsf(y) < lim && fabsf(z) < lim))) {
-    if (mine) sum = field_far<STRIDE>(R.base, x, y, z, octaves);
+  if (__any_sync(0xFFFFFFFFu, mine && !is_near(x, y, z, octaves))) {
+    if (mine) sum = field_far<STRIDE, G>(R.base, x, y, z, octaves);
     return __fmaf_rn(-amp, sum, p.y);
   }
   const uint32_t src = nth_set(live, lane / L);  // past the last point: lane 31's, unused
@@ -515,7 +565,13 @@ __device__ __forceinline__ float warp_density(const FieldTable<STRIDE, G>& R, V3
   const uint32_t n = __popc(mask);
   if (n <= 8u) return terrain_density_shared<4>(R, p, mask, octaves, scale, amp);
   if (SHARED2 && n <= 16u) return terrain_density_shared<2>(R, p, mask, octaves, scale, amp);
-  return live ? terrain_density<UNROLL>(R, p, octaves, scale, amp) : 0.0f;
+  if (STRIDE != kRowBytes) return live ? terrain_density<UNROLL>(R, p, octaves, scale, amp) : 0.0f;
+  // one far lane takes the others with it: the far form's result is the near
+  // one's, and the warp then runs one of the two
+  const float x = scale * p.x, y = scale * p.y, z = scale * p.z;
+  if (!__all_sync(0xFFFFFFFFu, !live || is_near(x, y, z, octaves)))
+    return live ? __fmaf_rn(-amp, field_far<STRIDE, G>(R.base, x, y, z, octaves), p.y) : 0.0f;
+  return live ? __fmaf_rn(-amp, field_near<UNROLL>(R, x, y, z, octaves), p.y) : 0.0f;
 }
 
 // Gradient of perlin() at (x, y, z), from the same lattice, fade and blend
@@ -613,14 +669,13 @@ __device__ __forceinline__ f32x2 minus2(f32x2 a, f32x2 b, float one) {
 template <class FT>
 __device__ __forceinline__ void perlin_grad2(const FT& R, f32x2 x, f32x2 y, f32x2 z, float one,
                                              f32x2& rx, f32x2& ry, f32x2& rz) {
-  const f32x2 kInt = pack2(12582912.0f, 12582912.0f), kOne = pack2(1.0f, 1.0f);
-  const f32x2 k30 = pack2(30.0f, 30.0f);
-  const f32x2 ix = add2_down(x, kInt), iy = add2_down(y, kInt), iz = add2_down(z, kInt);
-  const f32x2 tx = sub2(x, sub2(ix, kInt)), ty = sub2(y, sub2(iy, kInt)),
-              tz = sub2(z, sub2(iz, kInt));
+  const f32x2 kOne = pack2(1.0f, 1.0f), k30 = pack2(30.0f, 30.0f);
+  uint32_t xl, xh, yl, yh, zl, zh;
+  const f32x2 tx = lattice2<false>(x, xl, xh), ty = lattice2<false>(y, yl, yh),
+              tz = lattice2<false>(z, zl, zh);
   uint32_t lo[8], hi[8];
-  cell_words(R, (uint32_t)ix, (uint32_t)iy, (uint32_t)iz, lo);
-  cell_words(R, (uint32_t)(ix >> 32), (uint32_t)(iy >> 32), (uint32_t)(iz >> 32), hi);
+  cell_words(R, xl, yl, zl, lo);
+  cell_words(R, xh, yh, zh, hi);
   const f32x2 x1 = sub2(tx, kOne), y1 = sub2(ty, kOne), z1 = sub2(tz, kOne);
   const f32x2 u = quintic2(tx), v = quintic2(ty), w = quintic2(tz);
   const f32x2 uv = mul2(u, v), uw = mul2(u, w), vw = mul2(v, w), uvw = mul2(uv, w);

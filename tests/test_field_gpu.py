@@ -62,3 +62,24 @@ def test_frames_of_few_rays(cuda, w, h, octaves):
     assert np.array_equal(u[hit, 3:6], ref["normal"][hit].view(np.uint32))
     want = po.sdf_frame(po.perm(cfg.seed), cfg.camera(), w, h, cfg.params(), shade)
     assert np.array_equal(img.cpu().numpy().view(np.uint32), want)
+
+
+# frames with some rays, most and all of them past the near form's range, odd
+# and even octave counts, coordinates past 2^23 and up to the largest integers
+# (beyond those the oracle's conversion is undefined in C)
+@pytest.mark.parametrize("octaves,scale", [(16, 1.0), (17, 0.25), (32, 0.004), (8, 300.0),
+                                           (3, 1e6), (8, 70000.0)])
+def test_frames_past_the_near_range(cuda, octaves, scale):
+    w, h = 67, 41
+    cfg = rb.configs.TerrainConfig(width=w, height=h, octaves=octaves, scale=scale)
+    got = rb.sphere_trace(cfg.params(), cfg.camera(), w, h).cpu().numpy().view(np.uint32)
+    ref = po.sdf_image(po.perm(cfg.seed), cfg.camera(), w, h, octaves=octaves, scale=scale)
+    u = got.reshape(-1, 8)
+    assert np.array_equal(u[:, 6], ref["steps"])
+    assert np.array_equal(u[:, 7], ref["status"])
+    hit = ref["status"] == 1
+    assert np.array_equal(u[hit, 0:3], ref["pos"][hit].view(np.uint32))
+    normal, want = u[hit, 3:6].view(np.float32), ref["normal"][hit]
+    nan = np.isnan(want)  # whose payload is not compared
+    assert np.array_equal(np.isnan(normal), nan)
+    assert np.array_equal(normal[~nan].view(np.uint32), want[~nan].view(np.uint32))
