@@ -717,6 +717,7 @@ struct re_batch {
   uint64_t total_pixels = 0;
   std::vector<uint64_t> offsets;
   uint64_t cap[2] = {0, 0};  // pixels of mesh / terrain scenes (queue capacity)
+  uint64_t paired_pixels = 0;  // of terrain scenes that the paired field suits
   re::batch::SceneDev* d_scenes = nullptr;
   uint8_t* d_perms = nullptr;
   float4* d_queue = nullptr;
@@ -800,6 +801,16 @@ uint32_t blocks_per_sm(size_t smem, uint32_t block_threads) {
 constexpr uint32_t kFieldTablesMax = 12, kWordTablesMax = 16;
 constexpr size_t kMaxSmem = 232448;
 
+// Fields of at least four octaves whose near form (is_near) holds over the
+// scene about the camera: four times its distance from the origin and a
+// sixteenth of the march's range.
+bool paired_suits(const re_sdf_params& f, const CamDev& c) {
+  const float away = std::max(std::fabs(c.campos.x),
+                              std::max(std::fabs(c.campos.y), std::fabs(c.campos.z)));
+  return f.octaves >= 4u && std::fabs(f.scale) * (4.0f * away + f.tmax / 16.0f) <
+                                std::ldexp(1.0f, 22 - (int)f.octaves);
+}
+
 int table_of(const re_batch* b, uint32_t stage_total, uint32_t block_threads) {
   const size_t seeds = b->perms.size() / 512;
   if (seeds == 0) return kNoTables;
@@ -811,6 +822,7 @@ int table_of(const re_batch* b, uint32_t stage_total, uint32_t block_threads) {
       blocks_per_sm(smem_bytes(b, kFieldTables, stage_total, block_threads), block_threads);
   const uint32_t word =
       blocks_per_sm(smem_bytes(b, kWordTables, stage_total, block_threads), block_threads);
+  if (2u * b->paired_pixels < b->cap[kTerrain]) return kWordTables;
   const bool terrain = b->cap[kTerrain] >= b->cap[kMesh];
   return (terrain ? 2u : 1u) * field >= word ? kFieldTables : kWordTables;
 }
@@ -980,6 +992,7 @@ RE_API re_status re_batch_create(const re_batch_scene* scenes, uint32_t n, const
       // |fBm| <= 2 (2 - 2^(1 - octaves)) and the density is positive above
       d.ceiling = 2.0f * std::fabs(f.amplitude) * (2.0f - std::ldexp(1.0f, 1 - (int)f.octaves)) + 1e-3f;
       b->cap[1] += (uint64_t)s.width * s.height;
+      if (re::paired_suits(f, d.cam)) b->paired_pixels += (uint64_t)s.width * s.height;
     } else {
       delete b;
       return re::fail(RE_ERR_INVALID_ARG, "re_batch_create: scene %u: unknown kind", i);

@@ -76,12 +76,13 @@ struct SdfDev {
 // B200, 64x36 213 -> 131 us, 480x270 483 -> 392, 1366x768 1512 -> 1435.
 constexpr uint32_t kSdfRefill = 4;
 
-__global__ void __launch_bounds__(kRowsThreads) k_sdf(PermTable perm, SdfDev sp, CamDev cam,
-                                                      uint32_t w, uint32_t h, RowsSpread spread,
-                                                      float4* __restrict__ out,
-                                                      uint32_t* __restrict__ cursor) {
+template <class FORM>
+__global__ void __launch_bounds__(FORM::kThreads) k_sdf(PermTable perm, SdfDev sp, CamDev cam,
+                                                        uint32_t w, uint32_t h, RowsSpread spread,
+                                                        float4* __restrict__ out,
+                                                        uint32_t* __restrict__ cursor) {
   extern __shared__ uint32_t rows_smem[];
-  const FieldRows P = load_rows(perm, rows_smem);
+  const auto P = FORM::load(perm, rows_smem);
   if ((threadIdx.x >> 5) >= spread.warps) return;
   uint32_t lane = threadIdx.x & 31u;
   uint32_t tiles_x = (w + 7) / 8;
@@ -244,11 +245,14 @@ RE_API re_status re_sdf_trace(const re_sdf_params* p, const re_camera* cam, uint
   const re::LaunchWords cursor = re::launch_words(st);
   if (!cursor.words) return re::cuda_fail(cursor.error, "re_sdf_trace: claim cursor");
   RE_CUDA(cudaMemsetAsync(cursor.words, 0, 4, st));
-  RE_CUDA(cudaFuncSetAttribute(re::k_sdf, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)re::kRowsSmemBytes));
-  re::k_sdf<<<re::sm_count(), re::kRowsThreads, re::kRowsSmemBytes, st>>>(
-      t, sp, cd, w, h, re::rows_spread((uint64_t)w * h, (uint32_t)re::sm_count()),
-      reinterpret_cast<float4*>(d_out), cursor.words);
+  const re_status rs = re::launch_field(
+      re::field_on_rows(p->octaves, (uint64_t)w * h), re::k_sdf<re::RowsForm>,
+      re::k_sdf<re::CopyForm>, (uint64_t)w * h, [](uint32_t) { return 0u; },
+      [&](auto k, int grid, uint32_t threads, uint32_t smem, re::RowsSpread spread) {
+        k<<<grid, threads, smem, st>>>(t, sp, cd, w, h, spread, reinterpret_cast<float4*>(d_out),
+                                       cursor.words);
+      });
+  if (rs != RE_OK) return rs;
   RE_CHECK_LAUNCH("re_sdf_trace: launch");
   return RE_OK;
 }

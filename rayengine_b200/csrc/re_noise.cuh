@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "re_common.hpp"
 #include "re_math.cuh"
 
 namespace re {
@@ -572,6 +573,59 @@ __device__ __forceinline__ float warp_density(const FieldTable<STRIDE, G>& R, V3
   if (!__all_sync(0xFFFFFFFFu, !live || is_near(x, y, z, octaves)))
     return live ? __fmaf_rn(-amp, field_far<STRIDE, G>(R.base, x, y, z, octaves), p.y) : 0.0f;
   return live ? __fmaf_rn(-amp, field_near<UNROLL>(R, x, y, z, octaves), p.y) : 0.0f;
+}
+
+template <class PT>
+__device__ __forceinline__ float warp_density(const PT& P, V3 p, bool live, uint32_t octaves,
+                                              float scale, float amp) {
+  return live ? terrain_density(P, p, octaves, scale, amp) : 0.0f;
+}
+
+// How a kernel holds the field: pairs of octaves on the rows, or an octave at a
+// time on 16 copies of the permutation, with up to twice the warps.
+struct RowsForm {
+  static constexpr uint32_t kThreads = kRowsThreads, kBytes = kRowsSmemBytes;
+  static __device__ __forceinline__ FieldRows load(const PermTable& t, uint32_t* smem) {
+    return load_rows(t, smem);
+  }
+};
+struct CopyForm {
+  static constexpr uint32_t kThreads = 256, kBytes = kPermSmemBytes;
+  static __device__ __forceinline__ Perm load(const PermTable& t, uint32_t* smem) {
+    load_perm(t, smem);
+    return perm_view(smem);
+  }
+};
+
+// Whether the marches' kernels take the rows: a single octave is half a pair,
+// and two are too little work to need few warps until the frame is large.
+// Measured on B200, exact terrain, copies | rows: one octave 480x270 340 | 513
+// us, 1920x1080 1245 | 1682; two octaves 428 | 475, 960x540 762 | 683; three 565
+// | 512.  STENCIL: the neural tracer's exact phase with a stencil for the
+// normal, which mixes a warp's rays: two octaves 492 | 578, 1920x1080 1589 |
+// 1686; three 64x36 184 | 169, 160x90 472 | 491, 1920x1080 1915 | 2011.
+template <bool STENCIL = false>
+inline bool field_on_rows(uint32_t octaves, uint64_t rays) {
+  if (STENCIL) return octaves > 3u || (octaves == 3u && rays < (1u << 13));
+  return octaves > 2u || (octaves == 2u && rays >= (1u << 18));
+}
+
+// Launches the kernel's form for a frame of `rays` rays: call(kernel, grid,
+// threads, shared bytes, spread).  extra(warps): shared bytes past the table.
+template <class K, class E, class F>
+re_status launch_field(bool rows, K rows_kernel, K copy_kernel, uint64_t rays, E extra, F call) {
+  const uint32_t threads = rows ? RowsForm::kThreads : CopyForm::kThreads;
+  const uint32_t smem = (rows ? RowsForm::kBytes : CopyForm::kBytes) + extra(threads / 32u);
+  const K kernel = rows ? rows_kernel : copy_kernel;
+  RE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 1;
+  if (!rows && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)threads,
+                                                              smem) != cudaSuccess ||
+                per_sm < 1))
+    per_sm = 1;
+  call(kernel, per_sm * sm_count(), threads, smem,
+       rows ? rows_spread(rays, (uint32_t)sm_count()) : RowsSpread{32u, CopyForm::kThreads / 32u});
+  return RE_OK;
 }
 
 // Gradient of perlin() at (x, y, z), from the same lattice, fade and blend

@@ -52,13 +52,20 @@ __device__ __forceinline__ uint32_t mix32(uint32_t a, uint32_t b, uint32_t c) {
 __device__ __forceinline__ float u01(uint32_t h) { return (float)(h >> 8) * 5.9604644775390625e-08f; }
 
 // ------------------------------------------------------ data generation
-__global__ void __launch_bounds__(kRowsThreads) k_nsdf_data(PermTable perm, FieldDev f, CamDev cam,
+// 768 threads: with 640 a second round of rays begins at 94,720 points (130,000
+// points 750 -> 647 us, one octave at a time on 16 copies 693); 1,000 points
+// 256 -> 131 us with a warp to each SM.
+constexpr uint32_t kDataThreads = 768;
+
+__global__ void __launch_bounds__(kDataThreads) k_nsdf_data(PermTable perm, FieldDev f, CamDev cam,
                                                             uint32_t w, uint32_t h, float3 bmin,
                                                             float3 bmax, uint32_t n, uint32_t seed,
                                                             float4* __restrict__ out) {
   extern __shared__ uint32_t rows_smem[];
   const FieldRows P = load_rows(perm, rows_smem);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  // the warps of all blocks in turn, so that few points spread over the SMs
+  const uint32_t first = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32u + (threadIdx.x & 31u);
+  for (uint32_t i = first; i < n; i += gridDim.x * blockDim.x) {
     float px = 0.f, py = 0.f, pz = 0.f;
     bool placed = false;
     if (i & 1u) {
@@ -1492,12 +1499,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_nsdf_cone(InputMap m,
 enum : uint32_t { kMarch = 0, kProbe = 1, kRoot = 2, kNormal = 3 };
 
 // the field's table, then the warps' rings (64 entries of 32 bytes each)
-constexpr uint32_t kRefineSmemBytes = kRowsSmemBytes + (kRowsThreads / 32) * 64 * 32;
+constexpr uint32_t kRefineRing = 64 * 32;
 
 // NT: the normal (RefineDev::normal_taps), fixed at compile time so that
 // the analytic-gradient form (1) carries no stencil state.
-template <uint32_t NT>
-__global__ void __launch_bounds__(kRowsThreads) k_sdf_refine(
+template <uint32_t NT, class FORM>
+__global__ void __launch_bounds__(FORM::kThreads) k_sdf_refine(
     PermTable perm, FieldDev f, RefineDev rd, CamDev cam, uint32_t w, uint32_t h, RowsSpread spread,
     int direct, const uint4* __restrict__ queue, uint32_t* __restrict__ counters,
     unsigned long long* __restrict__ totals, float4* __restrict__ out) {
@@ -1509,9 +1516,9 @@ __global__ void __launch_bounds__(kRowsThreads) k_sdf_refine(
   // the few lanes that happen to be idle; idle lanes then take entries.
   // Entry: {d.xyz, t} and {pixel (0xFFFFFFFF: no ray), t_lo bits, base
   // steps, 0}.
-  float4(*ring_a)[64] = reinterpret_cast<float4(*)[64]>(rows_smem + kRowsSmemBytes / 4);
-  uint4(*ring_b)[64] = reinterpret_cast<uint4(*)[64]>(ring_a + kRowsThreads / 32);
-  const FieldRows P = load_rows(perm, rows_smem);
+  float4(*ring_a)[64] = reinterpret_cast<float4(*)[64]>(rows_smem + FORM::kBytes / 4);
+  uint4(*ring_b)[64] = reinterpret_cast<uint4(*)[64]>(ring_a + FORM::kThreads / 32);
+  const auto P = FORM::load(perm, rows_smem);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   if (warp >= spread.warps) return;
   // direct mode claims pixels in 8x4 tiles (claim i = lane i & 31 of tile
@@ -2131,7 +2138,7 @@ RE_API re_status re_nsdf_generate(re_nsdf* s, const re_sdf_params* field, const 
   bmax.z = s->map.center[2] + 1.f / s->map.inv_half[2];
   RE_CUDA(cudaFuncSetAttribute(re::nsdf::k_nsdf_data, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)re::kRowsSmemBytes));
-  re::nsdf::k_nsdf_data<<<re::sm_count(), re::kRowsThreads, re::kRowsSmemBytes, cs>>>(
+  re::nsdf::k_nsdf_data<<<re::sm_count(), re::nsdf::kDataThreads, re::kRowsSmemBytes, cs>>>(
       re::perm_of(field->seed), re::field_of(*field), re::cam_dev(*cam), w, h, bmin, bmax,
       num_points, seed, s->data);
   RE_CHECK_LAUNCH("re_nsdf_generate: launch");
@@ -2463,11 +2470,6 @@ RE_API re_status re_nsdf_trace_exact(re_nsdf* s, const re_sdf_params* field,
     return re::fail(RE_ERR_INVALID_ARG, "re_nsdf_trace_exact: no network phase for this image");
   cudaStream_t cs = (cudaStream_t)stream;
   unsigned long long* totals = reinterpret_cast<unsigned long long*>(s->counters + 4);
-  auto kr = tp->normal_taps == 1u   ? re::nsdf::k_sdf_refine<1u>
-            : tp->normal_taps == 4u ? re::nsdf::k_sdf_refine<4u>
-                                    : re::nsdf::k_sdf_refine<6u>;
-  RE_CUDA(cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)re::nsdf::kRefineSmemBytes));
   re::nsdf::RefineDev rd;
   rd.max_steps = tp->max_exact_steps ? tp->max_exact_steps : field->max_steps;
   rd.root_steps = tp->root_steps ? tp->root_steps : 4;
@@ -2482,10 +2484,27 @@ RE_API re_status re_nsdf_trace_exact(re_nsdf* s, const re_sdf_params* field,
   rd.tile_t = cone ? s->cone_t : nullptr;
   rd.cone_tile = cone ? s->cone_tile : 1u;
   rd.cone_tiles_x = cone ? s->cone_tiles_x : 0u;
-  kr<<<re::sm_count(), re::kRowsThreads, re::nsdf::kRefineSmemBytes, cs>>>(
-      re::perm_of(field->seed), re::field_of(*field), rd, re::cam_dev(*cam), w, h,
-      re::rows_spread((uint64_t)w * h, (uint32_t)re::sm_count()),
-      exact_only || cone ? 1 : 0, s->queue, s->counters, totals, reinterpret_cast<float4*>(d_out));
+  auto refine = [&](auto rows_kernel, auto copy_kernel) {
+    return re::launch_field(
+        rd.normal_taps == 1u ? re::field_on_rows(field->octaves, (uint64_t)w * h)
+                             : re::field_on_rows<true>(field->octaves, (uint64_t)w * h),
+        rows_kernel, copy_kernel, (uint64_t)w * h, [](uint32_t warps) { return warps * re::nsdf::kRefineRing; },
+        [&](auto k, int grid, uint32_t threads, uint32_t smem, re::RowsSpread spread) {
+          k<<<grid, threads, smem, cs>>>(re::perm_of(field->seed), re::field_of(*field), rd,
+                                         re::cam_dev(*cam), w, h, spread,
+                                         exact_only || cone ? 1 : 0, s->queue, s->counters, totals,
+                                         reinterpret_cast<float4*>(d_out));
+        });
+  };
+  using re::CopyForm;
+  using re::RowsForm;
+  st = rd.normal_taps == 1u ? refine(re::nsdf::k_sdf_refine<1u, RowsForm>,
+                                     re::nsdf::k_sdf_refine<1u, CopyForm>)
+       : rd.normal_taps == 4u ? refine(re::nsdf::k_sdf_refine<4u, RowsForm>,
+                                       re::nsdf::k_sdf_refine<4u, CopyForm>)
+                              : refine(re::nsdf::k_sdf_refine<6u, RowsForm>,
+                                       re::nsdf::k_sdf_refine<6u, CopyForm>);
+  if (st != RE_OK) return st;
   RE_CHECK_LAUNCH("re_nsdf_trace_exact: refine launch");
   if (rd.normal_taps == 1u) {
     RE_CUDA(cudaFuncSetAttribute(re::nsdf::k_sdf_grad_normal,

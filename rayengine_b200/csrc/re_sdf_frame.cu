@@ -127,7 +127,8 @@ __device__ __forceinline__ void light_setup(const ShadeDev& S, V3 p, V3& L, floa
 // One step of a live lane's march; all 32 lanes call it.  live turns false
 // when the march is over (step bound, range, or the ray is occluded: prel =
 // 0).  The march starts with t = shadow_tmin, prel = 1, i = 0.
-__device__ __forceinline__ void shadow_step(const FieldRows& P, const ShadeDev& S, V3 p, V3 L,
+template <class PT>
+__device__ __forceinline__ void shadow_step(const PT& P, const ShadeDev& S, V3 p, V3 L,
                                             bool& live, float& t, float& prel, uint32_t& i,
                                             uint32_t& evals) {
   live = live && i < S.shadow_max_steps && t < S.shadow_tmax;
@@ -302,12 +303,13 @@ __device__ __forceinline__ uint32_t finish_pixel(const ShadeDev& S, V3 col, V3 o
 // Same operations, in the same order per pixel, as one loop per pixel.
 constexpr uint32_t kShadeRefill = 4;
 
-__global__ void __launch_bounds__(kRowsThreads) k_sdf_shadow(
+template <class FORM>
+__global__ void __launch_bounds__(FORM::kThreads) k_sdf_shadow(
     PermTable perm, ShadeDev S, uint32_t w, uint32_t h, RowsSpread spread,
     const float4* __restrict__ hits, uint32_t* __restrict__ rgba, uint32_t* __restrict__ cursor,
     unsigned long long* __restrict__ evals_out) {
   extern __shared__ uint32_t rows_smem[];
-  const FieldRows P = load_rows(perm, rows_smem);
+  const auto P = FORM::load(perm, rows_smem);
   if ((threadIdx.x >> 5) >= spread.warps) return;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t tiles_x = (w + 7) / 8;
@@ -462,13 +464,16 @@ re_status shade(const re_sdf_params& f, const re_sdf_shade_params& s, const re_c
     const LaunchWords cursor = launch_words(st);
     if (!cursor.words) return cuda_fail(cursor.error, "re_render_sdf_frame: claim cursor");
     RE_CUDA(cudaMemsetAsync(cursor.words, 0, 4, st));
-    RE_CUDA(cudaFuncSetAttribute(k_sdf_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kRowsSmemBytes));
-    k_sdf_shadow<<<sm_count(), kRowsThreads, kRowsSmemBytes, st>>>(
-        perm_table(f.seed), shade_dev(f, s), w, h,
-        rows_spread((uint64_t)w * h, (uint32_t)sm_count()),
-        reinterpret_cast<const float4*>(d_hits), d_rgba, cursor.words,
-        reinterpret_cast<unsigned long long*>(d_evals));
+    const re_status rs = launch_field(
+        field_on_rows(f.octaves, (uint64_t)w * h), k_sdf_shadow<RowsForm>, k_sdf_shadow<CopyForm>,
+        (uint64_t)w * h, [](uint32_t) { return 0u; },
+        [&](auto k, int grid, uint32_t threads, uint32_t smem, RowsSpread spread) {
+          k<<<grid, threads, smem, st>>>(perm_table(f.seed), shade_dev(f, s), w, h, spread,
+                                         reinterpret_cast<const float4*>(d_hits), d_rgba,
+                                         cursor.words,
+                                         reinterpret_cast<unsigned long long*>(d_evals));
+        });
+    if (rs != RE_OK) return rs;
     RE_CHECK_LAUNCH("re_render_sdf_frame: shadow launch");
   }
   int fin_sm = 0;

@@ -162,11 +162,23 @@ __device__ __forceinline__ float sample(const GridDev& g, V3 p) {
   return result;
 }
 
-__global__ void __launch_bounds__(kRowsThreads) k_bake(PermTable perm, uint32_t octaves,
-                                                       float scale, float amp, GridDev g,
-                                                       float2* __restrict__ out) {
+// Whether a grid of n voxels is baked on the rows: their 128 KB take 2 us more
+// to fill than the copies, and a single octave past an even number costs a
+// pair.  Measured on B200, copies | rows, us: 8 octaves 32^3 8.3 | 10.3, 48^3
+// 12.4 | 12.4, 64^3 18.6 | 16.5; 4 octaves 48^3 8.4 | 10.4, 64^3 12.4 | 12.4; 5
+// octaves 128^3 65.7 | 65.7; 3 octaves 128^3 47.2 | 49.3, 256^3 332 | 331; one
+// octave 256^3 176 | 212.
+inline bool bake_on_rows(uint32_t octaves, uint64_t n) {
+  const bool odd = octaves < 7u && octaves % 2u != 0u;
+  return octaves > 1u && n >= (odd ? 1u << 22 : 200000u);
+}
+
+template <class FORM>
+__global__ void __launch_bounds__(FORM::kThreads) k_bake(PermTable perm, uint32_t octaves,
+                                                         float scale, float amp, GridDev g,
+                                                         float2* __restrict__ out) {
   extern __shared__ uint32_t rows_smem[];
-  const FieldRows P = load_rows(perm, rows_smem);
+  const auto P = FORM::load(perm, rows_smem);
   size_t n = (size_t)g.dim[0] * g.dim[1] * g.dim[2];
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
@@ -446,9 +458,13 @@ RE_API re_status re_voxel_bake(const re_sdf_params* field, const re_voxel_grid* 
   re::perlin_permutation(field->seed, full);
   re::PermTable t;
   for (int i = 0; i < 512; ++i) t.p[i] = (uint8_t)full[i];
-  RE_CUDA(cudaFuncSetAttribute(re::voxel::k_bake, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)re::kRowsSmemBytes));
-  re::voxel::k_bake<<<re::sm_count(), re::kRowsThreads, re::kRowsSmemBytes, (cudaStream_t)stream>>>(
+  const uint64_t n = (uint64_t)g->dim[0] * g->dim[1] * g->dim[2];
+  const bool rows = re::voxel::bake_on_rows(field->octaves, n);
+  auto k = rows ? re::voxel::k_bake<re::RowsForm> : re::voxel::k_bake<re::CopyForm>;
+  const uint32_t threads = rows ? re::RowsForm::kThreads : re::CopyForm::kThreads;
+  const uint32_t smem = rows ? re::RowsForm::kBytes : re::CopyForm::kBytes;
+  RE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k<<<(rows ? 1 : 2) * re::sm_count(), threads, smem, (cudaStream_t)stream>>>(
       t, field->octaves, field->scale, field->amplitude, re::grid_dev(g, d_grid),
       reinterpret_cast<float2*>(d_grid));
   RE_CHECK_LAUNCH("re_voxel_bake: launch");

@@ -77,3 +77,26 @@ def test_no_more_nodes_staged_than_there_are(cuda):
         b.set_tuning(256, 8, 4096, 8)
         assert np.array_equal(b.render().cpu().numpy(), want)
     mesh.close()
+
+
+# fields that the paired form does not suit (few octaves, far coordinates) in
+# most of the terrain pixels and in half of them
+@pytest.mark.parametrize("fields", [[(3, 0.25), (3, 0.25), (8, 0.25)], [(1, 0.25), (8, 0.25)],
+                                    [(8, 300.0), (8, 300.0), (7, 0.25)], [(2, 0.25)]])
+def test_fields_the_pairs_do_not_suit(cuda, fields):
+    from oracle import pyoracle as po
+
+    specs, scenes = [], []
+    for i, (octaves, scale) in enumerate(fields):
+        tc = rb.configs.TerrainConfig(seed=40 + i, octaves=octaves, scale=scale, width=23, height=14)
+        specs.append(dict(terrain=tc.params(), camera=tc.camera(), width=23, height=14, albedo=0.6))
+        scenes.append(dict(kind=1, seed=tc.seed, octaves=octaves, scale=scale, amp=tc.amplitude,
+                           step_factor=tc.step_factor, eps=tc.eps, tmax=tc.tmax,
+                           max_steps=tc.max_steps, cam=tc.camera(), w=23, h=14, albedo=0.6))
+    with rb.Batch(specs, max_depth=3, seed=5, mesh_bias=1e-4) as b:
+        prim = torch.empty((b.total_pixels, 4), dtype=torch.int32, device="cuda")
+        rad = b.render(primary=prim).cpu().numpy()
+        g = np.arange(b.total_pixels, dtype=np.uint32)
+        orad, oprim, _ = po.batch_path(scenes, b.offsets, g, 3, 5, 1e-4)
+        assert np.array_equal(rad.view(np.uint32), orad.view(np.uint32))
+        assert np.array_equal(prim.cpu().numpy()[:, :2], oprim[:, :2])

@@ -83,3 +83,44 @@ def test_frames_past_the_near_range(cuda, octaves, scale):
     nan = np.isnan(want)  # whose payload is not compared
     assert np.array_equal(np.isnan(normal), nan)
     assert np.array_equal(normal[~nan].view(np.uint32), want[~nan].view(np.uint32))
+
+
+# the field's two forms (pairs on the rows, one octave at a time on copies) at
+# the octave counts and sizes where kernels go from one to the other
+@pytest.mark.parametrize("octaves,w,h", [(1, 64, 36), (2, 64, 36), (2, 512, 511), (2, 512, 512),
+                                         (3, 128, 63), (3, 128, 64), (4, 64, 36)])
+def test_forms_of_the_marches(cuda, octaves, w, h):
+    cfg = rb.configs.TerrainConfig(width=w, height=h, octaves=octaves)
+    shade = rb.sdf_shade_params(flags=1)
+    pix = np.random.default_rng(1).choice(w * h, min(w * h, 5000), replace=False).astype(np.uint32)
+    img, hits = rb.render_sdf_frame(cfg.params(), shade, cfg.camera(), w, h)
+    u = hits.cpu().numpy().view(np.uint32).reshape(-1, 8)[pix]
+    ref = po.sdf_image(po.perm(cfg.seed), cfg.camera(), w, h, octaves=octaves, pixels=pix)
+    assert np.array_equal(u[:, 6], ref["steps"]) and np.array_equal(u[:, 7], ref["status"])
+    hit = ref["status"] == 1
+    assert np.array_equal(u[hit, 0:3], ref["pos"][hit].view(np.uint32))
+    assert np.array_equal(u[hit, 3:6], ref["normal"][hit].view(np.uint32))
+    if w * h < 10000:
+        want = po.sdf_frame(po.perm(cfg.seed), cfg.camera(), w, h, cfg.params(), shade)
+        assert np.array_equal(img.cpu().numpy().view(np.uint32), want)
+    # the neural tracer's exact phase alone starts at the camera: the same
+    # steps until a ray's crossing is bracketed, so the same hit or miss
+    net = rb.NeuralSDF((-40.0, -6.0, -20.0), (40.0, 11.0, 60.0), 0.5, 1)
+    for taps in (1, 4, 6):
+        tp = rb.nsdf_trace_params(exact_only=True, normal_taps=taps, root_steps=4)
+        out = net.trace(cfg.params(), tp, cfg.camera(), w, h).cpu().numpy()
+        far = rb.nsdf_trace_params(exact_only=True, normal_taps=1, root_steps=4)
+        base = net.trace(cfg.params(), far, cfg.camera(), w, h).cpu().numpy()
+        assert np.array_equal(out[:, :3], base[:, :3]) and np.array_equal(out[:, 7], base[:, 7])
+    net.close()
+
+
+@pytest.mark.parametrize("octaves,dim", [(1, (64, 65, 64)), (2, (50, 63, 63)), (2, (50, 64, 63)),
+                                         (8, (50, 64, 62)), (8, (50, 64, 63)), (3, (128, 129, 255)),
+                                         (3, (128, 129, 257)), (7, (50, 64, 63))])
+def test_forms_of_the_bake(cuda, octaves, dim):
+    field = rb.sdf_params(octaves=octaves, scale=0.25, amplitude=3.0)
+    sp, org = (0.2, 0.3, 0.25), (-9.0, -3.0, -2.0)
+    got = rb.VoxelGrid.bake(field, dim, sp, org).data.cpu().numpy()
+    want = po.voxel_bake(po.perm(2016), octaves, 0.25, 3.0, dim, sp, org)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
