@@ -84,7 +84,11 @@ __device__ __forceinline__ float bilerp(float tx, float ty, float c00, float c10
 // HIGH, with k_trace_high and k_brush below): 2.40 -> 0.81 ms; each of the 64
 // lookups had taken its own three clamps, 64-bit index and three B-spline
 // evaluations.
-template <uint32_t Q>
+// WARP: all 32 lanes call it, and one whose cell reaches past the grid takes
+// the others with it: of points in no order nearly every warp would run both
+// paths.  2,000,000 points about and in a 32^3 grid at HIGH 195 -> 166 us (each
+// lookup with its own 64 clamps, as it was, 170), MEDIUM 30.8 -> 28.8.
+template <uint32_t Q, bool WARP = false>
 __device__ __forceinline__ float sample(const GridDev& g, V3 p) {
   const float u[3] = {(p.x - g.origin[0]) / g.spacing[0], (p.y - g.origin[1]) / g.spacing[1],
                       (p.z - g.origin[2]) / g.spacing[2]};
@@ -111,6 +115,7 @@ __device__ __forceinline__ float sample(const GridDev& g, V3 p) {
     c[k] = min(max(__float2int_rd(cg), -N), g.dim[k] + N) + kFirst;
     inside = inside && c[k] >= 0 && c[k] <= g.dim[k] - N;
   }
+  if (WARP) inside = __all_sync(0xFFFFFFFFu, inside);
   // v(x, y, z) of the cell, x innermost; rows by pointer
   float w[3][4];
   if (Q == RE_VOXEL_HIGH) {
@@ -193,9 +198,10 @@ __global__ void __launch_bounds__(FORM::kThreads) k_bake(PermTable perm, uint32_
 template <uint32_t Q>
 __global__ void __launch_bounds__(256) k_sample(GridDev g, const float* __restrict__ pts,
                                                 uint32_t n, float* __restrict__ out) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  out[i] = sample<Q>(g, v3(pts[3 * (size_t)i], pts[3 * (size_t)i + 1], pts[3 * (size_t)i + 2]));
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t at = 3 * (size_t)min(i, n - 1u);  // past the last point: its value, not stored
+  const float v = sample<Q, true>(g, v3(pts[at], pts[at + 1], pts[at + 2]));
+  if (i < n) out[i] = v;
 }
 
 struct MarchDev {

@@ -115,3 +115,23 @@ def test_small_grids_and_ragged_frames(cuda, dim, quality):
         # a flat neighbourhood (nearest voxel) has no normal: NaN on both sides
         assert np.array_equal(u[hit, 3:6].view(np.float32), ref["normal"][hit], equal_nan=True)
         assert not u[~hit, 0:6].any()
+
+
+@pytest.mark.parametrize("quality", [0, 1, 2])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 257, 1000])
+def test_lookups_whatever_their_neighbours(cuda, quality, n):
+    """A warp takes the path that suits all its points: each point's value is
+    the one it has alone, inside the grid, across its faces and far outside."""
+    rng = np.random.default_rng(4)
+    dim, spacing, origin = (13, 9, 11), (0.5, 0.7, 0.6), (-3.0, -2.0, -1.0)
+    grid = rb.VoxelGrid(dim, spacing, origin, rng.normal(size=(dim[0] * dim[1] * dim[2], 2)))
+    pts = rng.uniform(-6.0, 8.0, (n, 3)).astype(np.float32)
+    pts[::7] = rng.uniform(-1.0, 2.0, (len(pts[::7]), 3))
+    pts[5::40] = 1e30
+    d = torch.from_numpy(pts).cuda()
+    got = grid.sample(d, quality).cpu().numpy()
+    alone = np.array([float(grid.sample(d[i:i + 1].contiguous(), quality)) for i in range(min(n, 64))],
+                     np.float32)
+    assert np.array_equal(got[:64].view(np.uint32), alone.view(np.uint32))
+    inner = grid.sample(d[::7].contiguous(), quality).cpu().numpy()
+    assert np.array_equal(got[::7].view(np.uint32), inner.view(np.uint32))
