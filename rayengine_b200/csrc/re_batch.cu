@@ -814,17 +814,17 @@ bool paired_suits(const re_sdf_params& f, const CamDev& c) {
 int table_of(const re_batch* b, uint32_t stage_total, uint32_t block_threads) {
   const size_t seeds = b->perms.size() / 512;
   if (seeds == 0) return kNoTables;
-  if (seeds > kWordTablesMax) return kByteTables;
-  if (seeds > kFieldTablesMax ||
-      smem_bytes(b, kFieldTables, stage_total, 512) > kMaxSmem)
-    return kWordTables;
-  const uint32_t field =
-      blocks_per_sm(smem_bytes(b, kFieldTables, stage_total, block_threads), block_threads);
-  const uint32_t word =
-      blocks_per_sm(smem_bytes(b, kWordTables, stage_total, block_threads), block_threads);
-  if (2u * b->paired_pixels < b->cap[kTerrain]) return kWordTables;
-  const bool terrain = b->cap[kTerrain] >= b->cap[kMesh];
-  return (terrain ? 2u : 1u) * field >= word ? kFieldTables : kWordTables;
+  const uint32_t share = b->cap[kTerrain] >= b->cap[kMesh] ? 2u : 1u;
+  // `large` instead of `small`: it fits and leaves enough blocks
+  const auto worth = [&](int large, int small) {
+    return smem_bytes(b, large, stage_total, 512) <= kMaxSmem &&
+           share * blocks_per_sm(smem_bytes(b, large, stage_total, block_threads), block_threads) >=
+               blocks_per_sm(smem_bytes(b, small, stage_total, block_threads), block_threads);
+  };
+  if (seeds <= kFieldTablesMax && 2u * b->paired_pixels >= b->cap[kTerrain] &&
+      worth(kFieldTables, kWordTables))
+    return kFieldTables;
+  return seeds <= kWordTablesMax || worth(kWordTables, kByteTables) ? kWordTables : kByteTables;
 }
 
 using Kernel = void (*)(BatchDev);

@@ -100,3 +100,34 @@ def test_fields_the_pairs_do_not_suit(cuda, fields):
         orad, oprim, _ = po.batch_path(scenes, b.offsets, g, 3, 5, 1e-4)
         assert np.array_equal(rad.view(np.uint32), orad.view(np.uint32))
         assert np.array_equal(prim.cpu().numpy()[:, :2], oprim[:, :2])
+
+
+# the terrain tables past 16 seeds: words or bytes, by the blocks they leave an SM
+# and the kind of most pixels
+@pytest.mark.parametrize("meshes,terrains", [(0, 17), (0, 40), (3, 40), (0, 64), (40, 24)])
+def test_many_seeds(cuda, meshes, terrains):
+    from oracle import pyoracle as po
+
+    cfg = rb.configs.SoupConfig(num_tris=2000)
+    mesh = rb.KDScene.from_packed(cfg.packed(), cfg.kd_params())
+    specs = [dict(mesh=mesh, camera=_cam(15, 12), width=15, height=12, albedo=0.7)] * meshes
+    scenes = []
+    for i in range(terrains):
+        tc = rb.configs.TerrainConfig(seed=70 + i, octaves=5 + i % 4, width=11, height=7)
+        specs = specs + [dict(terrain=tc.params(), camera=tc.camera(), width=11, height=7,
+                              albedo=0.6)]
+        scenes.append(dict(kind=1, seed=tc.seed, octaves=tc.octaves, scale=tc.scale,
+                           amp=tc.amplitude, step_factor=tc.step_factor, eps=tc.eps, tmax=tc.tmax,
+                           max_steps=tc.max_steps, cam=tc.camera(), w=11, h=7, albedo=0.6))
+    with rb.Batch(specs, max_depth=3, seed=5, mesh_bias=1e-4) as b:
+        rad = b.render().cpu().numpy()
+        counts = b.counts()
+        if not meshes:
+            g = np.arange(b.total_pixels, dtype=np.uint32)
+            orad, _, _ = po.batch_path(scenes, b.offsets, g, 3, 5, 1e-4)
+            assert np.array_equal(rad.view(np.uint32), orad.view(np.uint32))
+        for tuning in ((128, 8, 0, 8), (64, 32, 256, 64)):
+            b.set_tuning(*tuning)
+            assert np.array_equal(b.render(graph=True).cpu().numpy(), rad), tuning
+            assert b.counts() == counts and b.stats()["error"] == 0
+    mesh.close()
