@@ -1234,7 +1234,11 @@ def run_reference(args):
         return 0
     from oracle import pyoracle as po
 
-    desc, built_by, kind, step, shipped = reference_workload(args.config)
+    try:
+        desc, built_by, kind, step, shipped = reference_workload(args.config)
+    except FileNotFoundError as e:
+        print(json.dumps({"impl": "reference", "unavailable": f"not built here: {e}"}))
+        return 0
     # size one step to about a second of work on all host cores, less when
     # many steps are asked for, so that the whole run stays within minutes
     target_s = min(1.0, 90.0 / max(1, args.steps + args.warmup))

@@ -47,3 +47,16 @@ def test_reference_arm_prints_one_contract_line(config):
         assert d["cpu_baseline"]["kind"] == "reference" and "REF_MAPPED" in out.stdout
         assert "SAH kd-tree of the configured parameters" in d["cpu_baseline"]["sample"]
         assert 0 < d["as_shipped"]["value"] < d["value"]
+
+
+def test_reference_arm_without_the_reference_says_so():
+    """Without the reference's compiled host code the mesh arms print why and
+    exit with status 0."""
+    if os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libre_ref.so")):
+        pytest.skip("the reference's host code is built here")
+    out = subprocess.run([sys.executable, "bench.py", "--impl", "reference", "--config", "soup",
+                          "--steps", "1", "--warmup", "1"], capture_output=True, text=True,
+                         timeout=600, cwd=ROOT)
+    assert out.returncode == 0, out.stderr[-2000:]
+    d = json.loads(out.stdout.splitlines()[-1])
+    assert d["impl"] == "reference" and "libre_ref.so" in d["unavailable"] and "value" not in d
