@@ -72,3 +72,46 @@ def test_oracle_samplers_on_exact_fields():
     # clamping: far outside reads the edge voxel
     out = po.voxel_sample(grid, dim, sp, org, 0, np.array([[100.0, -100.0, 100.0]], np.float32))
     assert out[0] == lin[5, 0, 6]
+
+
+def test_a_sixth_by_its_reciprocal(tmp_path):
+    """The smooth lookup's weights divide by 6 as a product with the rounded
+    reciprocal and one correction by its exact remainder: the rounded quotient
+    for every mantissa, at the largest and the smallest arguments (the cubes of
+    multiples of 2^-23 from 0 to 1) and between."""
+    import shutil
+    import subprocess
+
+    gcc = shutil.which("gcc")
+    if gcc is None:
+        pytest.skip("no C compiler")
+    src = tmp_path / "sixth.c"
+    src.write_text("""
+#include <math.h>
+#include <stdio.h>
+static float sixth(float x) {
+  const float y = 1.0f / 6.0f, q = x * y;
+  return fmaf(fmaf(-6.0f, q, x), y, q);
+}
+int main(void) {
+  const int exps[] = {0, -1, -2, -23, -47, -69};
+  long bad = 0;
+  for (int e = 0; e < 6; ++e)
+    for (unsigned m = 0; m < 1u << 23; ++m) {
+      volatile float x = ldexpf(1.0f + (float)m * 0x1p-23f, exps[e] - 1);
+      if (sixth(x) != x / 6.0f) ++bad;
+    }
+  for (unsigned k = 0; k <= 1u << 23; ++k) {
+    volatile float a = (float)k * 0x1p-23f, c = a * a;
+    c = c * a;
+    if (sixth(c) != c / 6.0f) ++bad;
+  }
+  printf("%ld\\n", bad);
+  return 0;
+}
+""")
+    exe = str(tmp_path / "sixth")
+    subprocess.run([gcc, "-O2", "-std=c11", "-ffp-contract=off", "-o", exe, str(src), "-lm"],
+                   check=True)
+    out = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert out.stdout.strip() == "0"
