@@ -41,7 +41,7 @@ struct KdDev {
 // Two neighbouring float4 on a 32-byte boundary, in one load: a leaf's box
 // (records of 64 bytes), since divergent loads keep L1 two thirds busy.
 // Measured on B200, one load against two: the heightfield's 1920x1080 primary
-// rays in tiles 606 -> 588 us, its AO frame 2.55 -> 2.54 ms, soups level; AO
+// rays in tiles 606 -> 588 us, its AO frame 2512 -> 2503 us, soups level; AO
 // queue records loaded so: level.
 __device__ __forceinline__ void ldg_pair(const float4* p, float4& a, float4& b) {
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"

@@ -611,9 +611,9 @@ __global__ void __launch_bounds__(128) k_ref_eval(InputMap m, const float* __res
 // Measured on B200, 65,536 rows: one forward launch that stored 257 MB of
 // activations and four backward launches that read them back and transposed
 // the operands with 2-byte stores, the reduction and the copies took 308 us
-// a re_nsdf_loss_grad call; this kernel 59 us, the reduction 6 us, the call
-// 92 us.  What is left is the chain of links (issue slots 48 % busy, 4 rounds
-// of tiles at 15 us).
+// a re_nsdf_loss_grad call; this kernel 60 us, the reduction 7 us, the call
+// 80 us.  What is left is the chain of links (issue slots 41 % busy on the 128
+// SMs in use, 4 rounds of tiles at 15 us).
 constexpr int kTrainThreads = 512;
 constexpr uint32_t kActCols = 72;       // 64 activations, the ones column, 7 zeros
 constexpr uint32_t kOnesX = 99;         // column of ones in the features
@@ -971,8 +971,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_tc_train(
 // layer runs as two MMAs over the features of one chain each (48 columns,
 // then 48 with the position and bias inputs), which add in the order of one.
 //
-// Measured on B200, 1,000,003 points: kernel 154 -> 127 us, call 155 -> 128
-// (issue slots 53 -> 65 % busy; 4 groups with two threads a row: 139 us).
+// Measured on B200, 1,000,003 points: a call 155 -> 128 us (issue slots 53 ->
+// 65 % busy; 4 groups with two threads a row: 141 us).
 constexpr int kEvalGroups = 8;
 constexpr int kEvalThreads = kEvalGroups * kGroupRows;  // 1024
 constexpr uint32_t kEvalCols = 64 * kEvalGroups;        // tensor-memory columns
