@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <new>
 #include <random>
 #include <utility>
@@ -105,12 +106,21 @@ namespace {
 // back, after the device is idle, when this many streams have come by.
 constexpr size_t kSlots = 1024;
 
+struct StreamSlot {
+  uint32_t* words = nullptr;
+  std::atomic<int> held{0};
+};
+using CaptureKey = std::pair<unsigned long long, unsigned long long>;  // capture id, stream
+
 struct WordPool {
   std::mutex mu;
   std::vector<uint32_t*> free;
-  std::map<unsigned long long, uint32_t*> streams;  // by stream id
-  // by capture id and stream handle
-  std::map<std::pair<unsigned long long, unsigned long long>, uint32_t*> captures;
+  std::map<unsigned long long, StreamSlot> streams;  // by stream id
+  std::map<CaptureKey, uint32_t*> captures;
+  // Keys of graphs that are gone, under a lock that is never held across a
+  // CUDA call: CUDA's own thread adds them.
+  std::mutex gone_mu;
+  std::vector<CaptureKey> gone;
 };
 
 // Never destroyed: graphs may outlive the library's static objects.
@@ -127,6 +137,17 @@ struct RelaxedCapture {
 };
 
 cudaError_t take_slot(WordPool& p, uint32_t** out) {
+  std::vector<CaptureKey> gone;
+  {
+    std::lock_guard<std::mutex> lk(p.gone_mu);
+    gone.swap(p.gone);
+  }
+  for (const CaptureKey& k : gone) {
+    auto it = p.captures.find(k);
+    if (it == p.captures.end()) continue;
+    p.free.push_back(it->second);
+    p.captures.erase(it);
+  }
   if (p.free.empty()) {
     RelaxedCapture relaxed;
     uint32_t* slab = nullptr;
@@ -139,32 +160,44 @@ cudaError_t take_slot(WordPool& p, uint32_t** out) {
   return cudaSuccess;
 }
 
+// Words that no caller holds are in no launch that is still to come; those
+// that were enqueued have run once the device is idle.
+void take_back_idle(WordPool& p) {
+  std::vector<unsigned long long> idle;
+  for (auto& s : p.streams)
+    if (s.second.held.load(std::memory_order_acquire) == 0) idle.push_back(s.first);
+  RelaxedCapture relaxed;
+  if (cudaDeviceSynchronize() != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  for (unsigned long long id : idle) {
+    auto it = p.streams.find(id);
+    p.free.push_back(it->second.words);
+    p.streams.erase(it);
+  }
+}
+
 struct CapturedSlot {
   WordPool* pool;
-  std::pair<unsigned long long, unsigned long long> key;
+  CaptureKey key;
 };
 
 void release_captured(void* arg) {
   CapturedSlot* c = static_cast<CapturedSlot*>(arg);
-  {
-    std::lock_guard<std::mutex> lk(c->pool->mu);
-    auto it = c->pool->captures.find(c->key);
-    if (it != c->pool->captures.end()) {
-      c->pool->free.push_back(it->second);
-      c->pool->captures.erase(it);
-    }
+  try {
+    std::lock_guard<std::mutex> lk(c->pool->gone_mu);
+    c->pool->gone.push_back(c->key);
+  } catch (const std::bad_alloc&) {
+    // the slot stays taken
   }
   delete c;
 }
 
-}  // namespace
-
-namespace {
 LaunchWords find_words(cudaStream_t st) {
   LaunchWords w;
-  auto failed = [&w](cudaError_t e) {
+  const auto failed = [&w](cudaError_t e) {
     w.error = e;
-    if (w.lock.owns_lock()) w.lock.unlock();
     return std::move(w);
   };
   int dev = 0;
@@ -184,46 +217,43 @@ LaunchWords find_words(cudaStream_t st) {
     e = cudaStreamGetId(st, &id);
   if (e != cudaSuccess) return failed(e);
   WordPool& p = word_pool(dev);
-  w.lock = std::unique_lock<std::mutex>(p.mu);
+  std::lock_guard<std::mutex> lk(p.mu);
   if (status != cudaStreamCaptureStatusActive) {
     auto it = p.streams.find(id);
     if (it == p.streams.end()) {
-      if (p.streams.size() >= kSlots) {
-        RelaxedCapture relaxed;
-        if (cudaDeviceSynchronize() == cudaSuccess) {
-          for (auto& s : p.streams) p.free.push_back(s.second);
-          p.streams.clear();
-        } else {
-          cudaGetLastError();
-        }
-      }
+      if (p.streams.size() >= kSlots) take_back_idle(p);
       uint32_t* slot = nullptr;
       e = take_slot(p, &slot);
       if (e != cudaSuccess) return failed(e);
-      it = p.streams.emplace(id, slot).first;
+      it = p.streams.try_emplace(id).first;
+      it->second.words = slot;
     }
-    w.words = it->second;
+    it->second.held.fetch_add(1, std::memory_order_relaxed);
+    w.held = &it->second.held;
+    w.words = it->second.words;
     return w;
   }
-  const auto key = std::make_pair(capture, id);
+  const CaptureKey key(capture, id);
   auto it = p.captures.find(key);
   if (it == p.captures.end()) {
     uint32_t* slot = nullptr;
     e = take_slot(p, &slot);
     if (e != cudaSuccess) return failed(e);
+    it = p.captures.emplace(key, slot).first;
     CapturedSlot* c = new CapturedSlot{&p, key};
     cudaUserObject_t obj = nullptr;
     e = cudaUserObjectCreate(&obj, c, release_captured, 1, cudaUserObjectNoDestructorSync);
     if (e != cudaSuccess) {
       delete c;
+      p.captures.erase(it);
       p.free.push_back(slot);
       return failed(e);
     }
-    it = p.captures.emplace(key, slot).first;
     e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
     if (e != cudaSuccess) {
-      w.lock.unlock();
-      cudaUserObjectRelease(obj, 1);  // gives the slot back
+      p.captures.erase(it);
+      p.free.push_back(slot);
+      cudaUserObjectRelease(obj, 1);  // its key is no longer known
       return failed(e);
     }
   }

@@ -2,10 +2,11 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
-#include <mutex>
 #include <string>
+#include <utility>
 
 #include "../../include/rayengine_b200.h"
 
@@ -50,13 +51,19 @@ int sm_count();
 // that no launch which may run beside it uses: every stream has its own, and
 // every graph that is being captured has one per stream of the capture, until
 // the graph and what was instantiated from it are gone.  The caller sets it
-// and launches on `st` before it lets go of the lock.  words null: `error`
-// says why.
+// and launches on `st` while it holds this.  words null: `error` says why.
 constexpr unsigned kLaunchWords = 8;
 struct LaunchWords {
-  std::unique_lock<std::mutex> lock;
   uint32_t* words = nullptr;
   cudaError_t error = cudaSuccess;
+  std::atomic<int>* held = nullptr;  // counts the holders of a stream's words
+  LaunchWords() = default;
+  LaunchWords(LaunchWords&& o) noexcept
+      : words(o.words), error(o.error), held(std::exchange(o.held, nullptr)) {}
+  LaunchWords& operator=(LaunchWords&&) = delete;
+  ~LaunchWords() {
+    if (held) held->fetch_sub(1, std::memory_order_release);
+  }
 };
 LaunchWords launch_words(cudaStream_t st);
 

@@ -117,3 +117,44 @@ def test_more_streams_than_slots(cuda):
         assert rt.cudaStreamDestroy(s) == 0
     torch.cuda.synchronize()
     assert torch.equal(hits, want[0]) and torch.equal(rgba, want[1])
+
+
+_FIRST = """
+import torch
+import rayengine_b200 as rb
+
+tc = rb.configs.TerrainConfig(width=64, height=36)
+n = 64 * 36
+hits = torch.full((n, 8), -1, dtype=torch.int32, device="cuda")
+rgba = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+shade = rb.sdf_shade_params()
+s = torch.cuda.Stream()
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g, stream=s):
+    rb.render_sdf_frame(tc.params(), shade, tc.camera(), 64, 36, hits, rgba, stream=s)
+g.replay()
+torch.cuda.synchronize()
+want = rb.render_sdf_frame(tc.params(), shade, tc.camera(), 64, 36)
+assert torch.equal(rgba, want[0]) and torch.equal(hits, want[1])
+for _ in range(40):  # graphs that come and go
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        rb.render_sdf_frame(tc.params(), shade, tc.camera(), 64, 36, hits, rgba, stream=s)
+    g.replay()
+    del g
+torch.cuda.synchronize()
+assert torch.equal(rgba, want[0]) and torch.equal(hits, want[1])
+print("ok")
+"""
+
+
+def test_first_call_of_a_process_is_captured(cuda):
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", _FIRST], capture_output=True, text=True,
+                         timeout=200, cwd=root)
+    assert out.returncode == 0 and out.stdout.strip() == "ok", out.stderr[-2000:]
