@@ -12,9 +12,9 @@
 // The permutation table travels as a 512-byte kernel parameter and is
 // expanded into shared memory by every block (the march: one copy per lane,
 // so lattice lookups with divergent indices never conflict on a bank; the
-// fBm and heightfield kernels: 16 copies).  The march is bound by the FP32
-// pipes and instruction issue; it runs
-// as a per-lane state machine with lane refills so sky rays (few steps) and
+// fBm and heightfield kernels and marches of few octaves: 16 copies).  The
+// march is bound by the FP32 pipes and instruction issue; it runs as a
+// per-lane state machine with lane refills so sky rays (few steps) and
 // grazing rays (hundreds) keep the warps full.
 #include <cuda_runtime.h>
 

@@ -21,7 +21,8 @@ struct re_scene {
   uint32_t* d_entry = nullptr;  // the host's entry table (FlatTree::entry)
   // [0] tile cursor, [1] queue size, [2] queue cursor, [3] secondary rays,
   // [RE_SCENE_TRUNC_SLOT] rays of the last trace call stopped at the
-  // leaf-visit cap; every trace call clears the first RE_SCENE_RESET_BYTES
+  // leaf-visit cap; every trace call clears the first RE_SCENE_RESET_BYTES.
+  // [RE_SCENE_ORDER_SLOT] whether many caller rays lie side by side
   uint32_t* d_counters = nullptr;
   float4* d_queue = nullptr;
   size_t queue_cap = 0;  // rays
